@@ -234,6 +234,7 @@ struct ZeroList {
 };
 
 // mk_step.cu
+cudaError_t step_prepare();   // per-device kernel attributes; call outside stream capture
 cudaError_t launch_tick_reset(const ZeroList& z, int sm_count, cudaStream_t s);
 cudaError_t launch_integrate(const StepBuffers& b, const StepParams& p, const StepLaunch& l, cudaStream_t s);
 cudaError_t launch_world_masses(const StepBuffers& b, const StepParams& p, cudaStream_t s);
@@ -248,7 +249,6 @@ cudaError_t launch_warm_impulses(const StepBuffers& b, const StepLaunch& l, cons
 cudaError_t launch_warm_targets(const StepBuffers& b, int parity, uint32_t A, float* targets, cudaStream_t s);
 cudaError_t launch_contact_solver(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
                                   cudaStream_t s, const std::function<cudaError_t()>& before_solve = nullptr);
-cudaError_t launch_finish_tick(const StepBuffers& b, const StepParams& p, int parity, cudaStream_t s);
 // Contact solve forms of heavy ticks (MK_TUNE_HEAVY_SOLVE).
 constexpr uint32_t MK_HEAVY_SCATTER = 1, MK_HEAVY_GATHER = 2, MK_HEAVY_SPLIT = 3;
 void set_heavy_solve_form(uint32_t form);   // 0 = the default form
