@@ -1588,7 +1588,16 @@ int mk_read_buffer(MkHandle* h, uint32_t id, void* host, uint64_t cap_bytes, uin
         case MK_BUF_LINKS: src = h->mech.links_final; n = h->mech.links_final ? h->B : 0; row = 48; break;
         case MK_BUF_WARM_PREDICTIONS: src = b.warm_pred; n = b.warm_pred ? counts.active : 0; row = 4; break;
         case MK_BUF_WARM_FEATURES: src = b.warm_features; n = b.warm_features ? counts.active : 0; row = 64; break;
-        case MK_BUF_CLOSURE_SLOTS: src = h->mech.slot_v; n = h->mech.slot_v ? h->mech_params.slots : 0; row = 32; break;
+        case MK_BUF_CLOSURE_SLOTS:
+            if (host && h->mech.slot_v) {
+                e = mk::refresh_closure_columns(h->mech, h->mech_params, h->stream);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+                if (!check(e, err, "closure columns")) return MK_ERR_DEVICE_FAILURE;
+            }
+            src = h->mech.slot_v;
+            n = h->mech.slot_v ? h->mech_params.slots : 0;
+            row = 32;
+            break;
         case MK_BUF_CLOSURE_BLOCKS:   // computed for the 2 x 2 block preconditioners only
             src = h->mech.blk_feat;
             n = (h->mech.blk_feat && (h->mech_params.precond == MK_PRECOND_LEARNED ||

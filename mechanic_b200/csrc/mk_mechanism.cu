@@ -315,6 +315,7 @@ struct MDelta {
 __device__ __forceinline__ void mdelta_add(MDelta& acc, f3 l, f3 a) {
     const float s = 1048576.0f;
     acc.v[0] += (uint32_t)fixed_i32(l.x * s);
+    m.columns_stale = u32(1);
     acc.v[1] += (uint32_t)fixed_i32(l.y * s);
     acc.v[2] += (uint32_t)fixed_i32(l.z * s);
     acc.v[3] += (uint32_t)fixed_i32(a.x * s);
@@ -919,49 +920,42 @@ __device__ __forceinline__ bool finite3(f3 v) {
 // first + i * step of its branches: the joint's Jacobian column and the slot's
 // gradient and diagonal contributions (NaN: none).  With step 32 a warp walks
 // one closure; every slot's arithmetic is the same whoever computes it.
-__device__ __forceinline__ void evaluate_closure(const MechBuffers& m, uint32_t k, uint32_t* st, uint32_t* flags,
-                                                 uint32_t Q, uint32_t first, uint32_t step) {
-    const GpuBearing br = m.bearings[m.cl_bearings[k]];
-    f3 aa, ab, xa, xb;
-    closure_frames(m, br, aa, ab, xa, xb);
-    const f3 rp = aa - ab, ra = xa - xb;
-    const uint32_t s0 = m.cl_slot_off[k], s1 = m.cl_slot_off[k + 1], split = m.cl_split[k];
-    bool active = true;
-    if (!finite3(rp) || !finite3(ra)) {
-        if (first == 0) {
+struct ClosureFrame {
+    f3 aa, ab, xa, xb, rp, ra;   // anchors and axes of both bodies, their differences
+    bool active;                 // the residual is above the tolerance
+};
+// The frame of closure k; `record` adds its residual to the step's maxima.
+__device__ __forceinline__ ClosureFrame closure_frame(const MechBuffers& m, uint32_t k, uint32_t* st, uint32_t* flags,
+                                                      bool record) {
+    ClosureFrame f;
+    closure_frames(m, m.bearings[m.cl_bearings[k]], f.aa, f.ab, f.xa, f.xb);
+    f.rp = f.aa - f.ab;
+    f.ra = f.xa - f.xb;
+    f.active = true;
+    if (!finite3(f.rp) || !finite3(f.ra)) {
+        if (record) {
             atomicOr(flags, MK_INVALID_NUMERIC_FLAG);
             atomicMax(&st[0], 0xffffffffu);
             atomicMax(&st[1], 0xffffffffu);
         }
-        active = false;
+        f.active = false;
     } else {
-        const uint32_t um = round_u32(length(rp) * 1000000.0f);
+        const uint32_t um = round_u32(length(f.rp) * 1000000.0f);
         // axis error as atan2(|a x b|, a . b): FP32 acos (closure.wgsl:295) reads 0
         // below ~3.5e-4 rad, blind to the 1000 micro-degree tolerance
         const float deg = atan2_cr(length(cross(xa, xb)), clampf(dot(xa, xb), -1.0f, 1.0f)) * 57.295779513f;
         const uint32_t ud = round_u32(deg * 1000000.0f);
-        if (first == 0) {
+        if (record) {
             atomicMax(&st[0], um);
             atomicMax(&st[1], ud);
         }
-        active = !(um <= 10u && ud <= 1000u);
+        f.active = !(um <= 10u && ud <= 1000u);
     }
     for (uint32_t sl = s0 + first; sl < s1; sl += step) {
         float g = 0.0f, d = 0.0f;
         uint32_t valid = 0;
-        // the slot's Jacobian column: the links do not move during the
-        // step's PCG rounds, so closure.wgsl:194-266's recomputation in
-        // every round gives these same floats (sign * v == v * sign)
-        const bool side_a = sl < split;
-        const f3 ea = side_a ? aa : ab, ex = side_a ? xa : xb;
-        const float sign = side_a ? 1.0f : -1.0f;
-        f3 axis, anchor;
-        uint32_t coord;
-        joint_frame(m, m.slot_body[sl], axis, anchor, coord);
-        const f3 pd = cross(axis, ea - anchor) * sign;
-        const f3 ad = cross(axis, ex) * sign;
-        m.slot_v[2 * sl] = f4(pd, __uint_as_float(coord < Q ? coord : 0u));
-        m.slot_v[2 * sl + 1] = f4(ad, 0.0f);
+        f3 pd, ad;
+        const uint32_t coord = slot_column(m, f, sl, sl < split, Q, pd, ad);
         if (active) {
             if (coord >= Q) {
                 atomicOr(flags, MK_INVALID_NUMERIC_FLAG);
@@ -994,24 +988,30 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_loop(StepBuffers b,
     uint32_t* state = m.loop_state;
     float* part_a = m.chunk_part;
     float* part_b = m.chunk_part + chunks;
-    bool converged_prev = false;
     uint32_t steps = 0, rounds = 0;
     for (uint32_t step = 0; step < kClosureSteps; ++step) {
         uint32_t* st = state + 2 * step;
-        const bool evaluate = step == 0 || !converged_prev;
         // evaluate_closures (closure.wgsl:268-319): slot contributions
-        if (evaluate) {
-            if (p.wide_closures) {   // a warp per closure, its slots spread over the lanes
-                const uint32_t lane = threadIdx.x & 31u;
-                for (uint32_t k = gtid >> 5; k < NC; k += gnt >> 5) evaluate_closure(m, k, st, flags, Q, lane, 32u);
-            } else {
-                for (uint32_t k = gtid; k < NC; k += gnt) evaluate_closure(m, k, st, flags, Q, 0u, 1u);
-            }
+        if (p.wide_closures) {
+            // closures of dozens of slots: the residuals alone first (a thread per closure).  A
+            // converged step needs no slot: on the 100 x 100 x 10 loop lattice at rest (20M slots)
+            // that takes the loop from 1,160 to 15 us.  Then a warp per closure, its slots
+            // spread over the lanes.
+            for (uint32_t k = gtid; k < NC; k += gnt) closure_frame(m, k, st, flags, true);
+        } else {
+            for (uint32_t k = gtid; k < NC; k += gnt) evaluate_closure(m, k, st, flags, Q, 0u, 1u, true);
         }
         loop_sync<kGrid>(m.grid_barrier, flags);
         const bool unconverged = ld_relaxed_u32(&st[0]) > 10u || ld_relaxed_u32(&st[1]) > 1000u;
-        if (unconverged) ++steps;
-        if (evaluate && p.long_coords) gather_long_runs<kGrid, true>(m, p, m.grad, m.diag, flags);   // long runs first
+        if (p.wide_closures && gtid == 0) *m.columns_stale = unconverged ? 0u : 1u;
+        if (!unconverged) break;   // the steps after a converged one move nothing
+        if (p.wide_closures) {
+            for (uint32_t k = gtid >> 5; k < NC; k += gnt >> 5)
+                evaluate_closure(m, k, st, flags, Q, threadIdx.x & 31u, 32u, false);
+            loop_sync<kGrid>(m.grid_barrier, flags);
+        }
+        ++steps;
+        if (p.long_coords) gather_long_runs<kGrid, true>(m, p, m.grad, m.diag, flags);   // long runs first
         // gather per coordinate in the serial accumulation order, then the PCG's
         // initial vectors (solve_closure_pcg, closure.wgsl:333-427), chunk by chunk
         for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
@@ -1019,10 +1019,10 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_loop(StepBuffers b,
             float part = 0.0f;
             if (q < NQ) {
                 float g = 0.0f, d = 0.0f;
-                if (evaluate && long_run(m, q)) {
+                if (long_run(m, q)) {
                     g = m.grad[m.cq_coords[q]];
                     d = m.diag[m.cq_coords[q]];
-                } else if (evaluate) {
+                } else {
                     for (uint32_t i = m.cq_off[q]; i < m.cq_off[q + 1]; ++i) {
                         const float sg = m.slot_g[i];
                         if (sg == sg) { g += sg; d += m.slot_d[i]; }
@@ -1031,14 +1031,12 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_loop(StepBuffers b,
                 const uint32_t cc = m.cq_coords[q];
                 m.grad[cc] = g;
                 m.diag[cc] = d;
-                if (unconverged) {
-                    float r = 0.0f, z = 0.0f;
-                    if (d > 1.0e-12f) { r = -g; z = r / d; }
-                    sol[cc] = 0.0f; res[cc] = r; pre[cc] = z; dir[cc] = z; op[cc] = 0.0f;
-                    part = r * z;
-                }
+                float r = 0.0f, z = 0.0f;
+                if (d > 1.0e-12f) { r = -g; z = r / d; }
+                sol[cc] = 0.0f; res[cc] = r; pre[cc] = z; dir[cc] = z; op[cc] = 0.0f;
+                part = r * z;
             }
-            if (unconverged && NQ > kSerialDot) chunk_dot(part, part_a, c, s_red);
+            if (NQ > kSerialDot) chunk_dot(part, part_a, c, s_red);
         }
         if (unconverged) {
             loop_sync<kGrid>(m.grid_barrier, flags);
@@ -1112,7 +1110,6 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_loop(StepBuffers b,
                 a_src = !a_src;
             }
         }
-        converged_prev = !unconverged;
     }
     if (gtid == 0) {
         atomicAdd(&b.diag->reserved_b, steps);
@@ -1139,6 +1136,32 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_loop(StepBuffers b,
 // which every warp evaluates for itself (identical operands and order, so
 // identical bits) instead of warp 0 publishing it through shared memory: two
 // barriers per sum instead of four.
+    return f;
+}
+
+// The slot's Jacobian column, stored; returns its coordinate.  The links do not
+// move during the step's PCG rounds, so closure.wgsl:194-266's recomputation in
+// every round gives these same floats (sign * v == v * sign).
+__device__ __forceinline__ uint32_t slot_column(const MechBuffers& m, const ClosureFrame& f, uint32_t sl, bool side_a,
+                                                uint32_t Q, f3& pd, f3& ad) {
+    const f3 ea = side_a ? f.aa : f.ab, ex = side_a ? f.xa : f.xb;
+    const float sign = side_a ? 1.0f : -1.0f;
+    f3 axis, anchor;
+    uint32_t coord;
+    joint_frame(m, m.slot_body[sl], axis, anchor, coord);
+    pd = cross(axis, ea - anchor) * sign;
+    ad = cross(axis, ex) * sign;
+    m.slot_v[2 * sl] = f4(pd, __uint_as_float(coord < Q ? coord : 0u));
+    m.slot_v[2 * sl + 1] = f4(ad, 0.0f);
+    return coord;
+}
+
+__device__ __forceinline__ void evaluate_closure(const MechBuffers& m, uint32_t k, uint32_t* st, uint32_t* flags,
+                                                 uint32_t Q, uint32_t first, uint32_t step, bool record) {
+    const ClosureFrame f = closure_frame(m, k, st, flags, record && first == 0);
+    const f3 rp = f.rp, ra = f.ra;
+    const bool active = f.active;
+    const uint32_t s0 = m.cl_slot_off[k], s1 = m.cl_slot_off[k + 1], split = m.cl_split[k];
 __device__ __forceinline__ double block_sum_d(double v, double* scratch) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -1313,6 +1336,20 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_eval(StepBuffers b,
         const uint32_t qi = 2 * blk, qj = qi + 1;
         const uint32_t ci = m.cq_coords[qi];
         const bool pair = qj < NQ;
+// The columns that a converged step of a wide system did not need, for a read of
+// them (MK_BUF_CLOSURE_SLOTS): a warp per closure, from the links of that step.
+__global__ void __launch_bounds__(kMBlock) k_closure_columns(MechBuffers m, MechParams p) {
+    if (*m.columns_stale == 0u) return;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < p.closures; k += warps) {
+        const ClosureFrame f = closure_frame(m, k, nullptr, nullptr, false);
+        const uint32_t split = m.cl_split[k];
+        f3 pd, ad;
+        for (uint32_t sl = m.cl_slot_off[k] + (threadIdx.x & 31u); sl < m.cl_slot_off[k + 1]; sl += 32u)
+            slot_column(m, f, sl, sl < split, p.coordinate_count, pd, ad);
+    }
+}
+
         const uint32_t cj = pair ? m.cq_coords[qj] : ci;
         const float a = m.diag[ci], d = pair ? m.diag[cj] : 0.0f, bij = blk_b[blk];
         const uint32_t pb = blk ^ 1u;
@@ -1389,7 +1426,7 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_eval(StepBuffers b,
     }
     loop_sync<kGrid>(m.grid_barrier, flags);
     if (tid == 0) {
-        if (unconverged) {
+        {
             cs->live_blocks = p.blocks;
             ++cs->newton_steps;
         } else {
@@ -1799,3 +1836,9 @@ uint64_t mechanism_mlp_scratch_bytes(const MechParams& p) {
 }
 
 }  // namespace mk
+cudaError_t refresh_closure_columns(const MechBuffers& m, const MechParams& p, cudaStream_t s) {
+    if (p.closures == 0 || !p.wide_closures || pcg_residual_mode(p)) return cudaSuccess;
+    k_closure_columns<<<std::min(4096u, (p.closures + 7u) / 8u), kMBlock, 0, s>>>(m, p);
+    return cudaGetLastError();
+}
+

@@ -98,6 +98,7 @@ struct MechBuffers {
     float* blk_hist = nullptr;                  // 12 steps x blocks x 3: outputs used at each Newton step
     float* probe = nullptr;                     // 2 x Q: A * ones, A * alternating signs
     ClosureState* cstate = nullptr;
+    uint32_t* columns_stale = nullptr;          // wide systems: the last step converged before its columns were needed
     float* precond_params = nullptr;            // preconditioner network parameters (mlp::kParams)
     uint32_t* loop_off = nullptr;               // loops + 1: offsets into loop_q
     uint32_t* loop_q = nullptr;                 // closure-coordinate positions of each loop block
@@ -138,3 +139,5 @@ void read_mechanism_readback(const MechBuffers& m, const MechParams& p, const Gp
 uint64_t mechanism_mlp_scratch_bytes(const MechParams& p);
 
 }  // namespace mk
+// Brings slot_v up to date before it is read (reference loop, wide systems).
+cudaError_t refresh_closure_columns(const MechBuffers& m, const MechParams& p, cudaStream_t s);
