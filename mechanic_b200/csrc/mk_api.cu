@@ -770,6 +770,7 @@ int create_impl(const MkCreation* cr, const MkConfig* config, const MkCapacities
     bool ok = check(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), err, "stream");
     ok = ok && check(mk::sort_prepare(), err, "sort kernel attributes");
     ok = ok && check(mk::step_prepare(), err, "solve kernel attributes");
+    if (ok && h->mechanism_active) ok = check(mk::mechanism_prepare(), err, "closure kernel attributes");
     if (ok && (h->residual || h->mech_params.learned_precond))
         ok = check(mk::mlp::init(), err, "network kernel attributes");
     const uint64_t bytes = ok ? carve(h, nullptr) : 0;

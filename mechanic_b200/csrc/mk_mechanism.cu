@@ -19,6 +19,7 @@
 // The closure accumulators are gathered per coordinate from per-joint slots
 // in the serial accumulation order instead of float atomics.
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -41,6 +42,7 @@ constexpr uint32_t kMaxLoop = 8;           // coordinates of one per-loop precon
 // iteration diverged on 16-body loops).  Loops are cut into pieces of 5.
 constexpr uint32_t kLoopPiece = 5;
 constexpr uint32_t kBearingCache = 9;     // float4 per bearing in the projection cache
+constexpr uint32_t kWalkWidth = 4096;      // most bodies of a level of k_reconstruct_walk (two in shared memory)
 constexpr uint32_t kLongList = 256;        // slot runs longer than this are summed in chunks of this many
 
 // ----------------------------------------------------------------- host side
@@ -72,6 +74,64 @@ MechParams make_mech_params(const MkCreation* cr, const StepParams& p, uint32_t 
 
 bool pcg_residual_mode(const MechParams& p) { return p.closure_mode == MK_CLOSURE_PCG_RESIDUAL && p.closures > 0; }
 
+// Tables of the one-block closure solve (k_closure_block), for systems whose
+// counts it can hold; p.block_solve stays 0 for the others and for topologies
+// where a branch leaves its component or two joints share a coordinate.
+constexpr uint32_t kClosureSmem = 220u * 1024u;   // its dynamic shared memory at most
+constexpr uint32_t kBlockChunks = 2;              // 1,024-coordinate chunks that its registers hold
+static void derive_block_solve(const MkCreation* cr, MechParams& p, MechTopology& t) {
+    const GpuMechanismBody* mb = cr->mechanism_bodies;
+    const uint32_t NC = p.closures, S = p.slots, B = cr->body_count;
+    if (NC == 0 || p.long_coords || p.closure_coords > kBlockChunks * kClosureThreads || p.loops > kClosureThreads) return;
+    if ((uint64_t)S * 40u > kClosureSmem || (uint64_t)NC * 28u > kClosureSmem) return;
+    // closures by falling slot count, and the first entry of each place among their slots
+    auto slots_of = [&](uint32_t k) { return t.cl_slot_off[k + 1] - t.cl_slot_off[k]; };
+    t.cl_order.resize(NC);
+    for (uint32_t k = 0; k < NC; ++k) t.cl_order[k] = k;
+    std::stable_sort(t.cl_order.begin(), t.cl_order.end(),
+                     [&](uint32_t x, uint32_t y) { return slots_of(x) > slots_of(y); });
+    p.closure_depth = slots_of(t.cl_order[0]);
+    t.cl_columns.assign(p.closure_depth + 1, 0u);
+    for (uint32_t k : t.cl_order)
+        for (uint32_t j = 0; j < slots_of(k); ++j) ++t.cl_columns[j + 1];
+    for (uint32_t j = 0; j < p.closure_depth; ++j) t.cl_columns[j + 1] += t.cl_columns[j];
+    // in that order: coordinate (position) | closure << 16, and place in the runs
+    std::vector<uint32_t> q_of(S, 0u);
+    for (uint32_t q = 0; q < p.closure_coords; ++q)
+        for (uint32_t i = t.cq_off[q]; i < t.cq_off[q + 1]; ++i) q_of[t.cq_slots[i]] = q;
+    t.col_coord.resize(S);
+    t.col_pos.resize(S);
+    for (uint32_t k = 0; k < NC; ++k) {
+        const uint32_t s0 = t.cl_slot_off[t.cl_order[k]];
+        for (uint32_t j = 0; j < slots_of(t.cl_order[k]); ++j) {
+            t.col_coord[t.cl_columns[j] + k] = q_of[s0 + j] | (k << 16);
+            t.col_pos[t.cl_columns[j] + k] = t.slot_pos[s0 + j];
+        }
+    }
+    // places in cb_bodies: of the closures' bodies, each slot's parent, each coordinate's child body, the parents
+    bool ok = true;
+    std::vector<uint32_t> place(B, kInvalid);
+    for (uint32_t i = 0; i < p.closure_bodies; ++i) place[t.cb_bodies[i]] = i;
+    auto find = [&](uint32_t body) {
+        const uint32_t at = body < B ? place[body] : kInvalid;
+        ok = ok && at != kInvalid;
+        return at == kInvalid ? 0u : at;
+    };
+    for (uint32_t j : t.cl_bearings)
+        for (int side = 0; side < 2; ++side) t.cl_places.push_back(find(cr->bearings[j].metadata[side]));
+    for (uint32_t body : t.slot_body) t.slot_parent.push_back(find(mb[body].metadata[0]));
+    for (uint32_t q = 0; q < p.closure_coords; ++q) t.cq_child.push_back(find(t.slot_body[t.cq_slots[t.cq_off[q]]]));
+    std::vector<uint8_t> driven(cr->coordinate_count, 0);
+    for (uint32_t body : t.cb_bodies) {
+        t.cb_parents.push_back(find(mb[body].metadata[3] ? body : mb[body].metadata[0]));
+        if (mb[body].metadata[3]) continue;
+        const uint32_t coord = cr->bearings[mb[body].metadata[1]].metadata[2];
+        if (coord >= cr->coordinate_count || driven[coord]) ok = false;
+        else driven[coord] = 1;
+    }
+    p.block_solve = ok ? 1u : 0u;
+}
+
 MechTopology derive_topology(const MkCreation* cr, MechParams& p) {
     MechTopology t;
     const uint32_t B = cr->body_count;
@@ -86,6 +146,34 @@ MechTopology derive_topology(const MkCreation* cr, MechParams& p) {
     std::vector<uint32_t> fill(t.level_offsets.begin(), t.level_offsets.end() - 1);
     for (uint32_t i = 0; i < B; ++i)
         if (!mb[i].metadata[3] && mb[i].traversal[1] <= cr->max_depth) t.level_bodies[fill[mb[i].traversal[1]]++] = i;
+    // deep, narrow trees are walked by one block (k_reconstruct_walk): a launch per level costs about
+    // as much as 8 rounds of 1,024 bodies there (5 us against 0.6 us), and the row kernel a few launches
+    {
+        const uint32_t levels = (uint32_t)t.level_offsets.size() - 1u;
+        uint64_t rounds = 0;
+        uint32_t widest = 0;
+        bool filled = true;   // every level down to the deepest has its parents in the level before
+        for (uint32_t l = 1; l < levels; ++l) {
+            const uint32_t n = t.level_offsets[l + 1] - t.level_offsets[l];
+            rounds += (n + 1023) / 1024;
+            widest = std::max(widest, n);
+        }
+        std::vector<uint32_t> at(B, kInvalid);
+        if (levels > 16 && widest <= kWalkWidth && rounds <= 8ull * levels) {
+            for (uint32_t l = 0; l < levels; ++l)
+                for (uint32_t i = t.level_offsets[l]; i < t.level_offsets[l + 1]; ++i)
+                    at[t.level_bodies[i]] = i - t.level_offsets[l];
+            t.level_parent.resize(t.level_bodies.size());
+            for (uint32_t i = 0; i < (uint32_t)t.level_bodies.size(); ++i) {
+                const GpuMechanismBody& r = mb[t.level_bodies[i]];
+                const uint32_t up = r.metadata[0], depth = r.traversal[1];
+                const bool root = up < B && mb[up].metadata[3] != 0u;
+                filled = filled && up < B && depth >= 1 && (depth == 1 ? root : !root && mb[up].traversal[1] + 1 == depth);
+                t.level_parent[i] = depth == 1 ? up : up < B ? at[up] : 0u;
+            }
+            if (filled) p.walk_levels = levels;
+        }
+    }
     // closure branches: walk each endpoint to its root (closure.wgsl:154-192)
     std::map<uint32_t, std::vector<uint32_t>> coord_slots;
     std::vector<uint8_t> closure_root(B, 0);
@@ -170,6 +258,7 @@ MechTopology derive_topology(const MkCreation* cr, MechParams& p) {
         }
         p.loops = (uint32_t)t.loop_off.size() - 1;
     }
+    derive_block_solve(cr, p, t);
     return t;
 }
 
@@ -190,9 +279,24 @@ void carve_mechanism(MechBuffers& m, const MechParams& p, uint32_t B, uint32_t J
     m.deltas = reinterpret_cast<int32_t*>(take(24ull * B));
     m.bear_cache = reinterpret_cast<float4*>(take(16ull * kBearingCache * (J ? J : 1)));
     m.level_bodies = u32(B);
+    if (p.walk_levels) {
+        m.level_begin = u32(p.walk_levels + 1ull);
+        m.level_parent = u32(B);
+        m.level_rows = reinterpret_cast<float4*>(take(48ull * B));
+    }
     m.cl_bearings = u32(p.closures);
     m.cl_slot_off = u32(p.closures + 1);
     m.cl_split = u32(p.closures);
+    if (p.block_solve) {
+        m.cl_order = u32(p.closures);
+        m.cl_columns = u32(p.closure_depth + 1ull);
+        m.col_coord = u32(p.slots);
+        m.col_pos = u32(p.slots);
+        m.cl_places = u32(2ull * p.closures);
+        m.slot_parent = u32(p.slots);
+        m.cq_child = u32(p.closure_coords);
+        m.cb_parents = u32(p.closure_bodies);
+    }
     m.slot_body = u32(p.slots);
     m.cq_coords = u32(p.closure_coords);
     m.cq_off = u32(p.closure_coords + 1);
@@ -211,6 +315,7 @@ void carve_mechanism(MechBuffers& m, const MechParams& p, uint32_t B, uint32_t J
     m.pcg = f32(5ull * Q);
     m.grid_barrier = u32(64);   // its own 256-byte line
     m.loop_state = u32(2ull * kClosureSteps);
+    m.columns_stale = u32(1);
     m.chunk_part = f32(2ull * ((p.closure_coords + kClosureThreads - 1) / kClosureThreads));
     m.chunk_part_d = reinterpret_cast<double*>(take(16ull * ((p.closure_coords + kClosureThreads - 1) / kClosureThreads + 1)));
     m.links_final = p.final_is_a ? m.links_a : m.links_b;
@@ -263,9 +368,21 @@ bool upload_mechanism(MechBuffers& m, const MechParams& p, const MechTopology& t
         if (e == cudaSuccess) e = put(m.drives, d, s);
     }
     if (e == cudaSuccess) e = put(m.level_bodies, t.level_bodies, s);
+    if (e == cudaSuccess && p.walk_levels) e = put(m.level_begin, t.level_offsets, s);
+    if (e == cudaSuccess && p.walk_levels) e = put(m.level_parent, t.level_parent, s);
     if (e == cudaSuccess) e = put(m.cl_bearings, t.cl_bearings, s);
     if (e == cudaSuccess) e = put(m.cl_slot_off, t.cl_slot_off, s);
     if (e == cudaSuccess) e = put(m.cl_split, t.cl_split, s);
+    if (p.block_solve) {
+        if (e == cudaSuccess) e = put(m.cl_order, t.cl_order, s);
+        if (e == cudaSuccess) e = put(m.cl_columns, t.cl_columns, s);
+        if (e == cudaSuccess) e = put(m.col_coord, t.col_coord, s);
+        if (e == cudaSuccess) e = put(m.col_pos, t.col_pos, s);
+        if (e == cudaSuccess) e = put(m.cl_places, t.cl_places, s);
+        if (e == cudaSuccess) e = put(m.slot_parent, t.slot_parent, s);
+        if (e == cudaSuccess) e = put(m.cq_child, t.cq_child, s);
+        if (e == cudaSuccess) e = put(m.cb_parents, t.cb_parents, s);
+    }
     if (e == cudaSuccess && m.slot_closure) e = put(m.slot_closure, t.slot_closure, s);
     if (e == cudaSuccess && m.loop_off) e = put(m.loop_off, t.loop_off, s);
     if (e == cudaSuccess && m.loop_q) e = put(m.loop_q, t.loop_q, s);
@@ -315,7 +432,6 @@ struct MDelta {
 __device__ __forceinline__ void mdelta_add(MDelta& acc, f3 l, f3 a) {
     const float s = 1048576.0f;
     acc.v[0] += (uint32_t)fixed_i32(l.x * s);
-    m.columns_stale = u32(1);
     acc.v[1] += (uint32_t)fixed_i32(l.y * s);
     acc.v[2] += (uint32_t)fixed_i32(l.z * s);
     acc.v[3] += (uint32_t)fixed_i32(a.x * s);
@@ -681,6 +797,92 @@ __global__ void __launch_bounds__(kMBlock) k_reconstruct_level(StepBuffers b, Me
     b.ang[body] = f4(angular, 0.0f);
 }
 
+// The same for deep, narrow trees.  A launch per level costs about 5 us whatever
+// the level holds, so a tree of hundreds of levels is walked by one block
+// instead: first a row per body (in level order) with the parts that do not
+// depend on velocities, over the whole grid, then level by level with the
+// velocities of the level before in shared memory and the rows of two levels
+// loaded ahead; the results go to the rows' place, coalesced, and a last kernel
+// puts them to their bodies (stored out of order by the walk: 315 us).  Bound:
+// one block's issue and the barrier of each level.  100,000 bodies in 207
+// levels (one B200, sum of kernel times): 207 launches 1,400 us, this 268 us.
+// Rows, each an array over the level bodies: {axis * speed, parent's place in
+// the level before} {parent's anchor arm} {child's anchor arm}.
+__global__ void __launch_bounds__(kMBlock) k_reconstruct_rows(StepBuffers b, MechBuffers m, uint32_t count) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count) return;
+    const uint32_t body = m.level_bodies[t];
+    const GpuMechanismBody mb = m.bodies[body];
+    const GpuBearing& br = m.bearings[mb.metadata[1]];
+    const float4 rp = b.rot[mb.metadata[0]], rb = b.rot[body];
+    const bool reversed = mb.metadata[2] != 0u;
+    f3 axis = normalize(quat_rotate(rp, r3(reversed ? br.local_axis_b : br.local_axis_a)));
+    if (reversed) axis = -axis;
+    const f3 pa = quat_rotate(rp, r3(reversed ? br.local_anchor_b : br.local_anchor_a));
+    const f3 ca = quat_rotate(rb, r3(reversed ? br.local_anchor_a : br.local_anchor_b));
+    m.level_rows[t] = f4(axis * m.coords[br.metadata[2]].angular_velocity, __uint_as_float(m.level_parent[t]));
+    m.level_rows[count + t] = f4(pa, 0.0f);
+    m.level_rows[2ull * count + t] = f4(ca, 0.0f);
+}
+
+constexpr uint32_t kWalkThreads = 1024;
+constexpr uint32_t kWalkSmem = 2 * 6 * kWalkWidth * sizeof(float);
+__global__ void __launch_bounds__(kWalkThreads) k_reconstruct_walk(StepBuffers b, MechBuffers m, uint32_t levels,
+                                                                   uint32_t count) {
+    extern __shared__ float s_vel[];   // [level parity][component][place]
+    struct Row {
+        float4 r0, r1, r2;
+    };
+    float4* rows = m.level_rows;
+    auto load = [&](uint32_t at, uint32_t end) -> Row {
+        if (at >= end) return {};
+        return {rows[at], rows[count + at], rows[2ull * count + at]};
+    };
+    // this thread's row of the level at hand and of the two after it (an L2 round trip is longer than a level)
+    uint32_t begin = m.level_begin[1], end = m.level_begin[2];
+    uint32_t end1 = 2 < levels ? m.level_begin[3] : end, end2 = 3 < levels ? m.level_begin[4] : end1;
+    Row now = load(begin + threadIdx.x, end), next = load(end + threadIdx.x, end1);
+    for (uint32_t l = 1; l < levels; ++l) {
+        const Row after = load(end1 + threadIdx.x, end2);
+        const uint32_t end3 = l + 3 < levels ? m.level_begin[l + 4] : end2;
+        float* to = s_vel + (l & 1u) * 6u * kWalkWidth;
+        const float* from = s_vel + ((l & 1u) ^ 1u) * 6u * kWalkWidth;
+        for (uint32_t i = threadIdx.x; begin + i < end; i += kWalkThreads) {
+            const Row r = i < kWalkThreads ? now : load(begin + i, end);
+            const uint32_t up = __float_as_uint(r.r0.w);
+            f3 lp, wp;
+            if (l == 1) {   // `up` is the root's body
+                lp = xyz(b.lin[up]);
+                wp = xyz(b.ang[up]);
+            } else {
+                lp = mkf3(from[up], from[kWalkWidth + up], from[2 * kWalkWidth + up]);
+                wp = mkf3(from[3 * kWalkWidth + up], from[4 * kWalkWidth + up], from[5 * kWalkWidth + up]);
+            }
+            const f3 angular = wp + xyz(r.r0);
+            const f3 av = lp + cross(wp, xyz(r.r1));
+            const f3 linear = av - cross(angular, xyz(r.r2));
+            to[i] = linear.x; to[kWalkWidth + i] = linear.y; to[2 * kWalkWidth + i] = linear.z;
+            to[3 * kWalkWidth + i] = angular.x; to[4 * kWalkWidth + i] = angular.y; to[5 * kWalkWidth + i] = angular.z;
+            rows[begin + i] = f4(linear, 0.0f);
+            rows[count + begin + i] = f4(angular, 0.0f);
+        }
+        begin = end;
+        end = end1;
+        end1 = end2;
+        end2 = end3;
+        now = next;
+        next = after;
+        __syncthreads();
+    }
+}
+__global__ void __launch_bounds__(kMBlock) k_reconstruct_store(StepBuffers b, MechBuffers m, uint32_t count) {
+    const uint32_t t = m.level_begin[1] + blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count) return;
+    const uint32_t body = m.level_bodies[t];
+    b.lin[body] = m.level_rows[t];
+    b.ang[body] = m.level_rows[count + t];
+}
+
 // articulated.wgsl:458-484
 __global__ void __launch_bounds__(kMBlock) k_validate_state(StepBuffers b, MechBuffers m, MechParams p) {
     const uint32_t body = blockIdx.x * blockDim.x + threadIdx.x;
@@ -943,7 +1145,8 @@ __device__ __forceinline__ ClosureFrame closure_frame(const MechBuffers& m, uint
         const uint32_t um = round_u32(length(f.rp) * 1000000.0f);
         // axis error as atan2(|a x b|, a . b): FP32 acos (closure.wgsl:295) reads 0
         // below ~3.5e-4 rad, blind to the 1000 micro-degree tolerance
-        const float deg = atan2_cr(length(cross(xa, xb)), clampf(dot(xa, xb), -1.0f, 1.0f)) * 57.295779513f;
+        const float deg =
+            atan2_cr(length(cross(f.xa, f.xb)), clampf(dot(f.xa, f.xb), -1.0f, 1.0f)) * 57.295779513f;
         const uint32_t ud = round_u32(deg * 1000000.0f);
         if (record) {
             atomicMax(&st[0], um);
@@ -951,6 +1154,32 @@ __device__ __forceinline__ ClosureFrame closure_frame(const MechBuffers& m, uint
         }
         f.active = !(um <= 10u && ud <= 1000u);
     }
+    return f;
+}
+
+// The slot's Jacobian column, stored; returns its coordinate.  The links do not
+// move during the step's PCG rounds, so closure.wgsl:194-266's recomputation in
+// every round gives these same floats (sign * v == v * sign).
+__device__ __forceinline__ uint32_t slot_column(const MechBuffers& m, const ClosureFrame& f, uint32_t sl, bool side_a,
+                                                uint32_t Q, f3& pd, f3& ad) {
+    const f3 ea = side_a ? f.aa : f.ab, ex = side_a ? f.xa : f.xb;
+    const float sign = side_a ? 1.0f : -1.0f;
+    f3 axis, anchor;
+    uint32_t coord;
+    joint_frame(m, m.slot_body[sl], axis, anchor, coord);
+    pd = cross(axis, ea - anchor) * sign;
+    ad = cross(axis, ex) * sign;
+    m.slot_v[2 * sl] = f4(pd, __uint_as_float(coord < Q ? coord : 0u));
+    m.slot_v[2 * sl + 1] = f4(ad, 0.0f);
+    return coord;
+}
+
+__device__ __forceinline__ void evaluate_closure(const MechBuffers& m, uint32_t k, uint32_t* st, uint32_t* flags,
+                                                 uint32_t Q, uint32_t first, uint32_t step, bool record) {
+    const ClosureFrame f = closure_frame(m, k, st, flags, record && first == 0);
+    const f3 rp = f.rp, ra = f.ra;
+    const bool active = f.active;
+    const uint32_t s0 = m.cl_slot_off[k], s1 = m.cl_slot_off[k + 1], split = m.cl_split[k];
     for (uint32_t sl = s0 + first; sl < s1; sl += step) {
         float g = 0.0f, d = 0.0f;
         uint32_t valid = 0;
@@ -1038,7 +1267,7 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_loop(StepBuffers b,
             }
             if (NQ > kSerialDot) chunk_dot(part, part_a, c, s_red);
         }
-        if (unconverged) {
+        {
             loop_sync<kGrid>(m.grid_barrier, flags);
             float rz = dot_total(NQ, m, res, pre, part_a, s_red);
             for (uint32_t round = 0; round < kClosureRounds; ++round) {
@@ -1117,6 +1346,20 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_loop(StepBuffers b,
     }
 }
 
+// The columns that a converged step of a wide system did not need, for a read of
+// them (MK_BUF_CLOSURE_SLOTS): a warp per closure, from the links of that step.
+__global__ void __launch_bounds__(kMBlock) k_closure_columns(MechBuffers m, MechParams p) {
+    if (*m.columns_stale == 0u) return;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < p.closures; k += warps) {
+        const ClosureFrame f = closure_frame(m, k, nullptr, nullptr, false);
+        const uint32_t split = m.cl_split[k];
+        f3 pd, ad;
+        for (uint32_t sl = m.cl_slot_off[k] + (threadIdx.x & 31u); sl < m.cl_slot_off[k + 1]; sl += 32u)
+            slot_column(m, f, sl, sl < split, p.coordinate_count, pd, ad);
+    }
+}
+
 // ------------------------------------------------- closure PCG to a residual
 // MK_CLOSURE_PCG_RESIDUAL: each Newton step of the closure loop solves
 // (J^T J) dtheta = -g by preconditioned conjugate gradients until
@@ -1136,32 +1379,6 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_loop(StepBuffers b,
 // which every warp evaluates for itself (identical operands and order, so
 // identical bits) instead of warp 0 publishing it through shared memory: two
 // barriers per sum instead of four.
-    return f;
-}
-
-// The slot's Jacobian column, stored; returns its coordinate.  The links do not
-// move during the step's PCG rounds, so closure.wgsl:194-266's recomputation in
-// every round gives these same floats (sign * v == v * sign).
-__device__ __forceinline__ uint32_t slot_column(const MechBuffers& m, const ClosureFrame& f, uint32_t sl, bool side_a,
-                                                uint32_t Q, f3& pd, f3& ad) {
-    const f3 ea = side_a ? f.aa : f.ab, ex = side_a ? f.xa : f.xb;
-    const float sign = side_a ? 1.0f : -1.0f;
-    f3 axis, anchor;
-    uint32_t coord;
-    joint_frame(m, m.slot_body[sl], axis, anchor, coord);
-    pd = cross(axis, ea - anchor) * sign;
-    ad = cross(axis, ex) * sign;
-    m.slot_v[2 * sl] = f4(pd, __uint_as_float(coord < Q ? coord : 0u));
-    m.slot_v[2 * sl + 1] = f4(ad, 0.0f);
-    return coord;
-}
-
-__device__ __forceinline__ void evaluate_closure(const MechBuffers& m, uint32_t k, uint32_t* st, uint32_t* flags,
-                                                 uint32_t Q, uint32_t first, uint32_t step, bool record) {
-    const ClosureFrame f = closure_frame(m, k, st, flags, record && first == 0);
-    const f3 rp = f.rp, ra = f.ra;
-    const bool active = f.active;
-    const uint32_t s0 = m.cl_slot_off[k], s1 = m.cl_slot_off[k + 1], split = m.cl_split[k];
 __device__ __forceinline__ double block_sum_d(double v, double* scratch) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -1336,20 +1553,6 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_eval(StepBuffers b,
         const uint32_t qi = 2 * blk, qj = qi + 1;
         const uint32_t ci = m.cq_coords[qi];
         const bool pair = qj < NQ;
-// The columns that a converged step of a wide system did not need, for a read of
-// them (MK_BUF_CLOSURE_SLOTS): a warp per closure, from the links of that step.
-__global__ void __launch_bounds__(kMBlock) k_closure_columns(MechBuffers m, MechParams p) {
-    if (*m.columns_stale == 0u) return;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < p.closures; k += warps) {
-        const ClosureFrame f = closure_frame(m, k, nullptr, nullptr, false);
-        const uint32_t split = m.cl_split[k];
-        f3 pd, ad;
-        for (uint32_t sl = m.cl_slot_off[k] + (threadIdx.x & 31u); sl < m.cl_slot_off[k + 1]; sl += 32u)
-            slot_column(m, f, sl, sl < split, p.coordinate_count, pd, ad);
-    }
-}
-
         const uint32_t cj = pair ? m.cq_coords[qj] : ci;
         const float a = m.diag[ci], d = pair ? m.diag[cj] : 0.0f, bij = blk_b[blk];
         const uint32_t pb = blk ^ 1u;
@@ -1426,7 +1629,7 @@ __global__ void __launch_bounds__(kMBlock) k_closure_columns(MechBuffers m, Mech
     }
     loop_sync<kGrid>(m.grid_barrier, flags);
     if (tid == 0) {
-        {
+        if (unconverged) {
             cs->live_blocks = p.blocks;
             ++cs->newton_steps;
         } else {
@@ -1654,6 +1857,744 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_pcg(StepBuffers b, 
     }
 }
 
+// ------------------------------------------------ closure solve in one block
+// A closure system that fits one block's shared memory is solved there: its
+// Jacobian columns, slot values, search direction and (PCG) preconditioner stay
+// in shared memory, the PCG vectors in the registers of their coordinate's
+// thread, and all Newton steps run in one launch.  The kernels above keep all
+// of that in global memory, where every phase of a round is a chain of L2 round
+// trips.  The evaluation (a thread per slot) and the forward kinematics (a
+// thread per body) are spread over a cluster of blocks when the system is
+// large; the columns go straight to block 0's shared memory.  Each sum keeps
+// the order of those kernels (slots of a closure, slots of a coordinate, the
+// dot products' trees and chunks), so the results are theirs bit for bit.
+// Bound: the dependent chain of each phase and its barrier.  One B200, a tick's
+// closure solve: 380 loops of five bodies in the reference's loop 1,550 us in
+// the kernels above, 500 us here; 49 such loops by PCG to 1e-5 500 us (24
+// launches), 196 us.  The line (closure_block_shape) is what the registers and
+// the shared memory hold; systems with runs over kLongList slots keep the
+// kernels above.
+//
+// Slots are laid out by their place j in their closure, closures sorted by
+// falling slot count: slot j of closure k is column_off[j] + k, so the threads
+// of neighbouring closures read neighbouring words.
+constexpr uint32_t kClosureCluster = 8;                    // blocks of a spread system (portable cluster size)
+constexpr uint32_t kClosureFew = 256;                      // up to this many threads: compiled for 255 registers
+// Slots or bodies above which a system is spread over the cluster.  Reference
+// loop and PCG, one block / eight: 80 five-body loops (320 slots) 471 / 475 and
+// 193 / 207 us, 130 loops (520 slots) 333 / 323 and 217 / 222 us, 380 loops
+// 590 / 499 us; beyond, a block walks its slots and bodies in several rounds.
+constexpr uint32_t kClosureSpread = 512;
+constexpr uint32_t kPieceEntries = kLoopPiece * (kLoopPiece + 1) / 2;
+
+// Word offsets of the dynamic shared memory.
+struct ClosureLayout {
+    uint32_t all_max, clos, frame, slot, fk, angle, link_pos, link_rot, col_off;   // every block
+    uint32_t terms, len, sums, col, g, d, qi, pos, off, dir;                       // block 0
+    uint32_t diag, res, z, cqs, loop_off, loop_q, l, words;                        // block 0, PCG to a residual
+};
+__host__ __device__ inline ClosureLayout closure_layout(const MechParams& p, uint32_t blocks, bool pcg) {
+    ClosureLayout L{};
+    const uint32_t NC = p.closures, S = p.slots, NQ = p.closure_coords;
+    const uint32_t per = (NC + blocks - 1) / blocks, bodies = (p.closure_bodies + blocks - 1) / blocks;
+    uint32_t w = 0;
+    auto take = [&](uint32_t n) { const uint32_t at = w; w += (n + 3u) & ~3u; return at; };
+    L.all_max = take(2 * kClosureCluster);
+    L.clos = take(15 * per);   // positions of its bodies, local anchors and axes of the closure bearing, its row
+    L.frame = take(13 * per);  // its world anchors and axes of the step, and whether it is active
+    L.slot = take(8 * per * p.closure_depth);   // parent's position (with side and direction), local axis and anchor
+                                                // of the joint, place of its value in the runs
+    L.fk = take(14 * bodies);  // axis, anchors and bind rotation of the body's joint, and its direction
+    L.angle = take(bodies);    // the joint's angle
+    L.link_pos = take(2 * 4 * bodies);   // the links of the forward kinematics, two buffers:
+    L.link_rot = take(2 * 4 * bodies);   // {position, parent's position in the list | done}, rotation
+    L.col_off = take(p.closure_depth + 1);
+    L.terms = take(kBlockChunks * 32 * 33 * 2);   // terms of a dot product, 32-term groups 33 words apart
+    L.len = take(NC);          // slots of the closure, and of its branch a
+    L.sums = take(6 * NC);     // branch products of the closure
+    L.col = take(6 * S);       // the joint's Jacobian column
+    L.g = take(S);             // slot values, at their position in the coordinates' runs
+    L.d = take(S);
+    L.qi = take(S);            // coordinate (position in the list) and closure of the slot
+    L.pos = take(S);
+    L.off = take(NQ + 1);      // first slot value of each coordinate's run
+    L.dir = take(NQ);
+    if (pcg) {
+        L.diag = take(NQ);
+        L.res = take(NQ);
+        L.z = take(NQ);
+        L.cqs = take(S);
+        L.loop_off = take(p.loops + 1);
+        L.loop_q = take(NQ);
+        L.l = take(kPieceEntries * p.loops);
+    }
+    L.words = w;
+    return L;
+}
+
+constexpr uint32_t kSlotSideA = 1u << 30, kSlotReversed = 1u << 31, kSlotParent = kSlotSideA - 1u;
+constexpr uint32_t kLinkDone = 1u << 31;   // the link is relative to its root
+
+// The dot products of the one-block solve, in the order of chunk_dot and
+// dot_total (FP32) and of block_sum_d and chunk_total_d (FP64): the tree of a
+// shuffle-down over 32 consecutive terms, the same tree over a chunk's 32 group
+// sums, the chunks in order.  The terms go through shared memory: a thread sums
+// a group (its words 33 apart, so no two threads of the warp share a bank) and
+// one warp a chunk, which costs a third of the shuffles by every warp.  Terms
+// past `nq` stay zero.
+template <class T>
+__device__ __forceinline__ T block_dot(const T (&part)[kBlockChunks], uint32_t nq, T* terms, T* totals) {
+    const uint32_t tid = threadIdx.x, w = warp_id(), lane = lane_id();
+#pragma unroll
+    for (uint32_t c = 0; c < kBlockChunks; ++c)
+        if (c * kDotChunk + tid < nq) terms[c * 32 * 33 + tid + tid / 32] = part[c];
+    __syncthreads();
+    if (w < kBlockChunks && w * kDotChunk < nq) {
+        const T* r = terms + w * 32 * 33 + lane * 33;
+        T h[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) h[k] = (r[k] + r[k + 16]) + (r[k + 8] + r[k + 24]);
+        T v = ((h[0] + h[4]) + (h[2] + h[6])) + ((h[1] + h[5]) + (h[3] + h[7]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) totals[w] = v;
+    }
+    __syncthreads();
+    T acc = (T)0;
+#pragma unroll
+    for (uint32_t c = 0; c < kBlockChunks; ++c)
+        if (c * kDotChunk < nq) acc += totals[c];
+    return acc;
+}
+
+// Barrier over the cluster's blocks (release / acquire, global memory included).
+__device__ __forceinline__ void cluster_sync(uint32_t blocks) {
+    if (blocks == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+// The address in block `rank`'s shared memory that corresponds to `v` in this block's.
+template <class T>
+__device__ __forceinline__ T* cluster_map(T* v, uint32_t rank) {
+    T* out;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(v), "r"(rank));
+    return out;
+}
+
+template <bool kPcg, uint32_t kThreads>
+__global__ void __launch_bounds__(kThreads) k_closure_block(StepBuffers b, MechBuffers m, MechParams p) {
+    extern __shared__ __align__(16) float s_dyn[];
+    __shared__ uint32_t s_max[2];
+    __shared__ double s_tot[kBlockChunks];
+    const uint32_t blocks = gridDim.x, rank = blockIdx.x;   // the grid is one cluster of 2^shift blocks
+    const uint32_t shift = 31u - __clz(blocks), rank_mask = blocks - 1u;
+    const ClosureLayout L = closure_layout(p, blocks, kPcg);
+    const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = lane_id();
+    const uint32_t NC = p.closures, S = p.slots, NQ = p.closure_coords, Q = p.coordinate_count;
+    const uint32_t per = (NC + blocks - 1) / blocks;                   // closures of a block, [k0, k0 + per)
+    const uint32_t k0 = rank * per, mine = k0 < NC ? min(per, NC - k0) : 0u;
+    const uint32_t rows = (p.closure_bodies + blocks - 1) / blocks;    // bodies of a block: one per thread
+    const uint32_t place = tid * blocks + rank;                        // this thread's body in the list
+    const bool has_body = tid < rows && place < p.closure_bodies;
+    uint32_t* flags = &b.diag->error_flags;
+    uint32_t* all_max = reinterpret_cast<uint32_t*>(s_dyn + L.all_max);
+    float* clos = s_dyn + L.clos;
+    float* frame = s_dyn + L.frame;
+    float* slot = s_dyn + L.slot;
+    float* fk = s_dyn + L.fk;
+    float* angle_s = s_dyn + L.angle;
+    float4* link_pos = reinterpret_cast<float4*>(s_dyn + L.link_pos);
+    float4* link_rot = reinterpret_cast<float4*>(s_dyn + L.link_rot);
+    uint32_t* col_off = reinterpret_cast<uint32_t*>(s_dyn + L.col_off);
+    uint32_t* len = reinterpret_cast<uint32_t*>(s_dyn + L.len);
+    float* sums = s_dyn + L.sums;
+    float* col = s_dyn + L.col;
+    float* sg = s_dyn + L.g;
+    float* sd = s_dyn + L.d;
+    uint32_t* qi = reinterpret_cast<uint32_t*>(s_dyn + L.qi);
+    uint32_t* pos = reinterpret_cast<uint32_t*>(s_dyn + L.pos);
+    uint32_t* off = reinterpret_cast<uint32_t*>(s_dyn + L.off);
+    float* dir_s = s_dyn + L.dir;
+    auto at3 = [](const float* base, uint32_t i, uint32_t stride, uint32_t k) {
+        return mkf3(base[i * stride + k], base[(i + 1) * stride + k], base[(i + 2) * stride + k]);
+    };
+    auto put3 = [](float* base, uint32_t i, uint32_t stride, uint32_t k, f3 v) {
+        base[i * stride + k] = v.x;
+        base[(i + 1) * stride + k] = v.y;
+        base[(i + 2) * stride + k] = v.z;
+    };
+    // the link of the body at `at` in the list (in the memory of the block that owns it)
+    auto load_link = [&](uint32_t buffer, uint32_t at, float4& lp, float4& lr) {
+        const uint32_t i = buffer * rows + (at >> shift), owner = at & rank_mask;
+        lp = *cluster_map(link_pos + i, owner);
+        lr = *cluster_map(link_rot + i, owner);
+    };
+    const uint32_t final_buffer = p.final_is_a ? 0u : 1u;
+    // ---- the system's constant rows: this block's closures, joints and bodies
+    const uint32_t tasks = p.closure_depth * per;   // (place j, closure) of this block's slots
+    for (uint32_t j = tid; j <= p.closure_depth; j += nt) col_off[j] = m.cl_columns[j];
+    for (uint32_t i = tid; i < mine; i += nt) {
+        const uint32_t k = m.cl_order[k0 + i];
+        const GpuBearing br = m.bearings[m.cl_bearings[k]];
+        clos[i] = __uint_as_float(m.cl_places[2 * k]);
+        clos[per + i] = __uint_as_float(m.cl_places[2 * k + 1]);
+        put3(clos, 2, per, i, r3(br.local_anchor_a));
+        put3(clos, 5, per, i, r3(br.local_anchor_b));
+        put3(clos, 8, per, i, r3(br.local_axis_a));
+        put3(clos, 11, per, i, r3(br.local_axis_b));
+    }
+    for (uint32_t t = tid; t < tasks; t += nt) {
+        const uint32_t j = t / per, i = t - j * per;
+        if (i >= mine || k0 + i >= m.cl_columns[j + 1] - m.cl_columns[j]) continue;
+        const uint32_t k = m.cl_order[k0 + i], sl = m.cl_slot_off[k] + j;
+        const GpuMechanismBody* mb = m.bodies + m.slot_body[sl];
+        const GpuBearing& tb = m.bearings[mb->metadata[1]];
+        const bool reversed = mb->metadata[2] != 0u;
+        slot[t] = __uint_as_float(m.slot_parent[sl] | (sl < m.cl_split[k] ? kSlotSideA : 0u) |
+                                  (reversed ? kSlotReversed : 0u));
+        put3(slot, 1, tasks, t, reversed ? r3(tb.local_axis_b) : r3(tb.local_axis_a));
+        put3(slot, 4, tasks, t, reversed ? r3(tb.local_anchor_b) : r3(tb.local_anchor_a));
+        slot[7 * tasks + t] = __uint_as_float(m.slot_pos[sl]);
+    }
+    bool root = false;
+    uint32_t body = 0, parent = 0;
+    if (has_body) {   // prepare_link's constant part, and the links as they stand
+        body = m.cb_bodies[place];
+        parent = m.cb_parents[place];
+        const GpuMechanismBody mb = m.bodies[body];
+        root = mb.metadata[3] != 0u;
+        if (!root) {
+            const GpuBearing& br = m.bearings[mb.metadata[1]];
+            const bool reversed = mb.metadata[2] != 0u;
+            put3(fk, 0, rows, tid, normalize(reversed ? r3(br.local_axis_b) : r3(br.local_axis_a)));
+            put3(fk, 3, rows, tid, reversed ? r3(br.local_anchor_b) : r3(br.local_anchor_a));
+            put3(fk, 6, rows, tid, reversed ? r3(br.local_anchor_a) : r3(br.local_anchor_b));
+            const float4 bind = r4(mb.bind_relative_rotation);
+            put3(fk, 9, rows, tid, xyz(bind));
+            fk[12 * rows + tid] = bind.w;
+            fk[13 * rows + tid] = reversed ? -1.0f : 1.0f;
+            // the reference's loop adds 0 to the coordinates off the closure branches
+            const float angle = m.coords[br.metadata[2]].angle;
+            angle_s[tid] = kPcg ? angle : angle + 0.0f;
+        }
+        const Link l = ld_link(m.links_final, body);
+        link_pos[final_buffer * rows + tid] = l.pos;
+        link_rot[final_buffer * rows + tid] = l.rot;
+    }
+    uint32_t coord[kBlockChunks], child[kBlockChunks];   // this thread's coordinates and their joints' bodies
+    float angle[kBlockChunks];
+#pragma unroll
+    for (uint32_t c = 0; c < kBlockChunks; ++c) {
+        coord[c] = child[c] = 0u;
+        angle[c] = 0.0f;
+    }
+    if (rank == 0) {
+        for (uint32_t q = tid; q <= NQ; q += nt) off[q] = m.cq_off[q];
+        for (uint32_t i = tid; i < kBlockChunks * 32 * 33 * 2; i += nt) s_dyn[L.terms + i] = 0.0f;
+        for (uint32_t k = tid; k < NC; k += nt) {
+            const uint32_t c = m.cl_order[k], s0 = m.cl_slot_off[c], n = m.cl_slot_off[c + 1] - s0;
+            len[k] = n | ((m.cl_split[c] - s0) << 16);
+        }
+        if (kPcg) {
+            for (uint32_t i = tid; i <= p.loops; i += nt)
+                reinterpret_cast<uint32_t*>(s_dyn + L.loop_off)[i] = m.loop_off[i];
+            for (uint32_t i = tid; i < NQ; i += nt) reinterpret_cast<uint32_t*>(s_dyn + L.loop_q)[i] = m.loop_q[i];
+        }
+#pragma unroll
+        for (uint32_t c = 0; c < kBlockChunks; ++c) {
+            const uint32_t q = c * kDotChunk + tid;
+            if (q >= NQ) continue;
+            coord[c] = m.cq_coords[q];
+            child[c] = m.cq_child[q];
+            angle[c] = m.coords[coord[c]].angle;
+        }
+        for (uint32_t at = tid; at < S; at += nt) {
+            qi[at] = m.col_coord[at];
+            pos[at] = m.col_pos[at];
+            if (kPcg) reinterpret_cast<uint32_t*>(s_dyn + L.cqs)[pos[at]] = at;
+        }
+    }
+    if (tid == 0) s_max[0] = s_max[1] = 0u;
+    cluster_sync(blocks);   // every block's shared memory is up before another reads or writes it
+    float* col0 = cluster_map(col, 0u);
+    float* sg0 = cluster_map(sg, 0u);
+    float* sd0 = cluster_map(sd, 0u);
+
+    // sg[slot position] = the slot's share of J^T J dir (closure_products): the branch
+    // products, a closure's position or axis rows per thread, then a slot per thread
+    auto products = [&]() {
+        for (uint32_t t = tid; t < 2u * NC; t += nt) {
+            const uint32_t half = t >= NC ? 3u : 0u, k = t >= NC ? t - NC : t;
+            const uint32_t n = len[k] & 0xffffu, split = len[k] >> 16;
+            f3 sum_a = mkf3(0, 0, 0), sum_b = mkf3(0, 0, 0);
+#pragma unroll 4
+            for (uint32_t j = 0; j < n; ++j) {
+                const uint32_t at = col_off[j] + k;
+                const f3 term = at3(col, half, S, at) * dir_s[qi[at] & 0xffffu];
+                if (j < split) sum_a = sum_a + term;
+                else sum_b = sum_b + term;
+            }
+            put3(sums, half, NC, k, sum_a + sum_b);
+        }
+        __syncthreads();
+        for (uint32_t at = tid; at < S; at += nt) {
+            const uint32_t k = qi[at] >> 16;
+            sg[pos[at]] = dot(at3(col, 0, S, at), at3(sums, 0, NC, k)) + 1.0f * dot(at3(col, 3, S, at), at3(sums, 3, NC, k));
+        }
+    };
+    auto run_sum = [&](uint32_t q) {
+        float o = 0.0f;
+        for (uint32_t i = off[q]; i < off[q + 1]; ++i) o += sg[i];
+        return o;
+    };
+    // a dot product of the reference's loop: serial up to kSerialDot coordinates
+    auto dot_f = [&](const float (&x)[kBlockChunks], const float (&y)[kBlockChunks]) -> float {
+        if (NQ <= kSerialDot) {
+            float* prod = s_dyn + L.terms;
+            if (tid < NQ) prod[tid] = x[0] * y[0];
+            __syncthreads();
+            if (tid == 0) {
+                float acc = 0.0f;
+                const uint32_t whole = NQ & ~3u;
+#pragma unroll 8
+                for (uint32_t q = 0; q < whole; q += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(prod + q);
+                    acc = (((acc + v.x) + v.y) + v.z) + v.w;
+                }
+                for (uint32_t q = whole; q < NQ; ++q) acc += prod[q];
+                reinterpret_cast<float*>(s_tot)[0] = acc;
+            }
+            __syncthreads();
+            return reinterpret_cast<float*>(s_tot)[0];
+        }
+        float part[kBlockChunks];
+#pragma unroll
+        for (uint32_t c = 0; c < kBlockChunks; ++c) part[c] = c * kDotChunk + tid < NQ ? x[c] * y[c] : 0.0f;
+        return block_dot<float>(part, NQ, s_dyn + L.terms, reinterpret_cast<float*>(s_tot));
+    };
+    auto dot_d = [&](const float (&x)[kBlockChunks], const float (&y)[kBlockChunks]) -> double {
+        double part[kBlockChunks];
+#pragma unroll
+        for (uint32_t c = 0; c < kBlockChunks; ++c)
+            part[c] = c * kDotChunk + tid < NQ ? (double)x[c] * (double)y[c] : 0.0;
+        return block_dot<double>(part, NQ, reinterpret_cast<double*>(s_dyn + L.terms), s_tot);
+    };
+    uint32_t steps = 0, rounds = 0, done = 0, newton = 0, iterations = 0;
+    double worst = 0.0;
+    for (uint32_t step = 0; step < kClosureSteps; ++step) {
+        // ---- evaluate_closures (closure.wgsl:268-319): frames and residuals
+        uint32_t um = 0u, ud = 0u;
+        for (uint32_t i = tid; i < mine; i += nt) {
+            float4 pa, ra4, pb, rb4;
+            load_link(final_buffer, __float_as_uint(clos[i]), pa, ra4);
+            load_link(final_buffer, __float_as_uint(clos[per + i]), pb, rb4);
+            const f3 aa = xyz(pa) + quat_rotate(ra4, at3(clos, 2, per, i));
+            const f3 ab = xyz(pb) + quat_rotate(rb4, at3(clos, 5, per, i));
+            const f3 xa = normalize(quat_rotate(ra4, at3(clos, 8, per, i)));
+            const f3 xb = normalize(quat_rotate(rb4, at3(clos, 11, per, i)));
+            const f3 rp = aa - ab, ra = xa - xb;
+            bool active = false;
+            if (!finite3(rp) || !finite3(ra)) {
+                atomicOr(flags, MK_INVALID_NUMERIC_FLAG);
+                um = ud = 0xffffffffu;
+            } else {
+                const uint32_t u = round_u32(length(rp) * 1000000.0f);
+                const float deg = atan2_cr(length(cross(xa, xb)), clampf(dot(xa, xb), -1.0f, 1.0f)) * 57.295779513f;
+                const uint32_t v = round_u32(deg * 1000000.0f);
+                active = !(u <= 10u && v <= 1000u);
+                um = max(um, u);
+                ud = max(ud, v);
+            }
+            put3(frame, 0, per, i, aa);
+            put3(frame, 3, per, i, ab);
+            put3(frame, 6, per, i, xa);
+            put3(frame, 9, per, i, xb);
+            frame[12 * per + i] = active ? 1.0f : 0.0f;
+        }
+        um = __reduce_max_sync(0xffffffffu, um);
+        ud = __reduce_max_sync(0xffffffffu, ud);
+        if (lane == 0 && um) atomicMax(&s_max[0], um);
+        if (lane == 0 && ud) atomicMax(&s_max[1], ud);
+        __syncthreads();
+        if (tid < blocks) {   // this block's maxima to every block
+            uint32_t* to = cluster_map(all_max, tid);
+            to[2 * rank] = s_max[0];
+            to[2 * rank + 1] = s_max[1];
+        }
+        // ---- the joints' columns and their gradient and diagonal contributions
+        for (uint32_t t = tid; t < tasks; t += nt) {
+            const uint32_t j = t / per, i = t - j * per;
+            const uint32_t at = col_off[j] + k0 + i;
+            if (i >= mine || at >= col_off[j + 1]) continue;
+            const uint32_t word = __float_as_uint(slot[t]);
+            const bool side_a = word & kSlotSideA;
+            float4 lpos, lrot;
+            load_link(final_buffer, word & kSlotParent, lpos, lrot);
+            const uint32_t where = __float_as_uint(slot[7 * tasks + t]);
+            f3 axis = normalize(quat_rotate(lrot, at3(slot, 1, tasks, t)));
+            if (word & kSlotReversed) axis = -axis;
+            const f3 anchor = xyz(lpos) + quat_rotate(lrot, at3(slot, 4, tasks, t));
+            const f3 aa = at3(frame, 0, per, i), ab = at3(frame, 3, per, i);
+            const f3 xa = at3(frame, 6, per, i), xb = at3(frame, 9, per, i);
+            const f3 rp = aa - ab, ra = xa - xb;
+            const f3 ea = side_a ? aa : ab, ex = side_a ? xa : xb;
+            const float sign = side_a ? 1.0f : -1.0f;
+            const f3 pd = cross(axis, ea - anchor) * sign;
+            const f3 ad = cross(axis, ex) * sign;
+            put3(col0, 0, S, at, pd);
+            put3(col0, 3, S, at, ad);
+            float g = __int_as_float(0x7fffffff), d = 0.0f;   // NaN: no contribution
+            if (frame[12 * per + i] != 0.0f) {
+                const float gg = dot(rp, pd) + 1.0f * dot(ra, ad), dd = dot(pd, pd) + 1.0f * dot(ad, ad);
+                if (gg == gg && dd == dd) {
+                    g = gg;
+                    d = dd;
+                } else {
+                    atomicOr(flags, MK_INVALID_NUMERIC_FLAG);
+                }
+            }
+            sg0[where] = g;
+            sd0[where] = d;
+        }
+        cluster_sync(blocks);
+        um = ud = 0u;
+        for (uint32_t r = 0; r < blocks; ++r) {
+            um = max(um, all_max[2 * r]);
+            ud = max(ud, all_max[2 * r + 1]);
+        }
+        if (tid == 0) s_max[0] = s_max[1] = 0u;
+        if (!(um > 10u || ud > 1000u)) {   // every block takes the same branch
+            done = 1;
+            break;
+        }
+        ++steps;
+        if (rank == 0) {
+        // ---- per coordinate: gradient and diagonal in the serial accumulation order
+        float grad[kBlockChunks], diag[kBlockChunks];
+#pragma unroll
+        for (uint32_t c = 0; c < kBlockChunks; ++c) {
+            const uint32_t q = c * kDotChunk + tid;
+            float g = 0.0f, d = 0.0f;
+            if (q < NQ)
+                for (uint32_t i = off[q]; i < off[q + 1]; ++i) {
+                    const float v = sg[i];
+                    if (v == v) { g += v; d += sd[i]; }
+                }
+            grad[c] = g;
+            diag[c] = d;
+        }
+        float sol[kBlockChunks], res[kBlockChunks], dir[kBlockChunks], pre[kBlockChunks], op[kBlockChunks];
+        if constexpr (!kPcg) {   // solve_closure_pcg (closure.wgsl:333-427)
+#pragma unroll
+            for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                const uint32_t q = c * kDotChunk + tid;
+                sol[c] = 0.0f;
+                res[c] = pre[c] = 0.0f;
+                if (diag[c] > 1.0e-12f) {
+                    res[c] = -grad[c];
+                    pre[c] = res[c] / diag[c];
+                }
+                dir[c] = pre[c];
+                if (q < NQ) dir_s[q] = dir[c];
+            }
+            float rz = dot_f(res, pre);
+            if (NQ == 0) __syncthreads();
+            for (uint32_t round = 0; round < kClosureRounds; ++round) {
+                products();   // dir_s was published by the barrier of the dot product or the round before
+                __syncthreads();
+#pragma unroll
+                for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                    const uint32_t q = c * kDotChunk + tid;
+                    op[c] = q < NQ ? run_sum(q) : 0.0f;
+                }
+                const float dop = dot_f(dir, op);
+                const float alpha = fabsf(dop) > 1.0e-20f ? rz / dop : 0.0f;
+#pragma unroll
+                for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                    sol[c] += alpha * dir[c];
+                    res[c] -= alpha * op[c];
+                    pre[c] = 0.0f;
+                    if (diag[c] > 1.0e-12f) pre[c] = res[c] / diag[c];
+                }
+                const float nrz = dot_f(res, pre);
+                const float beta = fabsf(rz) > 1.0e-20f ? nrz / rz : 0.0f;
+#pragma unroll
+                for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                    const uint32_t q = c * kDotChunk + tid;
+                    dir[c] = pre[c] + beta * dir[c];
+                    if (q < NQ) dir_s[q] = dir[c];
+                }
+                rz = nrz;
+                ++rounds;
+                __syncthreads();
+            }
+        } else {   // PCG to a residual
+            float* diag_s = s_dyn + L.diag;
+            float* res_s = s_dyn + L.res;
+            float* z_s = s_dyn + L.z;
+            const uint32_t* cqs = reinterpret_cast<const uint32_t*>(s_dyn + L.cqs);
+            const uint32_t* loop_off = reinterpret_cast<const uint32_t*>(s_dyn + L.loop_off);
+            const uint32_t* loop_q = reinterpret_cast<const uint32_t*>(s_dyn + L.loop_q);
+            float* lf = s_dyn + L.l;   // packed lower triangles, entry-major
+            const uint32_t loops = p.loops;
+            const bool loop_blocks = p.precond == MK_PRECOND_BLOCK_JACOBI;
+#pragma unroll
+            for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                const uint32_t q = c * kDotChunk + tid;
+                sol[c] = 0.0f;
+                res[c] = -grad[c];
+                if (q < NQ) {
+                    diag_s[q] = diag[c];
+                    res_s[q] = res[c];
+                }
+            }
+            if (loop_blocks) {   // couplings of each loop's coordinates (closure_coupling), one entry per thread
+                constexpr uint32_t kOff = kLoopPiece * (kLoopPiece - 1) / 2;
+                for (uint32_t e = tid; e < loops * kOff; e += nt) {
+                    const uint32_t lp = e / kOff;
+                    uint32_t j = e % kOff, i = 1;
+                    while (j >= i) { j -= i; ++i; }   // (i, j): row i > column j
+                    const uint32_t o = loop_off[lp], n = loop_off[lp + 1] - o;
+                    if (i >= n) continue;
+                    const uint32_t a = loop_q[o + i], c = loop_q[o + j];
+                    float r = 0.0f;
+                    for (uint32_t x = off[a]; x < off[a + 1]; ++x) {
+                        const uint32_t sa = cqs[x];
+                        const uint32_t ka = qi[sa] >> 16;
+                        for (uint32_t y = off[c]; y < off[c + 1]; ++y) {
+                            const uint32_t sb = cqs[y];
+                            if (ka != qi[sb] >> 16) continue;
+                            r += dot(at3(col, 0, S, sa), at3(col, 0, S, sb)) +
+                                 1.0f * dot(at3(col, 3, S, sa), at3(col, 3, S, sb));
+                        }
+                    }
+                    lf[(i * (i + 1) / 2 + j) * loops + lp] = r;
+                }
+            }
+            __syncthreads();
+            if (loop_blocks && tid < loops) {   // Cholesky with a ridge; a failed pivot leaves the block diagonal
+                const uint32_t o = loop_off[tid], n = loop_off[tid + 1] - o;
+                float a[kPieceEntries], dg[kLoopPiece];
+                float mean = 0.0f;
+#pragma unroll
+                for (uint32_t i = 0; i < kLoopPiece; ++i) {
+                    dg[i] = i < n ? diag_s[loop_q[o + i]] : 0.0f;
+                    if (i < n) mean += dg[i];
+                }
+                mean = n ? mean / (float)n : 0.0f;
+#pragma unroll
+                for (uint32_t i = 0; i < kLoopPiece; ++i)
+#pragma unroll
+                    for (uint32_t j = 0; j <= i; ++j) {
+                        const uint32_t e = i * (i + 1) / 2 + j;
+                        a[e] = i >= n ? 0.0f : i == j ? dg[i] + 1.0e-6f * mean : lf[e * loops + tid];
+                    }
+                bool ok = mean > 1.0e-12f;
+#pragma unroll
+                for (uint32_t j = 0; j < kLoopPiece; ++j) {
+                    if (j < n && ok) {
+                        float dj = a[j * (j + 1) / 2 + j];
+#pragma unroll
+                        for (uint32_t k = 0; k < j; ++k) dj -= a[j * (j + 1) / 2 + k] * a[j * (j + 1) / 2 + k];
+                        if (!(dj > 0.0f)) {
+                            ok = false;
+                        } else {
+                            const float ljj = sqrtf(dj);
+                            a[j * (j + 1) / 2 + j] = ljj;
+#pragma unroll
+                            for (uint32_t i = j + 1; i < kLoopPiece; ++i) {
+                                if (i < n) {
+                                    float v = a[i * (i + 1) / 2 + j];
+#pragma unroll
+                                    for (uint32_t k = 0; k < j; ++k)
+                                        v -= a[i * (i + 1) / 2 + k] * a[j * (j + 1) / 2 + k];
+                                    a[i * (i + 1) / 2 + j] = v / ljj;
+                                }
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (uint32_t i = 0; i < kLoopPiece; ++i)
+#pragma unroll
+                    for (uint32_t j = 0; j <= i; ++j) {
+                        const uint32_t e = i * (i + 1) / 2 + j;
+                        float v = a[e];
+                        if (!ok) v = i == j ? (dg[i] > 1.0e-12f ? sqrtf(dg[i]) : 0.0f) : 0.0f;
+                        if (i < n) lf[e * loops + tid] = v;   // read by this thread only
+                    }
+            }
+            // pre = M^-1 res (precond_apply); res_s is published, z_s free
+            auto precondition = [&]() {
+                if (!loop_blocks) {
+#pragma unroll
+                    for (uint32_t c = 0; c < kBlockChunks; ++c) pre[c] = diag[c] > 1.0e-12f ? res[c] / diag[c] : 0.0f;
+                    return;
+                }
+                if (tid < loops) {
+                    const uint32_t o = loop_off[tid], n = loop_off[tid + 1] - o;
+                    float y[kLoopPiece];
+#pragma unroll
+                    for (uint32_t i = 0; i < kLoopPiece; ++i) {
+                        y[i] = 0.0f;
+                        if (i < n) {
+                            float v = res_s[loop_q[o + i]];
+#pragma unroll
+                            for (uint32_t k = 0; k < i; ++k) v -= lf[(i * (i + 1) / 2 + k) * loops + tid] * y[k];
+                            const float lii = lf[(i * (i + 1) / 2 + i) * loops + tid];
+                            y[i] = lii > 0.0f ? v / lii : 0.0f;
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t x = kLoopPiece; x > 0; --x) {
+                        const uint32_t i = x - 1;
+                        if (i < n) {
+                            float v = y[i];
+#pragma unroll
+                            for (uint32_t k = i + 1; k < kLoopPiece; ++k)
+                                if (k < n) v -= lf[(k * (k + 1) / 2 + i) * loops + tid] * y[k];
+                            const float lii = lf[(i * (i + 1) / 2 + i) * loops + tid];
+                            y[i] = lii > 0.0f ? v / lii : 0.0f;
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t i = 0; i < kLoopPiece; ++i)
+                        if (i < n) z_s[loop_q[o + i]] = y[i];
+                }
+                __syncthreads();
+#pragma unroll
+                for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                    const uint32_t q = c * kDotChunk + tid;
+                    pre[c] = q < NQ ? z_s[q] : 0.0f;
+                }
+            };
+            precondition();
+#pragma unroll
+            for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                const uint32_t q = c * kDotChunk + tid;
+                dir[c] = pre[c];
+                if (q < NQ) dir_s[q] = dir[c];
+            }
+            double rz = dot_d(res, pre);
+            const double rr0 = dot_d(res, res);
+            double rr = rr0;
+            const double tol2 = (double)p.closure_tol * (double)p.closure_tol;
+            uint32_t it = 0;
+            while (it < p.closure_max_it && rr > tol2 * rr0) {
+                products();
+                __syncthreads();
+#pragma unroll
+                for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                    const uint32_t q = c * kDotChunk + tid;
+                    op[c] = q < NQ ? run_sum(q) : 0.0f;
+                }
+                const double pq = dot_d(dir, op);
+                const float alpha = fabs(pq) > 1.0e-30 ? (float)(rz / pq) : 0.0f;
+#pragma unroll
+                for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                    const uint32_t q = c * kDotChunk + tid;
+                    sol[c] += alpha * dir[c];
+                    res[c] -= alpha * op[c];
+                    if (q < NQ) res_s[q] = res[c];
+                }
+                rr = dot_d(res, res);
+                ++it;
+                if (rr <= tol2 * rr0) break;
+                precondition();
+                const double nrz = dot_d(res, pre);
+                const float beta = fabs(rz) > 1.0e-300 ? (float)(nrz / rz) : 0.0f;
+#pragma unroll
+                for (uint32_t c = 0; c < kBlockChunks; ++c) {
+                    const uint32_t q = c * kDotChunk + tid;
+                    dir[c] = pre[c] + beta * dir[c];
+                    if (q < NQ) dir_s[q] = dir[c];
+                }
+                rz = nrz;
+                __syncthreads();
+            }
+            ++newton;
+            iterations += it;
+            const double rel = rr0 > 0.0 ? sqrt(rr / rr0) : 0.0;
+            if (rel > worst) worst = rel;
+        }
+        // ---- step the coordinates (closure.wgsl:416-427), to their joints' bodies
+#pragma unroll
+        for (uint32_t c = 0; c < kBlockChunks; ++c) {
+            if (c * kDotChunk + tid >= NQ) continue;
+            const float stp = clampf(0.35f * sol[c], -0.2f, 0.2f);
+            if (stp == stp) angle[c] += stp;
+            else atomicOr(flags, MK_INVALID_NUMERIC_FLAG);
+            *cluster_map(angle_s + (child[c] >> shift), child[c] & rank_mask) = angle[c];
+        }
+        }
+        cluster_sync(blocks);
+        // ---- forward kinematics of the closure components (prepare_link, jump_link), a body per thread
+        float4 lp = make_float4(0, 0, 0, 0), lr = make_float4(0, 0, 0, 1);
+        uint32_t up = parent | (root ? kLinkDone : 0u);
+        if (has_body) {
+            if (!root) {
+                const float h = (fk[13 * rows + tid] * angle_s[tid]) * 0.5f;
+                const f3 v = at3(fk, 0, rows, tid) * sin_cr(h);
+                const float4 bind = f4(at3(fk, 9, rows, tid), fk[12 * rows + tid]);
+                lr = quat_multiply(make_float4(v.x, v.y, v.z, cos_cr(h)), bind);
+                lp = f4(at3(fk, 3, rows, tid) - quat_rotate(lr, at3(fk, 6, rows, tid)), 0.0f);
+            }
+            link_pos[tid] = f4(xyz(lp), __uint_as_float(up));
+            link_rot[tid] = lr;
+        }
+        cluster_sync(blocks);
+        uint32_t src = 0;
+        for (uint32_t r = 0; r < p.jump_rounds; ++r) {
+            if (has_body) {
+                if (!(up & kLinkDone)) {
+                    float4 up_pos, up_rot;
+                    load_link(src, up, up_pos, up_rot);
+                    lp = f4(xyz(up_pos) + quat_rotate(up_rot, xyz(lp)), 0.0f);
+                    lr = normalize4(quat_multiply(up_rot, lr));
+                    up = __float_as_uint(up_pos.w);
+                }
+                link_pos[(src ^ 1u) * rows + tid] = f4(xyz(lp), __uint_as_float(up));
+                link_rot[(src ^ 1u) * rows + tid] = lr;
+            }
+            cluster_sync(blocks);
+            src ^= 1u;
+        }
+    }
+    // ---- results: the links, the coordinates and the columns of the last evaluated step
+    if (steps && has_body) {
+        const float4 lp = link_pos[final_buffer * rows + tid], lr = link_rot[final_buffer * rows + tid];
+        const uint32_t up = __float_as_uint(lp.w);
+        st_link(m.links_final, body,
+                {f4(xyz(lp), 0.0f), lr, make_uint4(m.cb_bodies[up & ~kLinkDone], up >> 31, 0u, 0u)});
+    }
+    if (rank == 0) {
+        if (!kPcg && steps) {
+            for (uint32_t c = tid; c < Q; c += nt) m.coords[c].angle += 0.0f;   // those off the closure branches
+            __syncthreads();
+        }
+#pragma unroll
+        for (uint32_t c = 0; c < kBlockChunks; ++c)
+            if (steps && c * kDotChunk + tid < NQ) m.coords[coord[c]].angle = angle[c];
+        for (uint32_t at = tid; at < S; at += nt) {
+            const uint32_t k = qi[at] >> 16, row = m.cl_order[k];
+            const uint32_t sl = m.cq_slots[pos[at]];
+            m.slot_v[2 * sl] = f4(at3(col, 0, S, at), __uint_as_float(m.cq_coords[qi[at] & 0xffffu]));
+            m.slot_v[2 * sl + 1] = f4(at3(col, 3, S, at), kPcg ? __uint_as_float(row) : 0.0f);
+        }
+    }
+    cluster_sync(blocks);   // no block leaves while another may still read its links
+    if (rank == 0 && tid == 0) {
+        if constexpr (kPcg) {
+            *m.cstate = ClosureState{done, done ? 0u : p.blocks, newton, iterations, 0u, 0u, worst};
+        } else {
+            atomicAdd(&b.diag->reserved_b, steps);
+            atomicAdd(&b.diag->reserved_c, rounds);
+        }
+    }
+}
+
 // --------------------------------------------------------------- launches
 static inline uint32_t nblocks(uint32_t n) { return (n + kMBlock - 1) / kMBlock; }
 
@@ -1682,7 +2623,14 @@ static cudaError_t forward_kinematics(MechBuffers& m, const MechParams& p, cudaS
     return cudaGetLastError();
 }
 
-static cudaError_t reconstruct(MechBuffers& m, const StepBuffers& b, cudaStream_t s) {
+static cudaError_t reconstruct(MechBuffers& m, const StepBuffers& b, const MechParams& p, cudaStream_t s) {
+    if (p.walk_levels) {
+        const uint32_t count = m.level_offsets[m.level_count];
+        k_reconstruct_rows<<<nblocks(count), kMBlock, 0, s>>>(b, m, count);
+        k_reconstruct_walk<<<1, kWalkThreads, kWalkSmem, s>>>(b, m, m.level_count, count);
+        k_reconstruct_store<<<nblocks(count), kMBlock, 0, s>>>(b, m, count);
+        return cudaGetLastError();
+    }
     for (uint32_t l = 1; l < m.level_count; ++l) {
         const uint32_t begin = m.level_offsets[l], end = m.level_offsets[l + 1];
         if (end > begin) k_reconstruct_level<<<nblocks(end - begin), kMBlock, 0, s>>>(b, m, begin, end);
@@ -1700,6 +2648,67 @@ constexpr uint32_t kGridClosures = 512;
 static uint32_t g_closure_grid = 0;
 void set_closure_grid(uint32_t mode) { g_closure_grid = mode <= 2u ? mode : 0u; }
 uint32_t closure_grid_mode() { return g_closure_grid; }
+
+// Launch shape of the one-block closure solve (blocks of its cluster, threads,
+// dynamic shared memory); false where the system does not fit it.  A thread per
+// coordinate (two above 1,024), per closure body of a block and per closure of
+// a block; the run positions and closures of the slots are 16-bit.  A cluster
+// where a block would walk its slots or bodies in several rounds.
+struct ClosureShape {
+    uint32_t blocks, threads, bytes;
+};
+static bool closure_block_shape(const MechParams& p, ClosureShape& sh) {
+    const bool pcg = pcg_residual_mode(p);
+    if (!p.block_solve) return false;
+    if ((uint64_t)p.closure_depth * p.closures > 64u * kClosureSmem) return false;   // 32-bit word offsets
+    if (pcg && p.precond != MK_PRECOND_BLOCK_JACOBI && p.precond != MK_PRECOND_DIAGONAL) return false;
+    sh.blocks = std::max(p.slots, p.closure_bodies) > kClosureSpread ? kClosureCluster : 1u;
+    const uint32_t rows = (p.closure_bodies + sh.blocks - 1) / sh.blocks;
+    if (rows > kClosureThreads) return false;
+    const uint32_t want = std::max({rows, std::min(p.closure_coords, kClosureThreads), 128u});
+    sh.threads = p.closure_coords > kDotChunk ? kClosureThreads : std::min(kClosureThreads, (want + 31u) & ~31u);
+    sh.bytes = 4u * closure_layout(p, sh.blocks, pcg).words;
+    return sh.bytes <= kClosureSmem;
+}
+
+// Dynamic shared memory of the one-block closure solves, set once per device
+// (outside stream capture: at handle creation).
+cudaError_t mechanism_prepare() {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load() & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(k_reconstruct_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem);
+    for (const void* k : {(const void*)k_closure_block<false, kClosureFew>, (const void*)k_closure_block<true, kClosureFew>,
+                          (const void*)k_closure_block<false, kClosureThreads>,
+                          (const void*)k_closure_block<true, kClosureThreads>})
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClosureSmem);
+    if (e == cudaSuccess) done.fetch_or(bit);
+    return e;
+}
+
+static cudaError_t launch_closure_block(const MechBuffers& m, const StepBuffers& b, const MechParams& p,
+                                        const ClosureShape& sh, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sh.blocks);
+    cfg.blockDim = dim3(sh.threads);
+    cfg.dynamicSmemBytes = sh.bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = sh.blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (sh.threads <= kClosureFew)
+        return pcg_residual_mode(p) ? cudaLaunchKernelEx(&cfg, k_closure_block<true, kClosureFew>, b, m, p)
+                                    : cudaLaunchKernelEx(&cfg, k_closure_block<false, kClosureFew>, b, m, p);
+    return pcg_residual_mode(p) ? cudaLaunchKernelEx(&cfg, k_closure_block<true, kClosureThreads>, b, m, p)
+                                : cudaLaunchKernelEx(&cfg, k_closure_block<false, kClosureThreads>, b, m, p);
+}
 
 // One co-resident 1,024-thread block per SM for the grid-wide closure kernels
 // (cooperative launch: they sync with grid barriers).  `step` is passed when
@@ -1731,6 +2740,12 @@ static cudaError_t launch_grid(const void* kernel, const StepBuffers& b, const M
     return cudaLaunchKernelExC(&cfg, kernel, step == kNoStep ? args3 : args4);
 }
 
+cudaError_t refresh_closure_columns(const MechBuffers& m, const MechParams& p, cudaStream_t s) {
+    if (p.closures == 0 || !p.wide_closures || pcg_residual_mode(p)) return cudaSuccess;
+    k_closure_columns<<<std::min(4096u, (p.closures + 7u) / 8u), kMBlock, 0, s>>>(m, p);
+    return cudaGetLastError();
+}
+
 void mechanism_tick_clears(const MechBuffers& m, const MechParams& p, void** ptr, uint64_t* bytes, uint32_t* count) {
     *count = 0;
     if (p.closures == 0) return;
@@ -1751,7 +2766,10 @@ cudaError_t enqueue_mechanism(MechBuffers& m, const StepBuffers& b, const MechPa
     if ((e = forward_kinematics(m, p, s)) != cudaSuccess) return e;
     const uint32_t mode = g_closure_grid;
     const bool grid = p.closures > 0 && (mode == 2u || (mode == 0u && p.closures >= kGridClosures));
-    if (pcg_residual_mode(p)) {
+    ClosureShape shape;
+    if (mode != 2u && closure_block_shape(p, shape)) {
+        if ((e = launch_closure_block(m, b, p, shape, s)) != cudaSuccess) return e;
+    } else if (pcg_residual_mode(p)) {
         for (uint32_t step = 0; step < kClosureSteps; ++step) {
             if (grid) {
                 if ((e = launch_grid((const void*)k_closure_eval<true>, b, m, p, step, s)) != cudaSuccess) return e;
@@ -1777,7 +2795,7 @@ cudaError_t enqueue_mechanism(MechBuffers& m, const StepBuffers& b, const MechPa
         }
     }
     k_publish<<<nblocks(p.body_count), kMBlock, 0, s>>>(b, m, p);
-    if ((e = reconstruct(m, b, s)) != cudaSuccess) return e;
+    if ((e = reconstruct(m, b, p, s)) != cudaSuccess) return e;
     // the published poses hold for the rest of the tick: the projection passes
     // during and after the contact solve share one cache
     return bearing_cache(m, b, p, s);
@@ -1803,7 +2821,7 @@ cudaError_t enqueue_post_contact(MechBuffers& m, const StepBuffers& b, const Mec
         for (uint32_t it = 0; it < std::max(1u, p.iterations); ++it)
             if ((e = bearing_projection_iteration(m, b, p, s)) != cudaSuccess) return e;
     k_capture_coordinates<<<nblocks(p.body_count), kMBlock, 0, s>>>(b, m, p);
-    if (!p.has_dynamic_root) return reconstruct(m, b, s);
+    if (!p.has_dynamic_root) return reconstruct(m, b, p, s);
     return cudaGetLastError();
 }
 
@@ -1836,9 +2854,3 @@ uint64_t mechanism_mlp_scratch_bytes(const MechParams& p) {
 }
 
 }  // namespace mk
-cudaError_t refresh_closure_columns(const MechBuffers& m, const MechParams& p, cudaStream_t s) {
-    if (p.closures == 0 || !p.wide_closures || pcg_residual_mode(p)) return cudaSuccess;
-    k_closure_columns<<<std::min(4096u, (p.closures + 7u) / 8u), kMBlock, 0, s>>>(m, p);
-    return cudaGetLastError();
-}
-

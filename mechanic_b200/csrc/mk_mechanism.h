@@ -28,6 +28,9 @@ struct MechParams {
     uint32_t wide_closures = 0;      // closures average 32 slots or more: a warp walks each
     uint32_t closure_coords = 0;     // distinct coordinates on closure branches
     uint32_t closure_bodies = 0;     // bodies of components that contain a closure
+    uint32_t closure_depth = 0;      // most slots of a closure
+    uint32_t walk_levels = 0;        // depth levels of a tree whose velocities one block reconstructs (0: a launch each)
+    uint32_t block_solve = 0;        // the one-block closure solve's tables exist
     // MK_CLOSURE_PCG_RESIDUAL
     float closure_tol = 1.0e-5f;     // relative PCG residual per Newton step
     uint32_t closure_max_it = 256;   // PCG iterations per Newton step
@@ -63,10 +66,21 @@ struct MechBuffers {
     uint32_t* level_bodies = nullptr;
     const uint32_t* level_offsets = nullptr;    // host memory owned by the handle, level_count + 1 entries
     uint32_t level_count = 0;
+    uint32_t* level_begin = nullptr;            // one-block walk: level_offsets on the device,
+    uint32_t* level_parent = nullptr;           // per level body: its parent's place in the level before (level 1: the root),
+    float4* level_rows = nullptr;               // 3 per level body: the velocity-independent parts
     // closure loop
     uint32_t* cl_bearings = nullptr;            // closure bearing rows
     uint32_t* cl_slot_off = nullptr;            // closures + 1: slots of closure k (branch a, then branch b)
     uint32_t* cl_split = nullptr;               // first branch-b slot of closure k
+    uint32_t* cl_order = nullptr;               // closures by falling slot count
+    uint32_t* cl_columns = nullptr;             // most slots + 1: first entry of the j-th slots, closures in that order
+    uint32_t* col_coord = nullptr;              // per slot in column order: coordinate's position | closure's << 16,
+    uint32_t* col_pos = nullptr;                // and its place in the coordinates' runs
+    uint32_t* cl_places = nullptr;              // places in cb_bodies: of each closure's bodies a and b,
+    uint32_t* slot_parent = nullptr;            // of each slot's parent body,
+    uint32_t* cq_child = nullptr;               // of the child body of each closure coordinate's joint,
+    uint32_t* cb_parents = nullptr;             // of each closure body's parent (its own for a root)
     uint32_t* slot_body = nullptr;              // child body of the joint of each slot
     uint32_t* cq_coords = nullptr;              // coordinates on closure branches (ascending)
     uint32_t* cq_off = nullptr;                 // closure_coords + 1: CSR into cq_slots
@@ -84,6 +98,7 @@ struct MechBuffers {
     float* diag = nullptr;                      // Q
     float* pcg = nullptr;                       // 5 x Q: sol, res, pre, dir, op (closure.wgsl:51-60)
     uint32_t* grid_barrier = nullptr;           // arrival word of the grid-wide closure loop (zero at rest)
+    uint32_t* columns_stale = nullptr;          // wide systems: the last step converged before its columns were needed
     uint32_t* loop_state = nullptr;             // 12 steps x 2: largest residuals (um, udeg), zeroed per tick
     float* chunk_part = nullptr;                // 2 x chunks of 1,024 closure coordinates: dot-product sums
     double* chunk_part_d = nullptr;             // the same in FP64 (closure PCG to a residual)
@@ -98,7 +113,6 @@ struct MechBuffers {
     float* blk_hist = nullptr;                  // 12 steps x blocks x 3: outputs used at each Newton step
     float* probe = nullptr;                     // 2 x Q: A * ones, A * alternating signs
     ClosureState* cstate = nullptr;
-    uint32_t* columns_stale = nullptr;          // wide systems: the last step converged before its columns were needed
     float* precond_params = nullptr;            // preconditioner network parameters (mlp::kParams)
     uint32_t* loop_off = nullptr;               // loops + 1: offsets into loop_q
     uint32_t* loop_q = nullptr;                 // closure-coordinate positions of each loop block
@@ -110,12 +124,14 @@ MechParams make_mech_params(const MkCreation* cr, const StepParams& p, uint32_t 
                             float closure_tol, uint32_t closure_max_it, uint32_t precond);
 // Host-side closure topology and depth levels; fills the counts in `p`.
 struct MechTopology {
-    std::vector<uint32_t> level_bodies, level_offsets;
+    std::vector<uint32_t> level_bodies, level_offsets, level_parent;
     std::vector<uint32_t> cl_bearings, cl_slot_off, cl_split, slot_body, cq_coords, cq_off, cq_slots, cb_bodies;
+    std::vector<uint32_t> cl_order, cl_columns, col_coord, col_pos, cl_places, slot_parent, cq_child, cb_parents;
     std::vector<uint32_t> slot_closure, slot_pos, long_q, long_chunk_off, chunk_long;
     std::vector<uint32_t> loop_off, loop_q;
 };
 MechTopology derive_topology(const MkCreation* cr, MechParams& p);
+cudaError_t mechanism_prepare();   // per-device kernel attributes; call outside stream capture
 // Reference-mode closure loop: 0 = by size, 1 = one block, 2 = the whole grid.
 void set_closure_grid(uint32_t mode);
 uint32_t closure_grid_mode();
@@ -127,6 +143,8 @@ bool upload_mechanism(MechBuffers& m, const MechParams& p, const MechTopology& t
                       cudaStream_t s, MkError* err);
 cudaError_t enqueue_mechanism(MechBuffers& m, const StepBuffers& b, const MechParams& p, cudaStream_t s);
 bool pcg_residual_mode(const MechParams& p);
+// Brings slot_v up to date before it is read (reference loop, wide systems).
+cudaError_t refresh_closure_columns(const MechBuffers& m, const MechParams& p, cudaStream_t s);
 cudaError_t enqueue_contact_solver_with_bearings(MechBuffers& m, const StepBuffers& b, const StepParams& sp,
                                                  const MechParams& p, const StepLaunch& l, int parity, cudaStream_t s);
 cudaError_t enqueue_post_contact(MechBuffers& m, const StepBuffers& b, const MechParams& p, cudaStream_t s);
@@ -139,5 +157,3 @@ void read_mechanism_readback(const MechBuffers& m, const MechParams& p, const Gp
 uint64_t mechanism_mlp_scratch_bytes(const MechParams& p);
 
 }  // namespace mk
-// Brings slot_v up to date before it is read (reference loop, wide systems).
-cudaError_t refresh_closure_columns(const MechBuffers& m, const MechParams& p, cudaStream_t s);
