@@ -318,7 +318,6 @@ cudaError_t enqueue_tick(MkHandle* h, int parity, bool capturing) {
             mk::sort_clear_region(b.pair_sort_scratch, h->pair_capacity, 2 * h->params.pair_shift, false, &r, &rb);
             z.add(r, rb);
         }
-        if (h->mechanism_active) z.add(h->mech.deltas, 24ull * std::max(h->B, 1u));
         if (h->mechanism_active) {   // the closure loop's barrier word and per-step maxima
             void* mp[2];
             uint64_t mb[2];

@@ -253,11 +253,16 @@ cudaError_t launch_contact_solver(const StepBuffers& b, const StepParams& p, con
 constexpr uint32_t MK_HEAVY_SCATTER = 1, MK_HEAVY_GATHER = 2, MK_HEAVY_SPLIT = 3;
 void set_heavy_solve_form(uint32_t form);   // 0 = the default form
 uint32_t heavy_solve_form();
-// Contact iterations as separate launches with a hook after each velocity
-// apply (bearing projection of mechanisms with a dynamic root).
-cudaError_t launch_contact_solver_stepwise(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
-                                           bool serial, const std::function<cudaError_t(bool)>& after_apply,
-                                           cudaStream_t s);
+// Contact iterations as separate launches, for ticks that interleave bearing
+// projection with them (mechanisms with a dynamic root).  Passes: `pass(it,
+// deltas, clear)` applies the iteration's deltas and projects, from velocity
+// buffers it & 1 into the other ones.  Serial: small mechanisms.
+cudaError_t launch_contact_solver_passes(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
+                                         float4* const* lin, float4* const* ang,
+                                         const std::function<cudaError_t(uint32_t, int32_t*, int32_t*)>& pass,
+                                         cudaStream_t s);
+cudaError_t launch_contact_solver_serial(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
+                                         const std::function<cudaError_t()>& after_apply, cudaStream_t s);
 cudaError_t launch_apply_impulse(const StepBuffers& b, uint32_t body, float3 point, float3 impulse,
                                  cudaStream_t s);
 cudaError_t launch_obb_sat(const float* boxes_a, const float* boxes_b, uint32_t count, float* np,

@@ -2,8 +2,8 @@
 //
 // Stage map (reference kernel -> this file), in the dispatch order of
 // device.rs:963-1155:
-//   articulated.wgsl project_bearing_velocities :287-316   -> k_project_bearings
-//   articulated.wgsl apply_velocity_deltas :318-337        -> k_apply_mdeltas
+//   articulated.wgsl project_bearing_velocities :287-316
+//   and apply_velocity_deltas :318-337                     -> k_bearing_pass
 //   articulated.wgsl advance_coordinates :366-415          -> k_advance_coordinates
 //   mechanism.wgsl prepare_links / jump_* :72-149          -> k_prepare_links / k_jump (list-restricted)
 //   closure.wgsl evaluate / finalize / solve_closure_pcg   -> k_closure_loop (one block, all 12 Newton steps)
@@ -32,6 +32,7 @@
 namespace mk {
 
 constexpr uint32_t kMBlock = 256;
+constexpr uint32_t kPassBlock = 128;       // threads of a bearing projection block
 constexpr uint32_t kClosureThreads = 1024;
 constexpr uint32_t kClosureSteps = 12;     // device.rs:974
 constexpr uint32_t kClosureRounds = 8;     // closure.wgsl:356
@@ -41,7 +42,7 @@ constexpr uint32_t kMaxLoop = 8;           // coordinates of one per-loop precon
 // singular (its Cholesky then hangs on the ridge alone, and the preconditioned
 // iteration diverged on 16-body loops).  Loops are cut into pieces of 5.
 constexpr uint32_t kLoopPiece = 5;
-constexpr uint32_t kBearingCache = 9;     // float4 per bearing in the projection cache
+constexpr uint32_t kSideRows = 6;         // float4 per bearing side in the projection cache
 constexpr uint32_t kWalkWidth = 4096;      // most bodies of a level of k_reconstruct_walk (two in shared memory)
 constexpr uint32_t kLongList = 256;        // slot runs longer than this are summed in chunks of this many
 
@@ -137,6 +138,57 @@ MechTopology derive_topology(const MkCreation* cr, MechParams& p) {
     const uint32_t B = cr->body_count;
     if (cr->max_depth == 0 || !cr->mechanism_bodies) return t;
     const GpuMechanismBody* mb = cr->mechanism_bodies;
+    // projection passes: bodies with bearings first; their bearing sides in lists of whole warps, a body's sides
+    // inside one warp (bodies of more than 32 in a list of their own)
+    {
+        std::vector<uint32_t> off(B + 1ull, 0u);
+        for (uint32_t j = 0; j < cr->bearing_count; ++j)
+            for (int side = 0; side < 2; ++side)
+                if (cr->bearings[j].metadata[side] < B) ++off[cr->bearings[j].metadata[side] + 1u];
+        for (uint32_t i = 0; i < B; ++i)
+            if (off[i + 1]) t.pass_bodies.push_back(i);
+        p.bearing_bodies = (uint32_t)t.pass_bodies.size();
+        for (uint32_t i = 0; i < B; ++i)
+            if (!off[i + 1]) t.pass_bodies.push_back(i);
+        for (uint32_t i = 0; i < B; ++i) off[i + 1] += off[i];
+        std::vector<uint2> entries(off[B]);   // 2 bearing + side, the other body
+        std::vector<uint32_t> at(off.begin(), off.end() - 1);
+        for (uint32_t j = 0; j < cr->bearing_count; ++j)
+            for (uint32_t side = 0; side < 2; ++side) {
+                const uint32_t body = cr->bearings[j].metadata[side], other = cr->bearings[j].metadata[side ^ 1u];
+                if (body < B) entries[at[body]++] = make_uint2(2u * j + side, std::min(other, B - 1u));
+            }
+        t.side_place.resize(cr->bearing_count, make_uint2(0u, 0u));
+        auto put_side = [&](const uint2& en) {
+            (en.x & 1u ? t.side_place[en.x >> 1].y : t.side_place[en.x >> 1].x) = (uint32_t)t.side_entries.size();
+            t.side_entries.push_back(make_uint2(en.x & 1u, en.y));
+        };
+        auto pad_to = [&](size_t n) {
+            t.side_body.resize(n, kInvalid);
+            t.side_entries.resize(n, make_uint2(0u, 0u));
+        };
+        for (uint32_t i = 0; i < p.bearing_bodies; ++i) {
+            const uint32_t body = t.pass_bodies[i], n = off[body + 1] - off[body];
+            if (n > 32u) {
+                t.hub_bodies.push_back(body);
+                continue;
+            }
+            const size_t used = t.side_body.size() % 32u;
+            if (used + n > 32u) pad_to(t.side_body.size() + 32u - used);
+            t.side_body.insert(t.side_body.end(), n, body);
+            for (uint32_t q = off[body]; q < off[body + 1]; ++q) put_side(entries[q]);
+            p.most_sides = std::max(p.most_sides, n);
+        }
+        pad_to((t.side_body.size() + kPassBlock - 1) / kPassBlock * kPassBlock);
+        p.padded_sides = (uint32_t)t.side_body.size();
+        t.hub_off.push_back(0u);
+        for (uint32_t body : t.hub_bodies) {
+            for (uint32_t q = off[body]; q < off[body + 1]; ++q) put_side(entries[q]);
+            t.hub_off.push_back((uint32_t)t.side_entries.size() - p.padded_sides);
+        }
+        p.hub_bodies = (uint32_t)t.hub_bodies.size();
+        p.all_sides = (uint32_t)t.side_entries.size();
+    }
     // depth levels 1..max_depth (roots are skipped by the reconstruction)
     t.level_offsets.assign(cr->max_depth + 2, 0);
     for (uint32_t i = 0; i < B; ++i)
@@ -276,8 +328,13 @@ void carve_mechanism(MechBuffers& m, const MechParams& p, uint32_t B, uint32_t J
     m.preorder = u32(B);
     m.links_a = reinterpret_cast<GpuLinkState*>(take(sizeof(GpuLinkState) * (uint64_t)B));
     m.links_b = reinterpret_cast<GpuLinkState*>(take(sizeof(GpuLinkState) * (uint64_t)B));
-    m.deltas = reinterpret_cast<int32_t*>(take(24ull * B));
-    m.bear_cache = reinterpret_cast<float4*>(take(16ull * kBearingCache * (J ? J : 1)));
+    m.pass_bodies = u32(B);
+    m.side_body = u32(p.padded_sides);
+    m.side_entries = reinterpret_cast<uint2*>(take(8ull * std::max(1u, p.all_sides)));
+    m.side_place = reinterpret_cast<uint2*>(take(8ull * J));
+    m.side_cache = reinterpret_cast<float4*>(take(16ull * kSideRows * std::max(1u, p.all_sides)));
+    m.hub_bodies = u32(p.hub_bodies);
+    m.hub_off = u32(p.hub_bodies + 1ull);
     m.level_bodies = u32(B);
     if (p.walk_levels) {
         m.level_begin = u32(p.walk_levels + 1ull);
@@ -367,6 +424,12 @@ bool upload_mechanism(MechBuffers& m, const MechParams& p, const MechTopology& t
         }
         if (e == cudaSuccess) e = put(m.drives, d, s);
     }
+    if (e == cudaSuccess) e = put(m.pass_bodies, t.pass_bodies, s);
+    if (e == cudaSuccess) e = put(m.side_body, t.side_body, s);
+    if (e == cudaSuccess) e = put(m.side_entries, t.side_entries, s);
+    if (e == cudaSuccess) e = put(m.side_place, t.side_place, s);
+    if (e == cudaSuccess) e = put(m.hub_bodies, t.hub_bodies, s);
+    if (e == cudaSuccess) e = put(m.hub_off, t.hub_off, s);
     if (e == cudaSuccess) e = put(m.level_bodies, t.level_bodies, s);
     if (e == cudaSuccess && p.walk_levels) e = put(m.level_begin, t.level_offsets, s);
     if (e == cudaSuccess && p.walk_levels) e = put(m.level_parent, t.level_parent, s);
@@ -423,39 +486,6 @@ __device__ __forceinline__ f3 wii(const StepBuffers& b, uint32_t body, f3 v) {
 }
 __device__ __forceinline__ float inv_mass(const StepBuffers& b, uint32_t body) { return b.mass[4ull * body].x; }
 
-// One body's fixed-point deltas summed in registers: a row's contribution is
-// converted as add_mdelta does and the integer sums wrap as the atomics do,
-// so one atomic per component gives the same totals as one per row.
-struct MDelta {
-    uint32_t v[6];
-};
-__device__ __forceinline__ void mdelta_add(MDelta& acc, f3 l, f3 a) {
-    const float s = 1048576.0f;
-    acc.v[0] += (uint32_t)fixed_i32(l.x * s);
-    acc.v[1] += (uint32_t)fixed_i32(l.y * s);
-    acc.v[2] += (uint32_t)fixed_i32(l.z * s);
-    acc.v[3] += (uint32_t)fixed_i32(a.x * s);
-    acc.v[4] += (uint32_t)fixed_i32(a.y * s);
-    acc.v[5] += (uint32_t)fixed_i32(a.z * s);
-}
-__device__ __forceinline__ void mdelta_flush(int32_t* deltas, uint32_t body, const MDelta& acc) {
-    int32_t* d = deltas + 6ull * body;
-#pragma unroll
-    for (int c = 0; c < 6; ++c)
-        if (acc.v[c]) atomicAdd(d + c, (int32_t)acc.v[c]);
-}
-
-__device__ __forceinline__ void add_mdelta(int32_t* deltas, uint32_t body, f3 l, f3 a) {   // :104-112
-    const float s = 1048576.0f;
-    int32_t* d = deltas + 6ull * body;
-    atomicAdd(d + 0, fixed_i32(l.x * s));
-    atomicAdd(d + 1, fixed_i32(l.y * s));
-    atomicAdd(d + 2, fixed_i32(l.z * s));
-    atomicAdd(d + 3, fixed_i32(a.x * s));
-    atomicAdd(d + 4, fixed_i32(a.y * s));
-    atomicAdd(d + 5, fixed_i32(a.z * s));
-}
-
 __device__ __forceinline__ void hinge_tangents(const StepBuffers& b, uint32_t a, uint32_t c, const GpuBearing& br,
                                                f3& ta, f3& tb) {
     const f3 axa = normalize(quat_rotate(b.rot[a], r3(br.local_axis_a)));
@@ -469,11 +499,15 @@ __device__ __forceinline__ void hinge_tangents(const StepBuffers& b, uint32_t a,
 // The parts of a bearing's five rows that depend on the poses only: they stay
 // fixed over a set of projection passes (the poses change at the forward
 // kinematics, not between passes), so they are computed once per set, with the
-// same expressions as the rows would compute them.  9 float4 per bearing:
-// {arm_a, 1/m_a} {arm_b, 1/m_b} {den0, den1, den2, -} {t_a, den3} {t_b, den4}
-// {I_a t_a} {I_b t_a} {I_a t_b} {I_b t_b}: arms of the three linear rows (world
-// axes), hinge tangents of the two angular rows, world inverse inertia products
-// and the rows' denominators.
+// same expressions as the rows would compute them.  Each of its two sides gets
+// its own copy, kSideRows float4 at the side's place in the passes' lists (an
+// array per row, so the passes read them coalesced: with 9 float4 per bearing,
+// 144 bytes apart, a pass of 198,009 bearings with contact deltas took 37 us,
+// with this 33 us):
+// {arm_a, 1/m own} {arm_b, den0} {t_a, den3} {t_b, den4} {I t_a own, den1}
+// {I t_b own, den2}: arms of the three linear rows (world axes), hinge tangents
+// of the two angular rows, the side's world inverse inertia products and the
+// rows' denominators.
 __global__ void __launch_bounds__(kMBlock) k_bearing_cache(StepBuffers b, MechBuffers m, MechParams p) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= p.bearing_count) return;
@@ -493,97 +527,182 @@ __global__ void __launch_bounds__(kMBlock) k_bearing_cache(StepBuffers b, MechBu
     const f3 ia3 = wii(b, a, ta), ib3 = wii(b, c, ta), ia4 = wii(b, a, tb), ib4 = wii(b, c, tb);
     den[3] = dot(ta, ia3 + ib3);
     den[4] = dot(tb, ia4 + ib4);
-    float4* o = m.bear_cache + (uint64_t)kBearingCache * j;
-    o[0] = f4(arm_a, ima);
-    o[1] = f4(arm_b, imb);
-    o[2] = make_float4(den[0], den[1], den[2], 0.0f);
-    o[3] = f4(ta, den[3]);
-    o[4] = f4(tb, den[4]);
-    o[5] = f4(ia3, 0.0f);
-    o[6] = f4(ib3, 0.0f);
-    o[7] = f4(ia4, 0.0f);
-    o[8] = f4(ib4, 0.0f);
-}
-
-// articulated.wgsl:114-155, 287-316
-// One bearing per group of kRowLanes lanes, one row per lane (three linear,
-// two angular); the rows' fixed-point deltas are summed over the group by
-// shuffles (integer sums: the same totals in any order) and one lane flushes
-// them.  Every row reads the velocities of before the pass (Jacobi); the
-// pose-only parts come from the set's bearing cache.
-constexpr uint32_t kRowLanes = 8;
-__global__ void __launch_bounds__(kMBlock) k_project_bearings(StepBuffers b, MechBuffers m, MechParams p) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t j = g / kRowLanes, row = g % kRowLanes;
-    const bool live = j < p.bearing_count;   // whole groups share this (the grid covers whole groups)
-    MDelta da{}, dc{};
-    uint32_t a = 0, c = 0;
-    if (live) {
-        const uint4 meta = *reinterpret_cast<const uint4*>(m.bearings[j].metadata);
-        a = meta.x;
-        c = meta.y;
-        const float4* cache = m.bear_cache + (uint64_t)kBearingCache * j;
-        if (row < 3) {
-            const float4 ca = __ldg(cache), cb = __ldg(cache + 1), cd = __ldg(cache + 2);
-            const f3 arm_a = xyz(ca), arm_b = xyz(cb);
-            const f3 va = xyz(b.lin[a]) + cross(xyz(b.ang[a]), arm_a);
-            const f3 vb = xyz(b.lin[c]) + cross(xyz(b.ang[c]), arm_b);
-            const f3 rel = vb - va;
-            const float ima = ca.w, imb = cb.w;
-            const f3 d = row == 0 ? mkf3(1, 0, 0) : row == 1 ? mkf3(0, 1, 0) : mkf3(0, 0, 1);
-            const float den = row == 0 ? cd.x : row == 1 ? cd.y : cd.z;
-            if (!(den <= 1.0e-12f)) {
-                const f3 imp = d * (0.5f * dot(rel, d) / den);
-                mdelta_add(da, imp * ima, wii(b, a, cross(arm_a, imp)));
-                mdelta_add(dc, -imp * imb, wii(b, c, cross(arm_b, -imp)));
-            }
-        } else if (row < 5) {
-            const float4 ax = __ldg(cache + row);   // {t_a, den3} or {t_b, den4}
-            const f3 ia = xyz(__ldg(cache + (row == 3 ? 5 : 7))), ib = xyz(__ldg(cache + (row == 3 ? 6 : 8)));
-            const f3 rang = xyz(b.ang[c]) - xyz(b.ang[a]);
-            const f3 axis = xyz(ax);
-            const float den = ax.w;
-            if (!(den <= 1.0e-12f)) {
-                const float imp = 0.5f * dot(rang, axis) / den;
-                mdelta_add(da, mkf3(0, 0, 0), ia * imp);
-                mdelta_add(dc, mkf3(0, 0, 0), -ib * imp);
-            }
-        }
-    }
+    const uint2 place = m.side_place[j];
 #pragma unroll
-    for (uint32_t o = kRowLanes / 2; o > 0; o >>= 1) {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            da.v[q] += __shfl_down_sync(0xffffffffu, da.v[q], o, kRowLanes);
-            dc.v[q] += __shfl_down_sync(0xffffffffu, dc.v[q], o, kRowLanes);
-        }
-    }
-    if (live && row == 0) {
-        mdelta_flush(m.deltas, a, da);
-        mdelta_flush(m.deltas, c, dc);
+    for (uint32_t side = 0; side < 2; ++side) {
+        float4* o = m.side_cache + (side ? place.y : place.x);
+        const uint64_t n = p.all_sides;
+        o[0] = f4(arm_a, side ? imb : ima);
+        o[n] = f4(arm_b, den[0]);
+        o[2 * n] = f4(ta, den[3]);
+        o[3 * n] = f4(tb, den[4]);
+        o[4 * n] = f4(side ? ib3 : ia3, den[1]);
+        o[5 * n] = f4(side ? ib4 : ia4, den[2]);
     }
 }
 
-// articulated.wgsl:318-337
-__global__ void __launch_bounds__(kMBlock) k_apply_mdeltas(StepBuffers b, MechBuffers m, MechParams p) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.body_count) return;
-    int2* d2 = reinterpret_cast<int2*>(m.deltas + 6ull * i);
-    const int2 x0 = d2[0], x1 = d2[1], x2 = d2[2];
-    if ((x0.x | x0.y | x1.x | x1.y | x2.x | x2.y) == 0) {
-        // most bodies have no bearing: their apply changes no bit unless a
-        // velocity holds -0.0 or NaN, so only those are written
-        if (zero_apply_is_identity(b.lin[i]) && zero_apply_is_identity(b.ang[i])) return;
-    } else {
-        d2[0] = make_int2(0, 0);
-        d2[1] = make_int2(0, 0);
-        d2[2] = make_int2(0, 0);
-    }
+// One projection pass (articulated.wgsl:114-155, 287-316 and the velocity apply
+// :318-337), gathered by body: every body of a bearing sums its own side of its
+// bearings' rows, so a pass is one launch that reads one pair of velocity
+// buffers and writes the other (every row reads the velocities of before the
+// pass, Jacobi).  The rows' impulses are converted to fixed point as the
+// reference does, and integer sums are order-free, so the result is that of its
+// atomics bit for bit.  A thread per bearing side computes the five rows (a
+// lane per row left three eighths of the lanes idle and issued both kinds of
+// row in every warp); a body's sides are neighbouring lanes of one warp and are
+// added by a segmented scan.  A row's pose-only parts come from the set's
+// bearing cache.  Bound: issue.  One B200, 198,009 bearings on 100,000 bodies: a
+// bearing per eight lanes with twelve atomics, and an apply launch, 52 us; this
+// 24 us (33 us against 60 with a contact iteration's apply).
+//
+// kContacts: the pass follows a contact iteration whose fixed-point deltas are
+// still to be applied (collision.wgsl:1050-1069): each body it reads gets them
+// on the way, and bodies without bearings are written too.  It then clears
+// `clear`, the delta buffer of the next iteration.
+struct VelocityPass {
+    const float4 *lin, *ang;       // velocities before the pass
+    float4 *lin_out, *ang_out;     // bodies with bearings
+    float4 *lin_rest, *ang_rest;   // the others
+    const int32_t* deltas;         // contact deltas of the iteration before (kContacts)
+    int32_t* clear;                // contact deltas of the next one (kContacts)
+};
+// v + delta / 2^20 (an apply of zeros changes -0.0, NaN payloads and w only)
+__device__ __forceinline__ void apply_fixed(const int32_t* v, float4& lin, float4& ang) {
     const float s = 1048576.0f;
-    const f3 ld = mkf3((float)x0.x, (float)x0.y, (float)x1.x) / s;
-    const f3 ad = mkf3((float)x1.y, (float)x2.x, (float)x2.y) / s;
-    b.lin[i] = f4(xyz(b.lin[i]) + ld, 0.0f);
-    b.ang[i] = f4(xyz(b.ang[i]) + ad, 0.0f);
+    lin = f4(xyz(lin) + mkf3((float)v[0], (float)v[1], (float)v[2]) / s, 0.0f);
+    ang = f4(xyz(ang) + mkf3((float)v[3], (float)v[4], (float)v[5]) / s, 0.0f);
+}
+// Blocks [0, side_blocks): padded bearing sides.  [side_blocks, side_blocks +
+// hub_blocks): bodies of more than 32 bearings, a warp each.  Then the rest.
+template <bool kContacts>
+__global__ void __launch_bounds__(kPassBlock) k_bearing_pass(StepBuffers b, MechBuffers m, MechParams p, VelocityPass f,
+                                                            uint32_t side_blocks, uint32_t hub_blocks) {
+    const bool contacts = kContacts && b.counts->active != 0u;   // collision.wgsl:744: no apply without active contacts
+    auto velocity = [&](uint32_t body, float4& lin, float4& ang) {
+        lin = __ldg(f.lin + body);
+        ang = __ldg(f.ang + body);
+        if (contacts) {
+            const int2* d2 = reinterpret_cast<const int2*>(f.deltas + 6ull * body);   // 24-byte rows
+            const int2 x0 = __ldg(d2), x1 = __ldg(d2 + 1), x2 = __ldg(d2 + 2);
+            const int32_t v[6] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y};
+            apply_fixed(v, lin, ang);
+        }
+    };
+    auto clear = [&](uint32_t body) {
+        if (!kContacts) return;
+        int2* d2 = reinterpret_cast<int2*>(f.clear + 6ull * body);
+        d2[0] = d2[1] = d2[2] = make_int2(0, 0);
+    };
+    auto finish = [&](uint32_t body, const uint32_t* sum, float4 lin, float4 ang) {
+        const int32_t total[6] = {(int32_t)sum[0], (int32_t)sum[1], (int32_t)sum[2],
+                                  (int32_t)sum[3], (int32_t)sum[4], (int32_t)sum[5]};
+        apply_fixed(total, lin, ang);
+        f.lin_out[body] = lin;
+        f.ang_out[body] = ang;
+        clear(body);
+    };
+    // the fixed-point deltas of one side of a bearing's five rows, added to `sum`
+    auto add_side = [&](uint32_t body, uint32_t at, const float4& lin, const float4& ang, uint32_t* sum) {
+        const uint2 ent = __ldg(m.side_entries + at);
+        const bool side_b = ent.x != 0u;
+        const float4* cache = m.side_cache + at;
+        const uint64_t n = p.all_sides;
+        const float4 ca = __ldg(cache), cb = __ldg(cache + n), t3 = __ldg(cache + 2 * n), t4 = __ldg(cache + 3 * n);
+        const float4 in3 = __ldg(cache + 4 * n), in4 = __ldg(cache + 5 * n);
+        float4 ol, oa;
+        velocity(ent.y, ol, oa);
+        auto add = [&](f3 l, f3 a) {
+            const float s = 1048576.0f;
+            sum[0] += (uint32_t)fixed_i32(l.x * s);
+            sum[1] += (uint32_t)fixed_i32(l.y * s);
+            sum[2] += (uint32_t)fixed_i32(l.z * s);
+            sum[3] += (uint32_t)fixed_i32(a.x * s);
+            sum[4] += (uint32_t)fixed_i32(a.y * s);
+            sum[5] += (uint32_t)fixed_i32(a.z * s);
+        };
+        const f3 arm_a = xyz(ca), arm_b = xyz(cb);
+        const f3 own = xyz(lin) + cross(xyz(ang), side_b ? arm_b : arm_a);
+        const f3 other = xyz(ol) + cross(xyz(oa), side_b ? arm_a : arm_b);
+        const f3 rel = side_b ? own - other : other - own;   // body b's minus body a's
+#pragma unroll
+        for (uint32_t row = 0; row < 3; ++row) {
+            const f3 d = row == 0 ? mkf3(1, 0, 0) : row == 1 ? mkf3(0, 1, 0) : mkf3(0, 0, 1);
+            const float den = row == 0 ? cb.w : row == 1 ? in3.w : in4.w;
+            if (den <= 1.0e-12f) continue;
+            const f3 imp = d * (0.5f * dot(rel, d) / den);
+            if (side_b) add(-imp * ca.w, wii(b, body, cross(arm_b, -imp)));
+            else add(imp * ca.w, wii(b, body, cross(arm_a, imp)));
+        }
+        const f3 rang = side_b ? xyz(ang) - xyz(oa) : xyz(oa) - xyz(ang);
+#pragma unroll
+        for (uint32_t row = 3; row < 5; ++row) {
+            const float4 ax = row == 3 ? t3 : t4;   // hinge tangent, denominator
+            const f3 inertia = xyz(row == 3 ? in3 : in4);
+            if (ax.w <= 1.0e-12f) continue;
+            const float imp = 0.5f * dot(rang, xyz(ax)) / ax.w;
+            add(mkf3(0, 0, 0), side_b ? -inertia * imp : inertia * imp);
+        }
+    };
+    const uint32_t lane = lane_id();
+    if (blockIdx.x < side_blocks) {
+        const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;   // the list is padded to whole blocks
+        const uint32_t body = __ldg(m.side_body + t);
+        uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+        float4 lin = make_float4(0, 0, 0, 0), ang = lin;
+        if (body != kInvalid) {
+            velocity(body, lin, ang);
+            add_side(body, t, lin, ang, sum);
+        }
+        // segmented sum over the body's lanes (a body never crosses a warp): its last lane finishes it
+        const uint32_t before = __shfl_up_sync(0xffffffffu, body, 1);
+        const uint32_t after = __shfl_down_sync(0xffffffffu, body, 1);
+        const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || before != body);
+        const uint32_t head = 31u - __clz(heads & ((2u << lane) - 1u));
+        for (uint32_t o = 1; o < p.most_sides; o <<= 1)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, sum[c], o);
+                if (lane >= head + o) sum[c] += u;
+            }
+        if (body != kInvalid && (lane == 31u || after != body)) finish(body, sum, lin, ang);
+        return;
+    }
+    if (blockIdx.x < side_blocks + hub_blocks) {
+        const uint32_t h = ((blockIdx.x - side_blocks) * blockDim.x + threadIdx.x) >> 5;
+        if (h >= p.hub_bodies) return;
+        const uint32_t body = m.hub_bodies[h];
+        uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+        float4 lin, ang;
+        velocity(body, lin, ang);
+        for (uint32_t e = m.hub_off[h] + lane; e < m.hub_off[h + 1]; e += 32u)
+            add_side(body, p.padded_sides + e, lin, ang, sum);
+#pragma unroll
+        for (uint32_t o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+        if (lane == 0) finish(body, sum, lin, ang);
+        return;
+    }
+    // bodies without bearings: the apply of zero deltas
+    const uint32_t i = (blockIdx.x - side_blocks - hub_blocks) * blockDim.x + threadIdx.x + p.bearing_bodies;
+    if (i >= p.body_count) return;
+    const uint32_t body = m.pass_bodies[i];
+    const int32_t zeros[6] = {0, 0, 0, 0, 0, 0};
+    float4 lin, ang;
+    velocity(body, lin, ang);
+    if (!kContacts && zero_apply_is_identity(lin) && zero_apply_is_identity(ang)) return;   // in place
+    apply_fixed(zeros, lin, ang);
+    f.lin_rest[body] = lin;
+    f.ang_rest[body] = ang;
+    clear(body);
+}
+// After an odd number of passes: the velocities of the listed bodies back into place.
+__global__ void __launch_bounds__(kMBlock) k_pass_back(MechBuffers m, uint32_t count, VelocityPass f) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const uint32_t body = m.pass_bodies[i];
+    f.lin_out[body] = f.lin[body];
+    f.ang_out[body] = f.ang[body];
 }
 
 // articulated.wgsl:157-285: forward then backward sweeps with immediate updates.
@@ -2604,11 +2723,37 @@ static cudaError_t bearing_cache(MechBuffers& m, const StepBuffers& b, const Mec
     return cudaGetLastError();
 }
 
-static cudaError_t bearing_projection_iteration(MechBuffers& m, const StepBuffers& b, const MechParams& p,
-                                                cudaStream_t s) {
-    // a group of kRowLanes lanes per bearing, in 64-thread blocks (8 bearings each)
-    if (p.bearing_count) k_project_bearings<<<(p.bearing_count + 7) / 8, 64, 0, s>>>(b, m, p);
-    k_apply_mdeltas<<<nblocks(p.body_count), kMBlock, 0, s>>>(b, m, p);
+// The two velocity buffer pairs that the passes alternate between: the live
+// velocities and the first iteration pair of the cooperative solve (not used
+// while bearings are projected).
+static void velocity_buffers(const StepBuffers& b, const MechParams& p, float4* lin[2], float4* ang[2]) {
+    lin[0] = b.lin;
+    ang[0] = b.ang;
+    lin[1] = b.vel_iter;
+    ang[1] = b.vel_iter + p.body_count;
+}
+static uint32_t side_blocks(const MechParams& p) { return p.padded_sides / kPassBlock; }
+static uint32_t hub_blocks(const MechParams& p) { return (p.hub_bodies * 32u + kPassBlock - 1) / kPassBlock; }
+static uint32_t rest_blocks(const MechParams& p) {
+    return (p.body_count - p.bearing_bodies + kPassBlock - 1) / kPassBlock;
+}
+
+// `iterations` projection passes over the live velocities (bodies without
+// bearings get their apply of zeros with the first one; it changes nothing after that).
+static cudaError_t bearing_projections(MechBuffers& m, const StepBuffers& b, const MechParams& p, cudaStream_t s) {
+    float4 *lin[2], *ang[2];
+    velocity_buffers(b, p, lin, ang);
+    const uint32_t sides = side_blocks(p), hubs = hub_blocks(p), passes = std::max(1u, p.iterations);
+    for (uint32_t it = 0; it < passes; ++it) {
+        const uint32_t from = it & 1u, to = from ^ 1u;
+        const uint32_t rest = it == 0 ? rest_blocks(p) : 0u;
+        if (sides + hubs + rest == 0) continue;
+        const VelocityPass f{lin[from], ang[from], lin[to], ang[to], lin[from], ang[from], nullptr, nullptr};
+        k_bearing_pass<false><<<sides + hubs + rest, kPassBlock, 0, s>>>(b, m, p, f, sides, hubs);
+    }
+    if ((passes & 1u) && p.bearing_bodies)
+        k_pass_back<<<nblocks(p.bearing_bodies), kMBlock, 0, s>>>(m, p.bearing_bodies,
+                                                                  VelocityPass{lin[1], ang[1], lin[0], ang[0]});
     return cudaGetLastError();
 }
 
@@ -2760,8 +2905,7 @@ void mechanism_tick_clears(const MechBuffers& m, const MechParams& p, void** ptr
 cudaError_t enqueue_mechanism(MechBuffers& m, const StepBuffers& b, const MechParams& p, cudaStream_t s) {
     cudaError_t e;
     if ((e = bearing_cache(m, b, p, s)) != cudaSuccess) return e;
-    for (uint32_t it = 0; it < std::max(1u, p.iterations); ++it)
-        if ((e = bearing_projection_iteration(m, b, p, s)) != cudaSuccess) return e;
+    if ((e = bearing_projections(m, b, p, s)) != cudaSuccess) return e;
     k_advance_coordinates<<<nblocks(p.body_count), kMBlock, 0, s>>>(b, m, p);
     if ((e = forward_kinematics(m, p, s)) != cudaSuccess) return e;
     const uint32_t mode = g_closure_grid;
@@ -2805,21 +2949,32 @@ cudaError_t enqueue_mechanism(MechBuffers& m, const StepBuffers& b, const MechPa
 cudaError_t enqueue_contact_solver_with_bearings(MechBuffers& m, const StepBuffers& b, const StepParams& sp,
                                                  const MechParams& p, const StepLaunch& l, int parity,
                                                  cudaStream_t s) {
-    return launch_contact_solver_stepwise(b, sp, l, parity, p.serial_contacts != 0u, [&](bool serial) {
-        if (serial) {
+    if (p.serial_contacts)
+        return launch_contact_solver_serial(b, sp, l, parity, [&]() {
             k_project_bearings_serial<<<1, 32, 0, s>>>(b, m, p);
             return cudaGetLastError();
-        }
-        return bearing_projection_iteration(m, b, p, s);
+        }, s);
+    float4 *lin[2], *ang[2];
+    velocity_buffers(b, p, lin, ang);
+    const uint32_t sides = side_blocks(p), hubs = hub_blocks(p), iterations = std::max(1u, l.iterations);
+    cudaError_t e = launch_contact_solver_passes(b, sp, l, parity, lin, ang, [&](uint32_t it, int32_t* deltas, int32_t* clear) {
+        const uint32_t from = it & 1u, to = from ^ 1u;
+        k_bearing_pass<true><<<sides + hubs + rest_blocks(p), kPassBlock, 0, s>>>(
+            b, m, p, VelocityPass{lin[from], ang[from], lin[to], ang[to], lin[to], ang[to], deltas, clear}, sides, hubs);
+        return cudaGetLastError();
     }, s);
+    if (e == cudaSuccess && (iterations & 1u)) {
+        k_pass_back<<<nblocks(p.body_count), kMBlock, 0, s>>>(m, p.body_count,
+                                                              VelocityPass{lin[1], ang[1], lin[0], ang[0]});
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 // device.rs:1128-1155
 cudaError_t enqueue_post_contact(MechBuffers& m, const StepBuffers& b, const MechParams& p, cudaStream_t s) {
     cudaError_t e;
-    if (!p.has_dynamic_root)
-        for (uint32_t it = 0; it < std::max(1u, p.iterations); ++it)
-            if ((e = bearing_projection_iteration(m, b, p, s)) != cudaSuccess) return e;
+    if (!p.has_dynamic_root && (e = bearing_projections(m, b, p, s)) != cudaSuccess) return e;
     k_capture_coordinates<<<nblocks(p.body_count), kMBlock, 0, s>>>(b, m, p);
     if (!p.has_dynamic_root) return reconstruct(m, b, p, s);
     return cudaGetLastError();

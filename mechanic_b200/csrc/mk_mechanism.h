@@ -18,6 +18,11 @@ struct MechParams {
     uint32_t iterations = 8;
     uint32_t closure_mode = 0;
     uint32_t has_dynamic_root = 0;
+    uint32_t bearing_bodies = 0;     // bodies with at least one bearing
+    uint32_t padded_sides = 0;       // bearing sides with their padding, whole blocks
+    uint32_t most_sides = 1;         // most sides of a body in that list (at most 32)
+    uint32_t hub_bodies = 0;         // bodies of more than 32 bearings
+    uint32_t all_sides = 0;          // padded_sides and the hub bodies' sides
     uint32_t serial_contacts = 0;    // dynamic root and <= 64 bearings (device.rs:1370-1373)
     float dt = 1.0f / 60.0f, ang_damp = 0.98f;
     // closure topology (host-derived, static)
@@ -60,9 +65,15 @@ struct MechBuffers {
     GpuLinkState* links_a = nullptr;            // B
     GpuLinkState* links_b = nullptr;            // B
     GpuLinkState* links_final = nullptr;        // alias of a or b
-    int32_t* deltas = nullptr;                  // 6 per body (bearing projection)
+    // bearing projection: bodies with bearings first, the others after them
+    uint32_t* pass_bodies = nullptr;            // B
+    uint32_t* side_body = nullptr;              // padded_sides: body of each bearing side (MK_INVALID_INDEX: padding)
+    uint2* side_entries = nullptr;              // all_sides: {side, the other body}; those of hub bodies at the end
+    uint2* side_place = nullptr;                // J: places of a bearing's two sides in that list
+    float4* side_cache = nullptr;               // rows x all_sides: pose-only parts of each side's projection rows
+    uint32_t* hub_bodies = nullptr;             // bodies of more than 32 bearings
+    uint32_t* hub_off = nullptr;
     // reconstruct_body_velocities by depth level (level l: bodies [off[l], off[l+1]))
-    float4* bear_cache = nullptr;               // 9 float4 per bearing: pose-only parts of its projection rows
     uint32_t* level_bodies = nullptr;
     const uint32_t* level_offsets = nullptr;    // host memory owned by the handle, level_count + 1 entries
     uint32_t level_count = 0;
@@ -124,6 +135,8 @@ MechParams make_mech_params(const MkCreation* cr, const StepParams& p, uint32_t 
                             float closure_tol, uint32_t closure_max_it, uint32_t precond);
 // Host-side closure topology and depth levels; fills the counts in `p`.
 struct MechTopology {
+    std::vector<uint32_t> pass_bodies, side_body, hub_bodies, hub_off;
+    std::vector<uint2> side_entries, side_place;
     std::vector<uint32_t> level_bodies, level_offsets, level_parent;
     std::vector<uint32_t> cl_bearings, cl_slot_off, cl_split, slot_body, cq_coords, cq_off, cq_slots, cb_bodies;
     std::vector<uint32_t> cl_order, cl_columns, col_coord, col_pos, cl_places, slot_parent, cq_child, cb_parents;

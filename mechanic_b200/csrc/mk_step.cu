@@ -2757,12 +2757,12 @@ cudaError_t launch_warm_targets(const StepBuffers& b, int parity, uint32_t A, fl
 }
 
 // Per-iteration kernels for ticks that interleave bearing projection with
-// the contact iterations (device.rs:1363-1416): velocities are updated in
-// place, so each phase is its own launch.
+// the contact iterations (device.rs:1363-1416).
 template <bool kWarm>
-__global__ void __launch_bounds__(kBlock) k_solve_iter(StepBuffers b, StepParams p, GpuContact* cur) {
+__global__ void __launch_bounds__(kBlock) k_solve_iter(StepBuffers b, StepParams p, GpuContact* cur,
+                                                       const float4* lin, const float4* ang) {
     const uint32_t A = b.counts->active;
-    solve_span<kWarm>(b, p, cur, contact_slice(A, gridDim.x), b.lin, b.ang);
+    solve_span<kWarm>(b, p, cur, contact_slice(A, gridDim.x), lin, ang);
 }
 
 __global__ void __launch_bounds__(kBlock) k_apply_iter(StepBuffers b, StepParams p) {
@@ -2964,6 +2964,14 @@ void set_heavy_solve_form(uint32_t form) { g_heavy_solve_form = form <= MK_HEAVY
 uint32_t heavy_solve_form() { return g_heavy_solve_form; }
 constexpr uint32_t kDefaultHeavyForm = MK_HEAVY_SPLIT;   // measured fastest: tick 1 of the 100,000-body config 4.44 ms (scatter 5.12, gather 6.02)
 
+static void launch_prepare(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity, cudaStream_t s) {
+    const uint32_t grid = (uint32_t)l.sm_count * (l.append_ctas ? l.append_ctas : 8u);
+    AppendSite prep{b.lookback + 3 * b.lookback_words, b.tickets + 3};
+    const int prev = parity ^ 1;
+    k_prepare<<<grid, kBlock, 0, s>>>(b, p, prep, b.contacts[parity], b.contact_keys[parity], b.features[parity],
+                                       b.contacts[prev], b.contact_keys[prev], b.features[prev]);
+}
+
 // Dynamic shared memory of the one-block solves, set once per device (outside
 // stream capture: at handle creation).
 cudaError_t step_prepare() {
@@ -2984,11 +2992,7 @@ cudaError_t step_prepare() {
 
 cudaError_t launch_contact_solver(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
                                   cudaStream_t s, const std::function<cudaError_t()>& before_solve) {
-    const uint32_t grid = (uint32_t)l.sm_count * (l.append_ctas ? l.append_ctas : 8u);
-    AppendSite prep{b.lookback + 3 * b.lookback_words, b.tickets + 3};
-    const int prev = parity ^ 1;
-    k_prepare<<<grid, kBlock, 0, s>>>(b, p, prep, b.contacts[parity], b.contact_keys[parity], b.features[parity],
-                                       b.contacts[prev], b.contact_keys[prev], b.features[prev]);
+    launch_prepare(b, p, l, parity, s);
     if (before_solve) {
         cudaError_t eb = before_solve();
         if (eb != cudaSuccess) return eb;
@@ -3038,31 +3042,39 @@ cudaError_t launch_contact_solver(const StepBuffers& b, const StepParams& p, con
     return cudaGetLastError();
 }
 
-cudaError_t launch_contact_solver_stepwise(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
-                                           bool serial, const std::function<cudaError_t(bool)>& after_apply,
-                                           cudaStream_t s) {
+cudaError_t launch_contact_solver_passes(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
+                                         float4* const* lin, float4* const* ang,
+                                         const std::function<cudaError_t(uint32_t, int32_t*, int32_t*)>& pass,
+                                         cudaStream_t s) {
     const uint32_t grid = (uint32_t)l.sm_count * (l.append_ctas ? l.append_ctas : 8u);
-    AppendSite prep{b.lookback + 3 * b.lookback_words, b.tickets + 3};
-    const int prev = parity ^ 1;
     GpuContact* cur = b.contacts[parity];
-    k_prepare<<<grid, kBlock, 0, s>>>(b, p, prep, cur, b.contact_keys[parity], b.features[parity], b.contacts[prev],
-                                       b.contact_keys[prev], b.features[prev]);
-    const uint32_t body_blocks = std::max<uint32_t>(1u, std::min<uint32_t>(blocks_for(p.body_count, kBlock), grid));
-    k_solve_iter<true><<<grid, kBlock, 0, s>>>(b, p, cur);
-    k_apply_iter<<<body_blocks, kBlock, 0, s>>>(b, p);
-    cudaError_t e = after_apply(serial);
-    if (e != cudaSuccess) return e;
-    const uint32_t iters = serial ? std::max<uint32_t>(1u, l.iterations) * 12u : std::max<uint32_t>(1u, l.iterations);
-    for (uint32_t it = 1; it < iters; ++it) {
-        if (serial) {
-            k_solve_serial<<<1, 32, 0, s>>>(b, p, cur);
-        } else {
-            k_solve_iter<false><<<grid, kBlock, 0, s>>>(b, p, cur);
-            k_apply_iter<<<body_blocks, kBlock, 0, s>>>(b, p);
-        }
-        if ((e = after_apply(serial)) != cudaSuccess) return e;
+    launch_prepare(b, p, l, parity, s);
+    int32_t* deltas[2] = {b.deltas, b.deltas_extra};   // a pass clears the next iteration's
+    for (uint32_t it = 0; it < std::max<uint32_t>(1u, l.iterations); ++it) {
+        StepBuffers bb = b;
+        bb.deltas = deltas[it & 1u];
+        if (it == 0) k_solve_iter<true><<<grid, kBlock, 0, s>>>(bb, p, cur, lin[0], ang[0]);
+        else k_solve_iter<false><<<grid, kBlock, 0, s>>>(bb, p, cur, lin[it & 1u], ang[it & 1u]);
+        cudaError_t e = pass(it, deltas[it & 1u], deltas[(it & 1u) ^ 1u]);
+        if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
+}
+
+cudaError_t launch_contact_solver_serial(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
+                                         const std::function<cudaError_t()>& after_apply, cudaStream_t s) {
+    const uint32_t grid = (uint32_t)l.sm_count * (l.append_ctas ? l.append_ctas : 8u);
+    GpuContact* cur = b.contacts[parity];
+    launch_prepare(b, p, l, parity, s);
+    const uint32_t body_blocks = std::max<uint32_t>(1u, std::min<uint32_t>(blocks_for(p.body_count, kBlock), grid));
+    k_solve_iter<true><<<grid, kBlock, 0, s>>>(b, p, cur, b.lin, b.ang);
+    k_apply_iter<<<body_blocks, kBlock, 0, s>>>(b, p);
+    cudaError_t e = after_apply();
+    for (uint32_t it = 1; e == cudaSuccess && it < std::max<uint32_t>(1u, l.iterations) * 12u; ++it) {
+        k_solve_serial<<<1, 32, 0, s>>>(b, p, cur);
+        e = after_apply();
+    }
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // Every region a tick needs at zero, cleared by one kernel (16-byte stores)
