@@ -76,14 +76,11 @@ __device__ __forceinline__ bool finite4(float4 v) {
            fabsf(v.y) < kFloatMax && fabsf(v.z) < kFloatMax && fabsf(v.w) < kFloatMax;
 }
 
-// i32(round(x)) with WGSL round-half-to-even and a saturating conversion.
-__device__ __forceinline__ int32_t fixed_i32(float x) {
-    float r = rintf(x);
-    if (r != r) return 0;
-    if (r >= 2147483647.0f) return INT32_MAX;
-    if (r <= -2147483648.0f) return INT32_MIN;
-    return (int32_t)r;
-}
+// i32(round(x)) with WGSL round-half-to-even and a saturating conversion (NaN
+// gives 0): the conversion instruction's own semantics, one instruction where
+// rounding, the range tests and the conversion were eight (twelve of these per
+// contact and pass).
+__device__ __forceinline__ int32_t fixed_i32(float x) { return __float2int_rn(x); }
 __device__ __forceinline__ uint32_t round_u32(float x) {
     float r = rintf(x);
     if (!(r > 0.0f)) return 0u;
