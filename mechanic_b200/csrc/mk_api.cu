@@ -1653,7 +1653,7 @@ int mk_op_sort_keys(const uint64_t* keys_in, const uint32_t* values_in, uint64_t
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // The error word lives at the end of the caller's scratch (inside the size).
     uint32_t* flags = nullptr;
-    cudaError_t e = mk::launch_sort(keys_in, values_in, keys_out, values_out, n, nullptr, key_bits, scratch,
+    cudaError_t e = mk::launch_sort(keys_in, values_in, keys_out, values_out, n, key_bits, scratch,
                                     scratch_bytes, flags, (cudaStream_t)stream, sms);
     if (e != cudaSuccess) {
         set_error(nullptr, MK_ERR_DEVICE_FAILURE, "sort: %s", cudaGetErrorString(e));

@@ -117,9 +117,12 @@ uint32_t pair_sort_items();                  // keys per thread of the pair-key 
 void set_pair_sort_items(uint32_t items);    // 0 = the default
 uint64_t sort_scratch_bytes(uint32_t n, uint32_t key_bits, bool values = true);
 cudaError_t launch_sort(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out, uint32_t* vals_out,
-                        uint32_t n, const uint32_t* n_dev, uint32_t key_bits, void* scratch,
-                        uint64_t scratch_bytes, uint32_t* error_flags, cudaStream_t stream, int sm_count,
-                        uint32_t items = 0, uint32_t ctas_per_sm = 0, bool precleared = false);
+                        uint32_t n, uint32_t key_bits, void* scratch, uint64_t scratch_bytes, uint32_t* error_flags,
+                        cudaStream_t stream, int sm_count, uint32_t items = 0, uint32_t ctas_per_sm = 0,
+                        bool precleared = false);
+cudaError_t launch_sort_counted(const uint64_t* keys_in, uint64_t* keys_out, uint32_t capacity, const uint32_t* n_dev,
+                                uint32_t key_bits, void* scratch, uint64_t scratch_bytes, uint32_t* error_flags,
+                                cudaStream_t stream, int sm_count, uint32_t items);
 void sort_clear_region(void* scratch, uint32_t n, uint32_t key_bits, bool values, void** ptr, uint64_t* bytes);
 
 // Device buffers of one handle's step (all device pointers).

@@ -93,7 +93,7 @@ int mk_op_sort_keys_static(const uint64_t* keys_in, const uint32_t* values_in, u
     }
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const cudaError_t e = mk::launch_sort(keys_in, values_in, keys_out, values_out, n, nullptr, key_bits, scratch,
+    const cudaError_t e = mk::launch_sort(keys_in, values_in, keys_out, values_out, n, key_bits, scratch,
                                           kStaticSortScratchBytes, nullptr, (cudaStream_t)stream, sms);
     if (e != cudaSuccess) {
         std::snprintf(msg, sizeof(msg), "sort_keys_static: %s", cudaGetErrorString(e));

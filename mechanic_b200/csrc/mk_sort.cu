@@ -23,32 +23,35 @@ constexpr uint32_t kDigitAggregate = 1u << 30;
 constexpr uint32_t kDigitInclusive = 2u << 30;
 constexpr uint32_t kDigitCountMask = (1u << 30) - 1;
 
-__global__ void __launch_bounds__(kSortThreads)
-k_radix_histogram(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ n_ptr, uint32_t n_fixed,
-                  uint32_t passes, uint32_t* __restrict__ hist /* passes x 256 */,
-                  uint32_t* __restrict__ lookback, uint64_t lookback_pass_words, uint32_t tile_keys,
-                  uint32_t small_n) {
-    __shared__ uint32_t s_hist[8][kRadixBins];
-    const uint32_t n = n_ptr ? min(*n_ptr, n_fixed) : n_fixed;   // a device count never exceeds the capacity
-    if (n <= small_n) return;   // sorted by k_radix_small
-    // clear the look-back words the onesweep passes will use for this n only
+// Digit counts of every pass over the keys, and the look-back words that the
+// passes will use for this n cleared.  `s_hist` holds 8 x 256 words.
+__device__ __forceinline__ void radix_histogram(const uint64_t* __restrict__ keys, uint32_t n, uint32_t passes,
+                                                uint32_t* __restrict__ hist /* passes x 256 */,
+                                                uint32_t* __restrict__ lookback, uint64_t lookback_pass_words,
+                                                uint32_t tile_keys, uint32_t* s_hist) {
     const uint64_t used = (uint64_t)((n + tile_keys - 1) / tile_keys) * kRadixBins;
     for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < used * passes;
          w += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t pass = w / used, off = w % used;
         lookback[pass * lookback_pass_words + off] = 0u;
     }
-    for (uint32_t i = threadIdx.x; i < 8 * kRadixBins; i += blockDim.x) (&s_hist[0][0])[i] = 0;
+    for (uint32_t i = threadIdx.x; i < 8 * kRadixBins; i += blockDim.x) s_hist[i] = 0;
     __syncthreads();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint64_t k = keys[i];
-        for (uint32_t p = 0; p < passes; ++p) atomicAdd(&s_hist[p][(k >> (8 * p)) & 0xffu], 1u);
+        uint64_t k = __ldcg(keys + i);
+        for (uint32_t p = 0; p < passes; ++p) atomicAdd(&s_hist[p * kRadixBins + ((k >> (8 * p)) & 0xffu)], 1u);
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < passes * kRadixBins; i += blockDim.x) {
-        uint32_t v = (&s_hist[0][0])[i];
+        uint32_t v = s_hist[i];
         if (v) atomicAdd(&hist[i], v);
     }
+}
+__global__ void __launch_bounds__(kSortThreads)
+k_radix_histogram(const uint64_t* __restrict__ keys, uint32_t n, uint32_t passes, uint32_t* __restrict__ hist,
+                  uint32_t* __restrict__ lookback, uint64_t lookback_pass_words, uint32_t tile_keys) {
+    __shared__ uint32_t s_hist[8 * kRadixBins];
+    radix_histogram(keys, n, passes, hist, lookback, lookback_pass_words, tile_keys, s_hist);
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
@@ -85,90 +88,57 @@ __device__ __forceinline__ void warp_rank(const uint32_t (&dig)[kItems], uint32_
     }
 }
 
-// Sorts up to kSmallSortKeys keys in one CTA, every pass in shared memory (no
-// look-back, no histogram kernel: the tile's digit counts are the whole
-// sort's); only the warps that hold keys rank.  Light ticks sort at most a few
-// thousand pair keys: one launch instead of a histogram and one onesweep launch
-// per digit.  With a device count above kSmallSortKeys it returns at once and
-// the onesweep passes sort (one SM ranking 8,192 keys per pass was slower than
-// four tiles on four SMs).
-constexpr uint32_t kSmallThreads = 512, kSmallItems = 8;
-constexpr uint32_t kSmallSortKeys = kSmallThreads * kSmallItems;
-constexpr size_t kSmallSmem = (size_t)kSmallSortKeys * 12 + (kSmallThreads / 32) * kRadixBins * 4;
+// Up to kSmallSortKeys keys: each key's place is the number of keys before it,
+// counted directly.  A block takes 32 keys, one per lane, and its warps split
+// the other keys between them (read from shared memory, the whole warp the same
+// word), so the work spreads over all SMs with one dependent step instead of a
+// chain of radix passes in one CTA.  Ties go by input order (a stable sort).
+// Measured on one B200 (the earlier one-CTA radix sort in brackets): 1,000 keys
+// of 39 bits with values 6 us (12.3), 3,400 pair keys 12 us (22.0).  The
+// n^2 compares of 4,096 keys are where the radix passes take over.
+constexpr uint32_t kSmallSortKeys = 4096;
+constexpr uint32_t kRankThreads = 512;
+constexpr size_t kRankSmem = (size_t)kSmallSortKeys * 8;
 
-__global__ void __launch_bounds__(kSmallThreads)
-k_radix_small(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-              uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, const uint32_t* __restrict__ n_ptr,
-              uint32_t n_fixed, uint32_t passes) {
-    const uint32_t n = n_ptr ? min(*n_ptr, n_fixed) : n_fixed;
-    if (n == 0 || n > kSmallSortKeys) return;
-    extern __shared__ __align__(16) unsigned char s_dyn[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(s_dyn);
-    uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_dyn + (size_t)kSmallSortKeys * 8);
-    uint32_t (*s_warp)[kRadixBins] = reinterpret_cast<uint32_t (*)[kRadixBins]>(s_dyn + (size_t)kSmallSortKeys * 12);
-    __shared__ uint32_t s_local_start[kRadixBins];
-    __shared__ uint32_t s_scan[33];
-    const uint32_t lane = lane_id(), w = warp_id();
-    const uint32_t d = threadIdx.x;   // the digit of threads below kRadixBins
-    const uint32_t warps = (n + 32 * kSmallItems - 1) / (32 * kSmallItems);   // warps holding keys
-    uint64_t k[kSmallItems];
-    uint32_t v[kSmallItems], dig[kSmallItems], rank[kSmallItems];
-#pragma unroll
-    for (uint32_t i = 0; i < kSmallItems; ++i) {   // warp-striped: items in index order
-        const uint32_t idx = w * 32 * kSmallItems + i * 32 + lane;
-        k[i] = idx < n ? keys_in[idx] : 0ull;
-        v[i] = (idx < n && vals_in) ? vals_in[idx] : 0u;
-    }
-    for (uint32_t pass = 0; pass < passes; ++pass) {
-        const uint32_t shift = 8 * pass;
-        for (uint32_t q = threadIdx.x; q < warps * kRadixBins; q += kSmallThreads) (&s_warp[0][0])[q] = 0;
+// `s_keys` holds n keys (an even count), `s_place` 32 words.
+__device__ __forceinline__ void rank_sort(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+                                          uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
+                                          uint64_t mask, uint64_t* s_keys, uint32_t* s_place) {
+    if (blockIdx.x * 32u >= n) return;
+    const uint32_t lane = lane_id(), w = warp_id(), warps = blockDim.x >> 5;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) s_keys[i] = __ldcg(keys_in + i) & mask;
+    if ((n & 1u) && threadIdx.x == 0) s_keys[n] = ~0ull;   // pads the last pair; an equal key comes before it
+    for (uint32_t first = blockIdx.x * 32u; first < n; first += gridDim.x * 32u) {
+        if (threadIdx.x < 32u) s_place[threadIdx.x] = 0u;
         __syncthreads();
-#pragma unroll
-        for (uint32_t i = 0; i < kSmallItems; ++i) {
-            const uint32_t idx = w * 32 * kSmallItems + i * 32 + lane;
-            dig[i] = idx < n ? (uint32_t)((k[i] >> shift) & 0xffu) : kRadixBins;
-        }
-        if (w < warps) warp_rank<kSmallItems>(dig, rank, s_warp[w], lane);
-        __syncthreads();
+        const uint32_t i = first + lane;
+        const uint64_t key = i < n ? s_keys[i] : 0ull;
+        // pairs [lo, hi) of this warp; the keys before i count when equal, those after do not
+        const uint32_t pairs = (n + 1u) >> 1, per = (pairs + warps - 1u) / warps;
+        const uint32_t lo = min(pairs, w * per), hi = min(pairs, lo + per);
         uint32_t count = 0;
-        if (d < kRadixBins) {
-            for (uint32_t ww = 0; ww < warps; ++ww) {
-                const uint32_t c = s_warp[ww][d];
-                s_warp[ww][d] = count;
-                count += c;
-            }
+#pragma unroll 8
+        for (uint32_t q = lo; q < hi; ++q) {
+            const ulonglong2 v = reinterpret_cast<const ulonglong2*>(s_keys)[q];
+            count += (v.x < key || (v.x == key && 2u * q < i)) ? 1u : 0u;
+            count += (v.y < key || (v.y == key && 2u * q + 1u < i)) ? 1u : 0u;
         }
-        uint32_t total;
-        const uint32_t start = block_exclusive_scan(count, s_scan, &total);
-        if (d < kRadixBins) s_local_start[d] = start;
+        if (count) atomicAdd(s_place + lane, count);
         __syncthreads();
-#pragma unroll
-        for (uint32_t i = 0; i < kSmallItems; ++i) {
-            if (dig[i] < kRadixBins) {
-                const uint32_t r = s_local_start[dig[i]] + s_warp[w][dig[i]] + rank[i];
-                s_keys[r] = k[i];
-                s_vals[r] = v[i];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (uint32_t i = 0; i < kSmallItems; ++i) {
-            const uint32_t idx = w * 32 * kSmallItems + i * 32 + lane;
-            if (idx < n) {
-                k[i] = s_keys[idx];
-                v[i] = s_vals[idx];
-            }
+        if (w == 0 && i < n) {
+            const uint32_t at = s_place[lane];
+            keys_out[at] = __ldcg(keys_in + i);
+            if (vals_out) vals_out[at] = __ldcg(vals_in + i);
         }
         __syncthreads();
     }
-#pragma unroll
-    for (uint32_t i = 0; i < kSmallItems; ++i) {
-        const uint32_t idx = w * 32 * kSmallItems + i * 32 + lane;
-        if (idx < n) {
-            keys_out[idx] = k[i];
-            if (vals_out) vals_out[idx] = v[i];
-        }
-    }
+}
+__global__ void __launch_bounds__(kRankThreads)
+k_rank_sort(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint64_t* __restrict__ keys_out,
+            uint32_t* __restrict__ vals_out, uint32_t n, uint64_t mask) {
+    __shared__ __align__(16) uint64_t s_keys[kSmallSortKeys];
+    __shared__ uint32_t s_place[32];
+    rank_sort(keys_in, vals_in, keys_out, vals_out, n, mask, s_keys, s_place);
 }
 
 // Shared-memory layout of a onesweep tile of kThreads x kItems keys: the
@@ -183,13 +153,13 @@ struct SortTile {
     static constexpr size_t kBytes = kWarpOff + (size_t)kWarps * kRadixBins * 4;
 };
 
+// One pass over n keys by the tiles that this block draws.
 template <uint32_t kThreads, uint32_t kItems>
-__global__ void __launch_bounds__(kThreads)
-k_radix_onesweep(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-                 uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-                 const uint32_t* __restrict__ n_ptr, uint32_t n_fixed, uint32_t shift,
-                 const uint32_t* __restrict__ digit_hist /* 256 */, uint32_t* __restrict__ lookback,
-                 uint32_t* __restrict__ ticket, uint32_t* __restrict__ error_flags, uint32_t small_n) {
+__device__ __forceinline__ void onesweep_pass(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+                                              uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
+                                              uint32_t n, uint32_t shift, const uint32_t* __restrict__ digit_hist,
+                                              uint32_t* __restrict__ lookback, uint32_t* __restrict__ ticket,
+                                              uint32_t* __restrict__ error_flags) {
     static_assert(kThreads >= kRadixBins && kThreads % 32 == 0, "one thread per digit at least");
     using L = SortTile<kThreads, kItems>;
     constexpr uint32_t kTile = L::kTile;
@@ -204,16 +174,13 @@ k_radix_onesweep(const uint64_t* __restrict__ keys_in, const uint32_t* __restric
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_digit_offsets[kRadixBins];
 
-    const uint32_t n = n_ptr ? min(*n_ptr, n_fixed) : n_fixed;   // a device count never exceeds the capacity
     const uint32_t tiles = (n + kTile - 1) / kTile;
-    // a small device count was sorted by k_radix_small; CTAs past the tile count
-    // leave before taking a ticket (the grid is sized for the capacity)
-    if (n <= small_n || blockIdx.x >= tiles) return;
+    if (blockIdx.x >= tiles) return;   // before taking a ticket (a grid sized for a capacity)
     const uint32_t lane = lane_id(), w = warp_id();
     const bool digit_thread = threadIdx.x < kRadixBins;
     const uint32_t d = threadIdx.x;   // the digit of a digit thread
     if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-    const uint32_t hist_d = digit_thread ? digit_hist[d] : 0u;   // scanned while the first tile loads
+    const uint32_t hist_d = digit_thread ? __ldcg(digit_hist + d) : 0u;   // scanned while the first tile loads
     bool have_offsets = false;
 
     for (;;) {
@@ -338,7 +305,50 @@ k_radix_onesweep(const uint64_t* __restrict__ keys_in, const uint32_t* __restric
     }
 }
 
+template <uint32_t kThreads, uint32_t kItems>
+__global__ void __launch_bounds__(kThreads)
+k_radix_onesweep(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+                 uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n, uint32_t shift,
+                 const uint32_t* __restrict__ digit_hist /* 256 */, uint32_t* __restrict__ lookback,
+                 uint32_t* __restrict__ ticket, uint32_t* __restrict__ error_flags) {
+    onesweep_pass<kThreads, kItems>(keys_in, vals_in, keys_out, vals_out, n, shift, digit_hist, lookback, ticket,
+                                    error_flags);
+}
+
+// A whole sort of keys (no values) whose count is known on the device only, in
+// one cooperative launch: small counts by rank, larger ones by the histogram
+// and the passes with a grid barrier between them.  As launches of their own,
+// the histogram and passes cost 2.5-3 us each on the ticks whose pairs the
+// small sort takes (7 launches, about 16 us a tick).
+template <uint32_t kThreads, uint32_t kItems>
+__global__ void __launch_bounds__(kThreads)
+k_sort_counted(const uint64_t* __restrict__ keys_in, uint64_t* __restrict__ tmp, uint64_t* __restrict__ keys_out,
+               const uint32_t* __restrict__ n_ptr, uint32_t capacity, uint32_t passes, uint64_t mask,
+               uint32_t* __restrict__ hist, uint32_t* __restrict__ lookback, uint64_t lookback_pass_words,
+               uint32_t* __restrict__ tickets, uint32_t* __restrict__ barrier, uint32_t* __restrict__ error_flags) {
+    using L = SortTile<kThreads, kItems>;
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ uint32_t s_place[32];
+    const uint32_t n = min(*n_ptr, capacity);   // a device count never exceeds the capacity
+    if (n <= kSmallSortKeys) {
+        rank_sort(keys_in, nullptr, keys_out, nullptr, n, mask, reinterpret_cast<uint64_t*>(s_dyn), s_place);
+        return;
+    }
+    radix_histogram(keys_in, n, passes, hist, lookback, lookback_pass_words, L::kTile,
+                    reinterpret_cast<uint32_t*>(s_dyn));
+    const uint64_t* src = keys_in;
+    for (uint32_t pass = 0; pass < passes; ++pass) {
+        grid_barrier(barrier, error_flags, gridDim.x);
+        uint64_t* dst = ((passes - 1 - pass) % 2) == 0 ? keys_out : tmp;   // the last pass writes keys_out
+        onesweep_pass<kThreads, kItems>(src, nullptr, dst, nullptr, n, 8 * pass, hist + pass * kRadixBins,
+                                        lookback + pass * lookback_pass_words, tickets + pass, error_flags);
+        src = dst;
+    }
+}
+
 uint32_t sort_passes(uint32_t key_bits) { return (key_bits + 7) / 8; }
+// The key bits that the passes order by.
+static uint64_t sort_mask(uint32_t passes) { return passes >= 8 ? ~0ull : (1ull << (8 * passes)) - 1ull; }
 
 // Keys per thread of a 256-thread onesweep tile.  The pass is latency bound:
 // its critical path is one tile's ranking (issue bound, so two tiles on one SM
@@ -382,7 +392,7 @@ void sort_clear_region(void* scratch, uint32_t n, uint32_t key_bits, bool values
     p += align256((uint64_t)n * 8);
     p += align256((uint64_t)(values ? n : 0) * 4);
     *ptr = p;
-    *bytes = align256((uint64_t)passes * kRadixBins * 4) + (uint64_t)passes * 4;
+    *bytes = align256((uint64_t)passes * kRadixBins * 4) + align256((uint64_t)passes * 4);
 }
 
 uint64_t sort_scratch_bytes(uint32_t n, uint32_t key_bits, bool values) {
@@ -397,12 +407,10 @@ uint64_t sort_scratch_bytes(uint32_t n, uint32_t key_bits, bool values) {
     return b;
 }
 
+// Shared memory of k_sort_counted: a tile, or the keys of a small sort.
 template <uint32_t kThreads, uint32_t kItems>
-static void launch_pass(const uint64_t* sk, const uint32_t* sv, uint64_t* dk, uint32_t* dv, const uint32_t* n_dev,
-                        uint32_t n, uint32_t shift, const uint32_t* offsets, uint32_t* lookback, uint32_t* ticket,
-                        uint32_t* error_flags, uint32_t grid, uint32_t small_n, cudaStream_t stream) {
-    k_radix_onesweep<kThreads, kItems><<<grid, kThreads, SortTile<kThreads, kItems>::kBytes, stream>>>(
-        sk, sv, dk, dv, n_dev, n, shift, offsets, lookback, ticket, error_flags, small_n);
+constexpr size_t counted_smem() {
+    return SortTile<kThreads, kItems>::kBytes > kRankSmem ? SortTile<kThreads, kItems>::kBytes : kRankSmem;
 }
 
 // Dynamic shared memory of every tile shape, set once per device (outside
@@ -417,7 +425,10 @@ cudaError_t sort_prepare() {
 #define MK_SORT_ATTR(T, I)                                                                                    \
     if (e == cudaSuccess)                                                                                    \
         e = cudaFuncSetAttribute(k_radix_onesweep<T, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                                 (int)SortTile<T, I>::kBytes);
+                                 (int)SortTile<T, I>::kBytes);                                                   \
+    if (e == cudaSuccess)                                                                                    \
+        e = cudaFuncSetAttribute(k_sort_counted<T, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,              \
+                                 (int)counted_smem<T, I>());
     MK_SORT_ATTR(kSortThreads, 2)
     MK_SORT_ATTR(kSortThreads, 4)
     MK_SORT_ATTR(kSortThreads, 6)
@@ -426,18 +437,35 @@ cudaError_t sort_prepare() {
     MK_SORT_ATTR(kSortThreads, 16)
     MK_SORT_ATTR(2 * kSortThreads, 16)
 #undef MK_SORT_ATTR
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_radix_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem);
     if (e == cudaSuccess) done.fetch_or(bit);
     return e;
 }
 
-// Stream-ordered sort.  `n_dev` (device count) may be null, then n is used;
-// with a device count, n is the capacity that sizes the grid and scratch.
+// The buffers of a sort inside its scratch.
+struct SortScratch {
+    uint64_t* keys;
+    uint32_t *vals, *hist, *tickets, *barrier, *lookback;
+    uint64_t lookback_words;   // per pass
+};
+static SortScratch sort_scratch(void* scratch, uint32_t n, uint32_t passes, bool values) {
+    char* p = (char*)scratch;
+    SortScratch c;
+    c.keys = (uint64_t*)p; p += align256((uint64_t)n * 8);
+    c.vals = values ? (uint32_t*)p : nullptr; p += align256((uint64_t)(values ? n : 0) * 4);
+    c.hist = (uint32_t*)p; p += align256((uint64_t)passes * kRadixBins * 4);
+    c.tickets = (uint32_t*)p;
+    c.barrier = c.tickets + 32;   // the tickets' 256 bytes hold at most 8 of them
+    p += align256((uint64_t)passes * 4);
+    c.lookback = (uint32_t*)p;
+    c.lookback_words = (uint64_t)((n + 511) / 512) * kRadixBins;   // smallest tile: 512 keys
+    return c;
+}
+
+// Stream-ordered sort of n keys with values.
 cudaError_t launch_sort(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out, uint32_t* vals_out,
-                        uint32_t n, const uint32_t* n_dev, uint32_t key_bits, void* scratch,
-                        uint64_t scratch_bytes, uint32_t* error_flags, cudaStream_t stream, int sm_count,
-                        uint32_t items_override, uint32_t ctas_per_sm, bool precleared) {
+                        uint32_t n, uint32_t key_bits, void* scratch, uint64_t scratch_bytes, uint32_t* error_flags,
+                        cudaStream_t stream, int sm_count, uint32_t items_override, uint32_t ctas_per_sm,
+                        bool precleared) {
     if (n == 0) return cudaSuccess;
     cudaError_t ep = sort_prepare();
     if (ep != cudaSuccess) return ep;
@@ -445,47 +473,38 @@ cudaError_t launch_sort(const uint64_t* keys_in, const uint32_t* vals_in, uint64
     if (passes == 0 || passes > 8) return cudaErrorInvalidValue;
     const bool values = vals_in != nullptr;
     if (scratch_bytes < sort_scratch_bytes(n, key_bits, values)) return cudaErrorInvalidValue;
-    // at most kSmallSortKeys keys: one CTA sorts them in shared memory; with a
-    // device count it runs first and the histogram and passes skip small counts
-    if (n_dev || n <= kSmallSortKeys)
-        k_radix_small<<<1, kSmallThreads, kSmallSmem, stream>>>(keys_in, vals_in, keys_out, vals_out, n_dev, n, passes);
-    if (!n_dev && n <= kSmallSortKeys) return cudaGetLastError();
-    const uint32_t small_n = n_dev ? kSmallSortKeys : 0u;
+    if (n <= kSmallSortKeys) {
+        k_rank_sort<<<(n + 31) / 32, kRankThreads, 0, stream>>>(keys_in, vals_in, keys_out, vals_out, n,
+                                                                sort_mask(passes));
+        return cudaGetLastError();
+    }
     const uint32_t items = valid_sort_items(items_override) ? items_override : sort_items_for(n, sm_count);
     const uint32_t tile_keys = kSortThreads * items;
     const uint64_t tiles = (n + tile_keys - 1) / tile_keys;
-    const uint64_t tiles_max = (n + 511) / 512;
-    char* p = (char*)scratch;
-    uint64_t* tmp_keys = (uint64_t*)p; p += align256((uint64_t)n * 8);
-    uint32_t* tmp_vals = values ? (uint32_t*)p : nullptr; p += align256((uint64_t)(values ? n : 0) * 4);
-    uint32_t* hist = (uint32_t*)p; p += align256((uint64_t)passes * kRadixBins * 4);
-    uint32_t* tickets = (uint32_t*)p; p += align256((uint64_t)passes * 4);
-    uint32_t* lookback = (uint32_t*)p;
+    const SortScratch c = sort_scratch(scratch, n, passes, values);
     // histogram bins and tile tickets are cleared here; look-back words by the
-    // histogram kernel, only as many as the device-side count needs
+    // histogram kernel, only as many as the count needs
     if (!precleared) {
-        cudaError_t e = cudaMemsetAsync(hist, 0, (uint64_t)((char*)tickets - (char*)hist) + passes * 4, stream);
+        cudaError_t e = cudaMemsetAsync(c.hist, 0, (uint64_t)((char*)c.tickets - (char*)c.hist) + passes * 4, stream);
         if (e != cudaSuccess) return e;
     }
     uint32_t hist_blocks = (uint32_t)std::min<uint64_t>((n + 4095) / 4096, (uint64_t)sm_count * 4);
-    if (hist_blocks == 0) hist_blocks = 1;
-    k_radix_histogram<<<hist_blocks, 256, 0, stream>>>(keys_in, n_dev, n, passes, hist, lookback,
-                                                       tiles_max * kRadixBins, tile_keys, small_n);
+    k_radix_histogram<<<hist_blocks, kSortThreads, 0, stream>>>(keys_in, n, passes, c.hist, c.lookback,
+                                                                c.lookback_words, tile_keys);
     const uint32_t per_sm = ctas_per_sm ? ctas_per_sm : default_sort_ctas(items);
-    uint32_t grid = (uint32_t)std::min<uint64_t>(tiles, (uint64_t)sm_count * per_sm);
-    if (grid == 0) grid = 1;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(tiles, (uint64_t)sm_count * per_sm);
     // passes alternate between (tmp, out) so that the last pass writes `out`.
     const uint64_t* src_k = keys_in;
     const uint32_t* src_v = vals_in;
     for (uint32_t pass = 0; pass < passes; ++pass) {
         bool to_out = ((passes - 1 - pass) % 2) == 0;
-        uint64_t* dk = to_out ? keys_out : tmp_keys;
-        uint32_t* dv = values ? (to_out ? vals_out : tmp_vals) : nullptr;
-        uint32_t* lb = lookback + (size_t)pass * tiles_max * kRadixBins;
-        const uint32_t* offs = hist + pass * kRadixBins;
+        uint64_t* dk = to_out ? keys_out : c.keys;
+        uint32_t* dv = values ? (to_out ? vals_out : c.vals) : nullptr;
+        uint32_t* lb = c.lookback + pass * c.lookback_words;
+        const uint32_t* offs = c.hist + pass * kRadixBins;
 #define MK_SORT_PASS(T, I)                                                                                       \
-    launch_pass<T, I>(src_k, src_v, dk, dv, n_dev, n, 8 * pass, offs, lb, tickets + pass, error_flags, grid, small_n, \
-                      stream)
+    k_radix_onesweep<T, I><<<grid, T, SortTile<T, I>::kBytes, stream>>>(src_k, src_v, dk, dv, n, 8 * pass, offs, lb, \
+                                                                        c.tickets + pass, error_flags)
         switch (items) {
             case 2: MK_SORT_PASS(kSortThreads, 2); break;
             case 4: MK_SORT_PASS(kSortThreads, 4); break;
@@ -500,6 +519,56 @@ cudaError_t launch_sort(const uint64_t* keys_in, const uint32_t* vals_in, uint64
         src_v = dv;
     }
     return cudaGetLastError();
+}
+
+template <uint32_t kThreads, uint32_t kItems>
+static cudaError_t launch_counted(const uint64_t* keys_in, uint64_t* keys_out, uint32_t capacity, const uint32_t* n_dev,
+                                  uint32_t passes, const SortScratch& c, uint32_t* error_flags, cudaStream_t stream,
+                                  int sm_count) {
+    constexpr size_t smem = counted_smem<kThreads, kItems>();
+    int per_sm = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sort_counted<kThreads, kItems>, kThreads, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    const uint64_t tiles = ((uint64_t)capacity + kThreads * kItems - 1) / (kThreads * kItems);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(std::max<uint64_t>(tiles, kSmallSortKeys / 32),
+                                                                         (uint64_t)sm_count * per_sm)));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_sort_counted<kThreads, kItems>, keys_in, c.keys, keys_out, n_dev, capacity, passes,
+                              sort_mask(passes), c.hist, c.lookback, c.lookback_words, c.tickets, c.barrier, error_flags);
+}
+
+// Stream-ordered sort of keys whose count is on the device (at most `capacity`);
+// bins, tickets and the barrier word (sort_clear_region) are clear.
+cudaError_t launch_sort_counted(const uint64_t* keys_in, uint64_t* keys_out, uint32_t capacity, const uint32_t* n_dev,
+                                uint32_t key_bits, void* scratch, uint64_t scratch_bytes, uint32_t* error_flags,
+                                cudaStream_t stream, int sm_count, uint32_t items) {
+    cudaError_t ep = sort_prepare();
+    if (ep != cudaSuccess) return ep;
+    const uint32_t passes = sort_passes(key_bits);
+    if (passes == 0 || passes > 8 || scratch_bytes < sort_scratch_bytes(capacity, key_bits, false))
+        return cudaErrorInvalidValue;
+    const SortScratch c = sort_scratch(scratch, capacity, passes, false);
+#define MK_SORT_COUNTED(T, I) \
+    return launch_counted<T, I>(keys_in, keys_out, capacity, n_dev, passes, c, error_flags, stream, sm_count)
+    switch (items) {
+        case 2: MK_SORT_COUNTED(kSortThreads, 2);
+        case 4: MK_SORT_COUNTED(kSortThreads, 4);
+        case 6: MK_SORT_COUNTED(kSortThreads, 6);
+        case 8: MK_SORT_COUNTED(kSortThreads, 8);
+        case 11: MK_SORT_COUNTED(kSortThreads, 11);
+        case 32: MK_SORT_COUNTED(2 * kSortThreads, 16);
+        default: MK_SORT_COUNTED(kSortThreads, 16);
+    }
+#undef MK_SORT_COUNTED
 }
 
 }  // namespace mk

@@ -2927,7 +2927,7 @@ cudaError_t launch_broadphase(const StepBuffers& b, const StepParams& p, const S
     if (l.morton_mode != MK_MORTON_REFERENCE_30)
         k_morton_keys<<<blocks_for(C, kBlock), kBlock, 0, s>>>(b, p, l.morton_mode);
     const uint32_t key_bits = sort_key_bits(l.morton_mode, p.scene_bits);
-    cudaError_t e = launch_sort(b.keys, b.values, b.skeys, b.svals, C, nullptr, key_bits, b.sort_scratch,
+    cudaError_t e = launch_sort(b.keys, b.values, b.skeys, b.svals, C, key_bits, b.sort_scratch,
                                 b.sort_scratch_bytes, &b.diag->error_flags, s, l.sm_count, l.sort_items, l.sort_ctas,
                                 true);   // bins and tickets cleared by the tick's reset
     if (e != cudaSuccess) return e;
@@ -2938,9 +2938,9 @@ cudaError_t launch_broadphase(const StepBuffers& b, const StepParams& p, const S
     k_refit_nodes<<<std::min<uint32_t>(blocks_for(C, kBlock), (uint32_t)l.sm_count * 2u), kBlock, 0, s>>>(b, p);
     if (b.collider_scene) k_traverse<true><<<blocks_for(C, kTravThreads), kTravThreads, 0, s>>>(b, p);
     else k_traverse<false><<<blocks_for(C, kTravThreads), kTravThreads, 0, s>>>(b, p);
-    e = launch_sort(b.pair_stage, nullptr, b.pair_keys, nullptr, p.pair_capacity, &b.counts->pairs_found,
-                    2 * p.pair_shift, b.pair_sort_scratch, b.pair_sort_scratch_bytes, &b.diag->error_flags, s,
-                    l.sm_count, pair_sort_items(), 0, true);
+    e = launch_sort_counted(b.pair_stage, b.pair_keys, p.pair_capacity, &b.counts->pairs_found, 2 * p.pair_shift,
+                            b.pair_sort_scratch, b.pair_sort_scratch_bytes, &b.diag->error_flags, s, l.sm_count,
+                            pair_sort_items());
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
