@@ -307,6 +307,7 @@ cudaError_t enqueue_tick(MkHandle* h, int parity, bool capturing) {
         if (h->collisions) {
             z.add(b.deltas, sizeof(int32_t) * 6ull * std::max(h->B, 1u));
             z.add(b.scene_bounds, 8 * sizeof(uint32_t));
+            z.add(b.inc_count, sizeof(uint32_t) * std::max(h->B, 1u));
             z.add(b.grid_barrier, 64 * sizeof(uint32_t));
             z.add(b.ground_tile_count, sizeof(uint32_t) * ((h->C + 1023) / 1024));
             z.add(b.lookback, sizeof(uint64_t) * 4 * b.lookback_words);

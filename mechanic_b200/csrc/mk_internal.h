@@ -169,11 +169,14 @@ struct StepBuffers {
     uint64_t* contact_keys[2];
     uint32_t* features[2];
     uint32_t* active;            // pair_capacity
-    // gather form of the contact solve (heavy ticks: more active contacts than 2 x bodies)
-    int32_t* contact_deltas;     // 12 per active contact: fixed-point deltas of body a, then of body b
-    uint32_t* inc_count;         // per body: contacts touching it (then a countdown while listing them)
+    // heavy ticks' contact solve (more active contacts than 2 x bodies)
+    int32_t* contact_deltas;     // gather form: 12 per active contact, fixed-point deltas of body a, then of body b;
+                                 // split form: 6 per active contact, body b's
+    uint32_t* inc_count;         // per body: entries of its list, then a countdown while they are listed
+                                 // (cleared per tick; the split form's are counted by k_prepare)
     uint32_t* inc_off;           // body_count + 1: each body's first entry in inc_list
-    uint32_t* inc_list;          // 2 x pair_capacity: 2 t + side of every active contact t, grouped by body
+    uint32_t* inc_list;          // grouped by body.  Gather form, 2 x pair_capacity: 2 t + side of every active
+                                 // contact t; split form: t of the active contacts where it is body b
     uint32_t* inc_blocks;        // per block of the cooperative solve: its bodies' entry total
     float* lam_heavy;            // split form: running normal impulse per active contact
     uint32_t heavy_form;         // heavy ticks: MK_HEAVY_SCATTER, MK_HEAVY_GATHER or MK_HEAVY_SPLIT

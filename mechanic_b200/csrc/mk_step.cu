@@ -1408,6 +1408,8 @@ __global__ void __launch_bounds__(kBlock) k_prepare(StepBuffers b, StepParams p,
                         row[2] = f4(arm_a, cached);
                         cur_feat[k] |= 1u << 24;
                         act = np.w > 1.0e-5f || vn < -1.0e-5f || cached > 1.0e-6f;
+                        if (act && bb != kInvalid && n > 2u * p.body_count)   // for the split solve's lists
+                            atomicAdd(b.inc_count + bb, 1u);
                         if (act && n <= kStampContacts) {   // for the one-block solve
                             b.body_stamp[a] = b.tick->generation;
                             if (bb != kInvalid) b.body_stamp[bb] = b.tick->generation;
@@ -1592,13 +1594,25 @@ __device__ __forceinline__ bool contact_project(const StepParams& p, const float
     return true;
 }
 
-// Adds a contact's body deltas: body A's through warp sums over runs of equal
-// bodies (contacts arrive grouped by collider A; integer sums are order-free),
-// body B's directly.
+// Adds a contact's body deltas (the whole warp calls it): body A's through warp
+// sums over runs of equal bodies (contacts arrive grouped by collider A; integer
+// sums are order-free), body B's directly.
 __device__ __forceinline__ void add_contact_deltas(int32_t* deltas, bool live, uint32_t a, uint32_t bb, int32_t* da,
                                                    const int32_t* db) {
     const uint32_t key_a = live ? a : kInvalid;
-    const bool tail = run_tail_sum(key_a, da, 6);
+    bool tail;
+    const uint32_t lives = __ballot_sync(0xffffffffu, live);
+    if (lives == 0u) return;
+    const uint32_t first = __shfl_sync(0xffffffffu, key_a, __ffs(lives) - 1);
+    if (__all_sync(0xffffffffu, !live || a == first)) {
+        // one body a in the whole warp, as on heavy ticks: six warp reductions instead of a
+        // segmented scan of thirty shuffles (3,686 -> 3,574 us on a tick of 9.5M contacts)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) da[c] = (int32_t)__reduce_add_sync(0xffffffffu, live ? (uint32_t)da[c] : 0u);
+        tail = lane_id() == __ffs(lives) - 1u;
+    } else {
+        tail = run_tail_sum(key_a, da, 6);
+    }
     if (tail && key_a != kInvalid) {
         int32_t* d = deltas + 6ull * key_a;
 #pragma unroll
@@ -1902,37 +1916,59 @@ __device__ void solve_gather(const StepBuffers& b, const StepParams& p, GpuConta
 // component, as in the scatter form), while body b's -- one atomic per
 // contact and component in the scatter form, spread over many bodies and
 // serialised per body -- go to the contact's own 24-byte slot and each body
-// sums its slots through an incidence list in the apply.  The running normal
-// impulses live in a dense array during the solve (the rows are read-only
-// until the last pass writes them back).  Same integer sums, same bits.
+// sums its slots through an incidence list in the apply.  k_prepare counts the
+// lists, a scan here places them and the first pass fills them (with passes of
+// their own over the contacts the set-up took 410 us of 3,686 on a tick of 9.5M
+// contacts; k_prepare is 23 us longer).  The running normal impulses live in a
+// dense array during the solve (the rows are read-only until the last pass
+// writes them back).  Same integer sums, same bits.
+//
+// The apply waits for dependent loads (list bounds, list, slots), so it takes as
+// many bodies at a time as their lists allow: a whole warp per body left 21 in a
+// chain, 35 us of a 60 us pass, where 100,000 bodies share 555,000 contacts
+// (lists of 5.5); with a group of 4 lanes per body the solve there takes 316 us
+// (533 before).  Above 64 entries per body the slots no longer fit into L2 and
+// what counts is that the warps stay together on neighbouring bodies, whose
+// slots share sectors: there the grouped loop took 4.6 ms against 3.7 for the
+// whole warp per body on the 9.5M contacts (now 3.2).  The denominators kept per
+// contact instead of recomputed were slower there (3.81 ms: the passes are bound
+// by memory).
 __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContact* cur, uint32_t A,
                             uint32_t iterations, uint32_t* barrier, uint32_t parts) {
     __shared__ uint32_t s_scan[33];
     uint32_t* flags = &b.diag->error_flags;
     const uint32_t B = p.body_count;
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, stride = parts * blockDim.x;
-    // ---- incidence lists of body b: counts, offsets, fill (active positions t)
-    for (uint32_t i = gtid; i < B; i += stride) b.inc_count[i] = 0u;
-    grid_barrier(barrier, flags, parts);
-    for (uint32_t t = gtid; t < A; t += stride) {
-        const uint2 ab = active_bodies(b, cur, t);
-        if (ab.y != kInvalid) atomicAdd(b.inc_count + ab.y, 1u);
-    }
-    grid_barrier(barrier, flags, parts);
+    // ---- incidence lists of body b: offsets (the first pass fills in active positions t)
     gather_scan(b, B, parts, barrier, flags, s_scan);
-    grid_barrier(barrier, flags, parts);
-    for (uint32_t t = gtid; t < A; t += stride) {
-        const uint2 ab = active_bodies(b, cur, t);
-        if (ab.y != kInvalid)
-            b.inc_list[__ldcg(b.inc_off + ab.y) + atomicSub(b.inc_count + ab.y, 1u) - 1u] = t;
-    }
     grid_barrier(barrier, flags, parts);
     const size_t Bs = B;
     const float s = (float)kFixedScale;
     const uint32_t lane = lane_id();
+    const uint32_t entries = __ldcg(b.inc_off + B);
+    const uint32_t average = (entries + B - 1u) / B;
+    const uint32_t group_bits = average <= 8u ? 2u : average <= 24u ? 3u : 4u;
+    const uint32_t group = 1u << group_bits;
+    const uint32_t in_group = lane & (group - 1u), per_warp = 32u >> group_bits;
     const uint32_t gwarp = gtid >> 5, nwarps = stride >> 5;
     const uint2 sl = contact_slice(A, parts);
     int2* slots = reinterpret_cast<int2*>(b.contact_deltas);   // 3 x int2 per active contact
+    // a body's new velocities from its slots' sums and body a's atomic sums, which it clears
+    auto apply = [&](uint32_t x, const uint32_t* sum, const float4* vl, const float4* va, float4* dl, float4* da_out) {
+        int2* d2 = reinterpret_cast<int2*>(b.deltas + 6ull * x);   // 24-byte rows are 8-byte aligned
+        const int2 v0 = __ldcg(d2), v1 = __ldcg(d2 + 1), v2 = __ldcg(d2 + 2);
+        if ((v0.x | v0.y | v1.x | v1.y | v2.x | v2.y) != 0) {
+            d2[0] = make_int2(0, 0);
+            d2[1] = make_int2(0, 0);
+            d2[2] = make_int2(0, 0);
+        }
+        const f3 ld = mkf3((float)(int32_t)(sum[0] + (uint32_t)v0.x), (float)(int32_t)(sum[1] + (uint32_t)v0.y),
+                           (float)(int32_t)(sum[2] + (uint32_t)v1.x)) / s;
+        const f3 ad = mkf3((float)(int32_t)(sum[3] + (uint32_t)v1.y), (float)(int32_t)(sum[4] + (uint32_t)v2.x),
+                           (float)(int32_t)(sum[5] + (uint32_t)v2.y)) / s;
+        dl[x] = f4(xyz(__ldg(vl + x)) + ld, 0.0f);
+        da_out[x] = f4(xyz(__ldg(va + x)) + ad, 0.0f);
+    };
     for (uint32_t it = 0; it < iterations; ++it) {
         const float4* vl = it == 0 ? b.lin : b.vel_iter + (2 * (it - 1)) * Bs;
         const float4* va = it == 0 ? b.ang : b.vel_iter + (2 * (it - 1) + 1) * Bs;
@@ -1970,6 +2006,8 @@ __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContac
                     }
                 }
                 b.lam_heavy[t] = acc;
+                if (it == 0 && bb != kInvalid)
+                    b.inc_list[__ldcg(b.inc_off + bb) + atomicSub(b.inc_count + bb, 1u) - 1u] = t;
                 if (bb != kInvalid) {
                     int2* q = slots + 3ull * t;
                     q[0] = make_int2(db[0], db[1]);
@@ -1984,42 +2022,41 @@ __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContac
         }
         grid_barrier(barrier, flags, parts);
         // ---- apply: body a's atomic sums plus the slots of the contacts where it is b
-        for (uint32_t x = gwarp; x < B; x += nwarps) {
-            const uint32_t e0 = __ldcg(b.inc_off + x), e1 = __ldcg(b.inc_off + x + 1);
-            int32_t sum[6] = {0, 0, 0, 0, 0, 0};
-            for (uint32_t e = e0 + lane; e < e1; e += 32) {
-                const int2* q = slots + 3ull * __ldcg(b.inc_list + e);
-                const int2 x0 = __ldcg(q), x1 = __ldcg(q + 1), x2 = __ldcg(q + 2);
-                sum[0] = (int32_t)((uint32_t)sum[0] + (uint32_t)x0.x);
-                sum[1] = (int32_t)((uint32_t)sum[1] + (uint32_t)x0.y);
-                sum[2] = (int32_t)((uint32_t)sum[2] + (uint32_t)x1.x);
-                sum[3] = (int32_t)((uint32_t)sum[3] + (uint32_t)x1.y);
-                sum[4] = (int32_t)((uint32_t)sum[4] + (uint32_t)x2.x);
-                sum[5] = (int32_t)((uint32_t)sum[5] + (uint32_t)x2.y);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int c = 0; c < 6; ++c)
-                    sum[c] = (int32_t)((uint32_t)sum[c] + (uint32_t)__shfl_down_sync(0xffffffffu, sum[c], o));
-            if (lane == 0) {
-                int2* d2 = reinterpret_cast<int2*>(b.deltas + 6ull * x);   // 24-byte rows are 8-byte aligned
-                const int2 x0 = __ldcg(d2), x1 = __ldcg(d2 + 1), x2 = __ldcg(d2 + 2);
-                if ((x0.x | x0.y | x1.x | x1.y | x2.x | x2.y) != 0) {
-                    d2[0] = make_int2(0, 0);
-                    d2[1] = make_int2(0, 0);
-                    d2[2] = make_int2(0, 0);
+        if (average > 64u) {
+            for (uint32_t x = gwarp; x < B; x += nwarps) {   // a warp per body
+                const uint32_t e0 = __ldcg(b.inc_off + x), e1 = __ldcg(b.inc_off + x + 1);
+                uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+                for (uint32_t e = e0 + lane; e < e1; e += 32) {
+                    const int2* q = slots + 3ull * __ldcg(b.inc_list + e);
+                    const int2 v0 = __ldcg(q), v1 = __ldcg(q + 1), v2 = __ldcg(q + 2);
+                    sum[0] += (uint32_t)v0.x; sum[1] += (uint32_t)v0.y;
+                    sum[2] += (uint32_t)v1.x; sum[3] += (uint32_t)v1.y;
+                    sum[4] += (uint32_t)v2.x; sum[5] += (uint32_t)v2.y;
                 }
-                const int32_t t0 = (int32_t)((uint32_t)sum[0] + (uint32_t)x0.x);
-                const int32_t t1 = (int32_t)((uint32_t)sum[1] + (uint32_t)x0.y);
-                const int32_t t2 = (int32_t)((uint32_t)sum[2] + (uint32_t)x1.x);
-                const int32_t t3 = (int32_t)((uint32_t)sum[3] + (uint32_t)x1.y);
-                const int32_t t4 = (int32_t)((uint32_t)sum[4] + (uint32_t)x2.x);
-                const int32_t t5 = (int32_t)((uint32_t)sum[5] + (uint32_t)x2.y);
-                const f3 ld = mkf3((float)t0, (float)t1, (float)t2) / s;
-                const f3 ad = mkf3((float)t3, (float)t4, (float)t5) / s;
-                dl[x] = f4(xyz(__ldg(vl + x)) + ld, 0.0f);
-                da_out[x] = f4(xyz(__ldg(va + x)) + ad, 0.0f);
+#pragma unroll
+                for (int c = 0; c < 6; ++c) sum[c] = __reduce_add_sync(0xffffffffu, sum[c]);
+                if (lane == 0) apply(x, sum, vl, va, dl, da_out);
+            }
+        } else {
+            for (uint32_t x0 = gwarp * per_warp; x0 < B; x0 += nwarps * per_warp) {   // a group of lanes per body
+                const uint32_t x = x0 + (lane >> group_bits);
+                uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+                if (x < B) {
+                    const uint32_t e0 = __ldcg(b.inc_off + x) + in_group, e1 = __ldcg(b.inc_off + x + 1);
+                    const uint32_t rounds = e1 > e0 ? (e1 - e0 + group - 1u) >> group_bits : 0u;
+#pragma unroll 4
+                    for (uint32_t i = 0; i < rounds; ++i) {   // (a counted loop: its loads are issued together)
+                        const int2* q = slots + 3ull * __ldcg(b.inc_list + e0 + (i << group_bits));
+                        const int2 v0 = __ldcg(q), v1 = __ldcg(q + 1), v2 = __ldcg(q + 2);
+                        sum[0] += (uint32_t)v0.x; sum[1] += (uint32_t)v0.y;
+                        sum[2] += (uint32_t)v1.x; sum[3] += (uint32_t)v1.y;
+                        sum[4] += (uint32_t)v2.x; sum[5] += (uint32_t)v2.y;
+                    }
+                }
+                for (uint32_t o = group >> 1; o > 0; o >>= 1)
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+                if (x < B && in_group == 0u) apply(x, sum, vl, va, dl, da_out);
             }
         }
         grid_barrier(barrier, flags, parts);
