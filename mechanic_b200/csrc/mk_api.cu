@@ -106,8 +106,6 @@ struct MkHandle {
     mk::ClosureState* d_cstate = nullptr;
     bool residual = false;              // contact solve runs to a residual
     float* warm_params = nullptr;       // warm-start network parameters (device, mlp::kParams)
-    void* mlp_scratch = nullptr;        // bf16 weights + partials of the network kernels
-    uint64_t mlp_scratch_bytes = 0;
     cudaEvent_t tick_done[kTickRing] = {};
     uint64_t tick_sub[kTickRing] = {};
     cudaEvent_t stage[kStageEvents] = {};
@@ -235,8 +233,6 @@ uint64_t carve(MkHandle* h, char* base) {
         b.warm_pred = c.take<float>(P);
         b.warm_features = c.take<float4>(4 * P);
         h->warm_params = c.take<float>(mk::mlp::kParams + 16);
-        h->mlp_scratch_bytes = mk::mlp::scratch_bytes(0);
-        h->mlp_scratch = c.take<char>(h->mlp_scratch_bytes);
         b.vel_res = c.take<float4>(8ull * B);
         b.solve_stats = c.take<mk::SolveStats>(1);
     }
@@ -357,7 +353,7 @@ cudaError_t enqueue_tick(MkHandle* h, int parity, bool capturing) {
                     if (ew != cudaSuccess || !l.learned_warm) return ew;
                     // network output (one column) into lam_alt, which the solve overwrites later
                     ew = mk::mlp::forward(h->warm_params, reinterpret_cast<const float*>(b.warm_features), 0,
-                                          &b.counts->active, h->pair_capacity, b.lam_alt, 1, h->mlp_scratch,
+                                          &b.counts->active, h->pair_capacity, b.lam_alt, 1,
                                           &b.diag->error_flags, s);
                     if (ew != cudaSuccess) return ew;
                     return mk::launch_warm_impulses(b, l, b.lam_alt, s);
@@ -860,7 +856,6 @@ int create_impl(const MkCreation* cr, const MkConfig* config, const MkCapacities
         ok = ok && check(cudaMemcpyAsync(b.snap_rot + (size_t)slot * h->B, b.rot, 16ull * h->B,
                                          cudaMemcpyDeviceToDevice, s), err, "snapshot init");
     }
-    if (ok && h->residual) ok = check(mk::mlp::pack(h->warm_params, h->mlp_scratch, s), err, "pack network");
     ok = ok && check(cudaStreamSynchronize(s), err, "create sync");
     if (ok && h->config.use_graph) ok = build_graphs(h, err);
     if (!ok) {
@@ -1094,7 +1089,6 @@ int mk_set_warm_start_network(MkHandle* h, const float* params, uint32_t count, 
     DeviceGuard guard(h->device);
     cudaStream_t s = h->stream;
     cudaError_t e = cudaMemcpyAsync(h->warm_params, params, sizeof(float) * count, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = mk::mlp::pack(h->warm_params, h->mlp_scratch, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return check(e, err, "set_warm_start_network") ? MK_OK : MK_ERR_DEVICE_FAILURE;
 }
@@ -1119,7 +1113,6 @@ int mk_set_preconditioner_network(MkHandle* h, const float* params, uint32_t cou
     DeviceGuard guard(h->device);
     cudaStream_t s = h->stream;
     cudaError_t e = cudaMemcpyAsync(h->mech.precond_params, params, sizeof(float) * count, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = mk::mlp::pack(h->mech.precond_params, h->mech.mlp_scratch, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return check(e, err, "set_preconditioner_network") ? MK_OK : MK_ERR_DEVICE_FAILURE;
 }

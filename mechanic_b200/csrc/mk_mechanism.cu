@@ -385,10 +385,7 @@ void carve_mechanism(MechBuffers& m, const MechParams& p, uint32_t B, uint32_t J
         m.blk_hist = f32(3ull * kClosureSteps * p.blocks);
         m.probe = f32(2ull * Q);
         m.cstate = reinterpret_cast<ClosureState*>(take(sizeof(ClosureState)));
-        if (p.learned_precond) {
-            m.precond_params = f32(mlp::kParams + 16);
-            m.mlp_scratch = take(mlp::scratch_bytes(0));
-        }
+        if (p.learned_precond) m.precond_params = f32(mlp::kParams + 16);
         m.loop_off = u32(p.loops + 1);
         m.loop_q = u32(p.closure_coords);
         m.loop_l = f32(36ull * p.loops);
@@ -449,7 +446,6 @@ bool upload_mechanism(MechBuffers& m, const MechParams& p, const MechTopology& t
     if (e == cudaSuccess && m.slot_closure) e = put(m.slot_closure, t.slot_closure, s);
     if (e == cudaSuccess && m.loop_off) e = put(m.loop_off, t.loop_off, s);
     if (e == cudaSuccess && m.loop_q) e = put(m.loop_q, t.loop_q, s);
-    if (e == cudaSuccess && m.precond_params) e = mlp::pack(m.precond_params, m.mlp_scratch, s);
     if (e == cudaSuccess) e = put(m.slot_body, t.slot_body, s);
     if (e == cudaSuccess) e = put(m.cq_coords, t.cq_coords, s);
     if (e == cudaSuccess) e = put(m.cq_off, t.cq_off, s);
@@ -2922,7 +2918,7 @@ cudaError_t enqueue_mechanism(MechBuffers& m, const StepBuffers& b, const MechPa
             }
             if (p.learned_precond) {
                 e = mlp::forward(m.precond_params, reinterpret_cast<const float*>(m.blk_feat), 0,
-                                 &m.cstate->live_blocks, p.blocks, m.blk_out, 3, m.mlp_scratch, &b.diag->error_flags, s);
+                                 &m.cstate->live_blocks, p.blocks, m.blk_out, 3, &b.diag->error_flags, s);
                 if (e != cudaSuccess) return e;
             }
             if (grid) {
@@ -3002,10 +2998,6 @@ void read_mechanism_readback(const MechBuffers& m, const MechParams& p, const Gp
         out->closure_iterations = d.reserved_c;
         out->closure_relative_residual = 0.0;
     }
-}
-
-uint64_t mechanism_mlp_scratch_bytes(const MechParams& p) {
-    return p.learned_precond ? mlp::scratch_bytes(0) : 0;
 }
 
 }  // namespace mk

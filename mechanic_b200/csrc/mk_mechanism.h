@@ -128,7 +128,6 @@ struct MechBuffers {
     uint32_t* loop_off = nullptr;               // loops + 1: offsets into loop_q
     uint32_t* loop_q = nullptr;                 // closure-coordinate positions of each loop block
     float* loop_l = nullptr;                    // 36 per loop: Cholesky factor (lower, row-major packed)
-    void* mlp_scratch = nullptr;
 };
 
 MechParams make_mech_params(const MkCreation* cr, const StepParams& p, uint32_t iterations, uint32_t closure_mode,
@@ -167,6 +166,5 @@ void enqueue_validate_bearings(MechBuffers& m, const StepBuffers& b, const MechP
 void read_mechanism_readback(const MechBuffers& m, const MechParams& p, const GpuDiagnostics& d,
                              const ClosureState* cs, MkTickReadback* out);
 // bytes of network scratch the learned preconditioner needs (0 without it)
-uint64_t mechanism_mlp_scratch_bytes(const MechParams& p);
 
 }  // namespace mk

@@ -6,7 +6,8 @@
 // with ReLU, 16 outputs (the caller uses the first few):
 //   h1 = relu(W1 x),  h2 = relu(W2 h1 + b2),  y = W3 h2 + b3.
 // Parameters are one f32 array (row-major [out][in]): W1 64x16 | W2 64x64 |
-// W3 16x64 | b2 64 | b3 16; the kernels read bf16 copies of the weights.
+// W3 16x64 | b2 64 | b3 16; every CTA rounds the weights to bf16 as it brings
+// them into shared memory.
 //
 // A CTA of 128 threads takes 128-sample tiles.  Thread t owns sample t of
 // the tile, which is TMEM lane t of every accumulator, so the epilogues are
@@ -18,8 +19,8 @@
 // ([dH2; dH1] x [H1; X]^T), whose off-diagonal blocks are unused except the
 // column of the constant input, which is the sum of dH2 over samples (db2).
 // Weight gradients accumulate in TMEM across a CTA's tiles; each CTA writes
-// one partial and a second kernel sums the partials in CTA order, so the
-// gradient of a batch is deterministic.
+// one partial, and after a grid barrier the partials are summed in CTA order,
+// so the gradient of a batch is deterministic.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -40,19 +41,34 @@ constexpr uint32_t kTmemCols = 256;
 constexpr uint32_t cAcc1 = 0, cAcc2 = 64, cAcc3 = 128, cDB = 144, cDA = 160;
 constexpr uint32_t kWaitLimit = 1u << 20;
 
-template <bool kTrain>
-struct Layout {
-    // F: [H1 (chunks 0-7) | X (8-9)]; G: [H2 (0-7) | dH2 (8-15) | dH1 (16-23)]; Y: dY (0-1)
-    static constexpr uint32_t F = 0;
-    static constexpr uint32_t G = F + 10 * kCH;
-    static constexpr uint32_t Y = G + (kTrain ? 24 : 8) * kCH;
-    static constexpr uint32_t W1 = Y + (kTrain ? 2 * kCH : 0);
+template <uint32_t kWeightsAt>
+struct WeightLayout {
+    static constexpr uint32_t W1 = kWeightsAt;
     static constexpr uint32_t W2 = W1 + 2048;
     static constexpr uint32_t W3 = W2 + 8192;
     static constexpr uint32_t B2 = W3 + 2048;
     static constexpr uint32_t B3 = B2 + 256;
-    static constexpr uint32_t RED = B3 + 64;              // 4 warps x 17 floats (db3, loss)
+    static constexpr uint32_t END = B3 + 64;
+};
+struct TrainLayout {
+    // F: [H1 (chunks 0-7) | X (8-9)]; G: [H2 (0-7) | dH2 (8-15) | dH1 (16-23)]; Y: dY (0-1)
+    static constexpr uint32_t F = 0;
+    static constexpr uint32_t G = F + 10 * kCH;
+    static constexpr uint32_t Y = G + 24 * kCH;
+    using W = WeightLayout<Y + 2 * kCH>;
+    static constexpr uint32_t RED = W::END;              // 4 warps x 17 floats (db3, loss)
     static constexpr uint32_t BAR = RED + 4 * 17 * 4 + 16;
+    static constexpr uint32_t SLOT = BAR + 8;
+    static constexpr uint32_t BYTES = SLOT + 8;
+};
+// Forward only: X, H1 and H2 take one another's place in one tile of 8 chunks (each is
+// dead once the MMAs of its layer are complete), and the three accumulators the same 64
+// TMEM columns, so that 7 CTAs fit on an SM.
+constexpr uint32_t kForwardTmem = 64, kForwardCtas = 7;
+struct ForwardLayout {
+    static constexpr uint32_t H = 0;
+    using W = WeightLayout<8 * kCH>;
+    static constexpr uint32_t BAR = W::END;
     static constexpr uint32_t SLOT = BAR + 8;
     static constexpr uint32_t BYTES = SLOT + 8;
 };
@@ -76,48 +92,79 @@ __device__ __forceinline__ void publish() {
     tc::fence_after_sync();
 }
 
-template <bool kTrain>
-__global__ void __launch_bounds__(kThreads) k_mlp(const __nv_bfloat16* __restrict__ wts, const float* __restrict__ params,
-                                                   const float* __restrict__ x, uint32_t n_host, const uint32_t* n_dev,
-                                                   float* __restrict__ y, uint32_t y_cols, const float* __restrict__ t,
-                                                   const float* __restrict__ out_w, float* __restrict__ partials,
-                                                   uint32_t* __restrict__ error_flags) {
-    using L = Layout<kTrain>;
+// Weights (rounded to bf16) into the core-matrix layout, W1 64 rows x 2 chunks, W2 64 x 8,
+// W3 16 x 8, and the biases.  Units of 8 consecutive parameters are one row of a chunk.
+// Read past L1: a training launch rewrites the parameters between its steps.
+template <class W>
+__device__ __forceinline__ void load_weights(unsigned char* smem, const float* params, uint32_t tid) {
+    constexpr uint32_t kUnits = kWeights / 8 / kThreads;
+    float w[kUnits][8];
+    if ((reinterpret_cast<uintptr_t>(params) & 15u) == 0) {
+#pragma unroll
+        for (uint32_t k = 0; k < kUnits; ++k) {
+            const float4* q = reinterpret_cast<const float4*>(params + 8 * (tid + k * kThreads));
+            const float4 lo = __ldcg(q), hi = __ldcg(q + 1);
+            w[k][0] = lo.x; w[k][1] = lo.y; w[k][2] = lo.z; w[k][3] = lo.w;
+            w[k][4] = hi.x; w[k][5] = hi.y; w[k][6] = hi.z; w[k][7] = hi.w;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t k = 0; k < kUnits; ++k)
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) w[k][i] = __ldcg(params + 8 * (tid + k * kThreads) + i);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kUnits; ++k) {
+        const uint32_t u = tid + k * kThreads;
+        uint32_t at;
+        if (u < 128) at = W::W1 + (u & 1u) * 1024 + (u >> 4) * 128 + ((u >> 1) & 7u) * 16;
+        else if (u < 640) at = W::W2 + (u & 7u) * 1024 + ((u - 128) >> 6) * 128 + ((u >> 3) & 7u) * 16;
+        else at = W::W3 + (u & 7u) * 256 + ((u - 640) >> 6) * 128 + ((u >> 3) & 7u) * 16;
+        *reinterpret_cast<uint4*>(smem + at) = make_uint4(pack_bf16(w[k][0], w[k][1]), pack_bf16(w[k][2], w[k][3]),
+                                                          pack_bf16(w[k][4], w[k][5]), pack_bf16(w[k][6], w[k][7]));
+    }
+    if (tid < 64) reinterpret_cast<float*>(smem + W::B2)[tid] = __ldcg(params + kB2 + tid);
+    if (tid < 16) reinterpret_cast<float*>(smem + W::B3)[tid] = __ldcg(params + kB3 + tid);
+}
+
+// One sample's inputs (slot 15 is the constant 1); zeros past the end.
+__device__ __forceinline__ void load_input(const float* __restrict__ x, uint32_t s, uint32_t n, float* v) {
+    if (s < n) {
+        const float4* xr = reinterpret_cast<const float4*>(x + (size_t)s * 16);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 f = __ldg(xr + q);
+            v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
+        }
+        v[15] = 1.0f;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+    }
+}
+
+// Forward pass.  A tile is a chain (inputs, three times MMA, read-back, ReLU and store)
+// that leaves the SM idle unless other tiles run beside it: with 2 CTAs per SM (256 TMEM
+// columns, 49 KB) 300,001 samples took 51 us, 6.4 us a tile; with 7, and the next tile's
+// inputs loaded during this one's first layer, 28 (24.6 in a run of calls, 48.1 before).
+__global__ void __launch_bounds__(kThreads, kForwardCtas)
+k_mlp_forward(const float* params, const float* __restrict__ x, uint32_t n_host, const uint32_t* n_dev,
+              float* __restrict__ y, uint32_t y_cols, uint32_t* __restrict__ error_flags) {
+    using L = ForwardLayout;
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char* F = smem + L::F;
-    unsigned char* G = smem + L::G;
-    unsigned char* Yb = smem + L::Y;
-    unsigned char* W1s = smem + L::W1;
-    unsigned char* W2s = smem + L::W2;
-    unsigned char* W3s = smem + L::W3;
-    float* sb2 = reinterpret_cast<float*>(smem + L::B2);
-    float* sb3 = reinterpret_cast<float*>(smem + L::B3);
-    float* sred = reinterpret_cast<float*>(smem + L::RED);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::SLOT);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const float* sb2 = reinterpret_cast<const float*>(smem + L::W::B2);
+    const float* sb3 = reinterpret_cast<const float*>(smem + L::W::B3);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5;
     const uint32_t n = n_dev ? *n_dev : n_host;
-
-    // weights into the core-matrix layout (W1: 64 rows x 2 chunks, W2: 64 x 8, W3: 16 x 8)
-    for (uint32_t u = tid; u < 128; u += kThreads) {
-        const uint32_t row = u >> 1, kc = u & 1u;
-        *reinterpret_cast<uint4*>(W1s + kc * 1024 + (row >> 3) * 128 + (row & 7) * 16) =
-            *reinterpret_cast<const uint4*>(wts + kW1 + row * 16 + kc * 8);
-    }
-    for (uint32_t u = tid; u < 512; u += kThreads) {
-        const uint32_t row = u >> 3, kc = u & 7u;
-        *reinterpret_cast<uint4*>(W2s + kc * 1024 + (row >> 3) * 128 + (row & 7) * 16) =
-            *reinterpret_cast<const uint4*>(wts + kW2 + row * 64 + kc * 8);
-    }
-    for (uint32_t u = tid; u < 128; u += kThreads) {
-        const uint32_t row = u >> 3, kc = u & 7u;
-        *reinterpret_cast<uint4*>(W3s + kc * 256 + (row >> 3) * 128 + (row & 7) * 16) =
-            *reinterpret_cast<const uint4*>(wts + kW3 + row * 64 + kc * 8);
-    }
-    if (tid < 64) sb2[tid] = params[kB2 + tid];
-    if (tid < 16) sb3[tid] = params[kB3 + tid];
+    const uint32_t tiles = (n + kTile - 1) / kTile;
+    if (blockIdx.x >= tiles) return;
+    float next[16];
+    load_input(x, blockIdx.x * kTile + tid, n, next);
+    load_weights<L::W>(smem, params, tid);
     if (tid == 0) tc::mbar_init(bar, 1);
-    if (warp == 0) tc::tmem_alloc(tslot, kTmemCols);
+    if (warp == 0) tc::tmem_alloc(tslot, kForwardTmem);
     publish();
     const uint32_t tbase = *tslot;
     const uint32_t tlane = tbase + ((32u * warp) << 16);
@@ -131,38 +178,135 @@ __global__ void __launch_bounds__(kThreads) k_mlp(const __nv_bfloat16* __restric
         phase ^= 1u;
         tc::fence_after_sync();
     };
+    const uint32_t sH = tc::smem_u32(smem + L::H);
+    const uint32_t sW1 = tc::smem_u32(smem + L::W::W1), sW2 = tc::smem_u32(smem + L::W::W2);
+    const uint32_t sW3 = tc::smem_u32(smem + L::W::W3);
+    constexpr uint32_t id64 = tc::idesc_bf16(128, 64, false, false);
+    constexpr uint32_t id16 = tc::idesc_bf16(128, 16, false, false);
+    const bool rows4 = (y_cols & 3u) == 0u && (reinterpret_cast<uintptr_t>(y) & 15u) == 0;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t s = tile * kTile + tid;
+        store8(smem + L::H, 0, tid, next);
+        store8(smem + L::H, 1, tid, next + 8);
+        publish();
+        // layer 1: [128 x 16] x W1^T
+        if (tid == 0) {
+            tc::mma_bf16(tbase, tc::sdesc(sH, kCH, 128), tc::sdesc(sW1, 1024, 128), id64, 0);
+            tc::commit(bar);
+        }
+        if (tile + gridDim.x < tiles) load_input(x, s + gridDim.x * kTile, n, next);
+        mma_wait();
+        float v[16];
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            tc::tmem_ld16(tlane + 16 * q, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = v[i] > 0.0f ? v[i] : 0.0f;
+            store8(smem + L::H, 2 * q, tid, v);
+            store8(smem + L::H, 2 * q + 1, tid, v + 8);
+        }
+        publish();
+        // layer 2: H1 [128 x 64] x W2^T
+        if (tid == 0) {
+#pragma unroll
+            for (uint32_t ks = 0; ks < 4; ++ks)
+                tc::mma_bf16(tbase, tc::sdesc(sH + 2 * ks * kCH, kCH, 128), tc::sdesc(sW2 + 2 * ks * 1024, 1024, 128),
+                             id64, ks > 0);
+            tc::commit(bar);
+        }
+        mma_wait();
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            tc::tmem_ld16(tlane + 16 * q, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                v[i] += sb2[16 * q + i];
+                v[i] = v[i] > 0.0f ? v[i] : 0.0f;
+            }
+            store8(smem + L::H, 2 * q, tid, v);
+            store8(smem + L::H, 2 * q + 1, tid, v + 8);
+        }
+        publish();
+        // layer 3: H2 [128 x 64] x W3^T
+        if (tid == 0) {
+#pragma unroll
+            for (uint32_t ks = 0; ks < 4; ++ks)
+                tc::mma_bf16(tbase, tc::sdesc(sH + 2 * ks * kCH, kCH, 128), tc::sdesc(sW3 + 2 * ks * 256, 256, 128),
+                             id16, ks > 0);
+            tc::commit(bar);
+        }
+        mma_wait();
+        tc::tmem_ld16(tlane, v);
+#pragma unroll
+        for (int o = 0; o < 16; ++o) v[o] += sb3[o];
+        if (s < n) {
+            float* row = y + (size_t)s * y_cols;
+            if (rows4) {
+#pragma unroll
+                for (uint32_t o = 0; o < 16; o += 4)
+                    if (o < y_cols)
+                        *reinterpret_cast<float4*>(row + o) = make_float4(v[o], v[o + 1], v[o + 2], v[o + 3]);
+            } else {
+#pragma unroll
+                for (uint32_t o = 0; o < 16; ++o)
+                    if (o < y_cols) row[o] = v[o];
+            }
+        }
+        tc::fence_before_sync();
+        __syncthreads();   // the accumulator is read by all before the next tile's layer 1 overwrites it
+        tc::fence_after_sync();
+    }
+    if (warp == 0) tc::tmem_free(tbase, kForwardTmem);
+}
+
+__device__ __forceinline__ void store16(float* at, const float* v) {
+#pragma unroll
+    for (int j = 0; j < 16; j += 4)
+        *reinterpret_cast<float4*>(at + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+}
+
+// Forward and backward over the tiles of CTA blockIdx.x of `parts`, and its partial.
+__device__ __forceinline__ void train_tiles(unsigned char* smem, const float* params, const float* __restrict__ x,
+                                            const float* __restrict__ t, const float* __restrict__ out_w, uint32_t n,
+                                            uint32_t parts, uint32_t tbase, uint32_t& phase, float* partials,
+                                            uint32_t* error_flags) {
+    using L = TrainLayout;
+    unsigned char* F = smem + L::F;
+    unsigned char* G = smem + L::G;
+    unsigned char* Yb = smem + L::Y;
+    const float* sb2 = reinterpret_cast<const float*>(smem + L::W::B2);
+    const float* sb3 = reinterpret_cast<const float*>(smem + L::W::B3);
+    float* sred = reinterpret_cast<float*>(smem + L::RED);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t tlane = tbase + ((32u * warp) << 16);
+    auto mma_wait = [&]() {
+        if (!tc::mbar_wait(bar, phase, kWaitLimit)) atomicOr(error_flags, MK_DEVICE_WAIT_TIMEOUT_FLAG);
+        phase ^= 1u;
+        tc::fence_after_sync();
+    };
     const uint32_t sF = tc::smem_u32(F), sG = tc::smem_u32(G), sY = tc::smem_u32(Yb);
-    const uint32_t sW1 = tc::smem_u32(W1s), sW2 = tc::smem_u32(W2s), sW3 = tc::smem_u32(W3s);
+    const uint32_t sW1 = tc::smem_u32(smem + L::W::W1), sW2 = tc::smem_u32(smem + L::W::W2);
+    const uint32_t sW3 = tc::smem_u32(smem + L::W::W3);
     constexpr uint32_t id64 = tc::idesc_bf16(128, 64, false, false);
     constexpr uint32_t id16 = tc::idesc_bf16(128, 16, false, false);
     constexpr uint32_t id64_bmn = tc::idesc_bf16(128, 64, false, true);
     constexpr uint32_t id80_mn = tc::idesc_bf16(128, 80, true, true);
     constexpr uint32_t id16_mn = tc::idesc_bf16(128, 16, true, true);
 
+    load_weights<L::W>(smem, params, tid);
     const float coef = n > 0 ? 2.0f / (float)n : 0.0f;
+    const uint32_t tiles = (n + kTile - 1) / kTile;
     float loss = 0.0f;
     float db3[16];
 #pragma unroll
     for (int o = 0; o < 16; ++o) db3[o] = 0.0f;
-
-    const uint32_t tiles = (n + kTile - 1) / kTile;
     uint32_t it = 0;
-    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += parts, ++it) {
         const uint32_t s = tile * kTile + tid;
         const bool valid = s < n;
         float v[16];
-        if (valid) {
-            const float4* xr = reinterpret_cast<const float4*>(x + (size_t)s * 16);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float4 f = __ldg(xr + q);
-                v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
-            }
-            v[15] = 1.0f;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0.0f;
-        }
+        load_input(x, s, n, v);
         store8(F, 8, tid, v);
         store8(F, 9, tid, v + 8);
         publish();
@@ -219,159 +363,176 @@ __global__ void __launch_bounds__(kThreads) k_mlp(const __nv_bfloat16* __restric
         tc::tmem_ld16(tlane + cAcc3, v);
 #pragma unroll
         for (int o = 0; o < 16; ++o) v[o] += sb3[o];
-        if constexpr (!kTrain) {
-            if (valid)
-                for (uint32_t o = 0; o < y_cols; ++o) y[(size_t)s * y_cols + o] = v[o];
-            tc::fence_before_sync();
-            __syncthreads();
-            tc::fence_after_sync();
-            continue;
-        } else {
-            // dL/dy of L = (1/n) sum w_o (y_o - t_o)^2
-            float tv[16];
-            if (valid) {
-                const float4* tr = reinterpret_cast<const float4*>(t + (size_t)s * 16);
+        // dL/dy of L = (1/n) sum w_o (y_o - t_o)^2
+        float tv[16];
+        if (valid) {
+            const float4* tr = reinterpret_cast<const float4*>(t + (size_t)s * 16);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float4 f = __ldg(tr + q);
-                    tv[4 * q] = f.x; tv[4 * q + 1] = f.y; tv[4 * q + 2] = f.z; tv[4 * q + 3] = f.w;
-                }
+            for (int q = 0; q < 4; ++q) {
+                const float4 f = __ldg(tr + q);
+                tv[4 * q] = f.x; tv[4 * q + 1] = f.y; tv[4 * q + 2] = f.z; tv[4 * q + 3] = f.w;
             }
-#pragma unroll
-            for (int o = 0; o < 16; ++o) {
-                float d = 0.0f;
-                if (valid) {
-                    const float e = v[o] - tv[o];
-                    const float w = __ldg(out_w + o);
-                    loss += w * e * e;
-                    d = bf16_round(coef * w * e);
-                }
-                db3[o] += d;
-                v[o] = d;
-            }
-            store8(Yb, 0, tid, v);
-            store8(Yb, 1, tid, v + 8);
-            publish();
-            // dH2 = dY [128 x 16] x W3 (W3 read MN-major)
-            if (tid == 0) {
-                tc::mma_bf16(tbase + cAcc2, tc::sdesc(sY, kCH, 128), tc::sdesc(sW3, 128, 256), id64_bmn, 0);
-                tc::commit(bar);
-            }
-            mma_wait();
-#pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                tc::tmem_ld16(tlane + cAcc2 + 16 * q, v);
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (!((mask2 >> (16 * q + i)) & 1ull)) v[i] = 0.0f;
-                store8(G, 8 + 2 * q, tid, v);
-                store8(G, 9 + 2 * q, tid, v + 8);
-            }
-            publish();
-            // dH1 = dH2 [128 x 64] x W2 (W2 read MN-major)
-            if (tid == 0) {
-#pragma unroll
-                for (uint32_t ks = 0; ks < 4; ++ks)
-                    tc::mma_bf16(tbase + cAcc1, tc::sdesc(sG + (8 + 2 * ks) * kCH, kCH, 128),
-                                 tc::sdesc(sW2 + ks * 256, 128, 1024), id64_bmn, ks > 0);
-                tc::commit(bar);
-            }
-            mma_wait();
-#pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                tc::tmem_ld16(tlane + cAcc1 + 16 * q, v);
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (!((mask1 >> (16 * q + i)) & 1ull)) v[i] = 0.0f;
-                store8(G, 16 + 2 * q, tid, v);
-                store8(G, 17 + 2 * q, tid, v + 8);
-            }
-            publish();
-            // weight gradients, reduced over the tile's samples (K = samples):
-            //   [dH2; dH1]^T-stack x [H1; X]  -> dW2 | db2 and dW1
-            //   [H2; dH2] x dY               -> dW3^T
-            if (tid == 0) {
-#pragma unroll
-                for (uint32_t ks = 0; ks < 8; ++ks) {
-                    const uint32_t acc = (it > 0 || ks > 0) ? 1u : 0u;
-                    tc::mma_bf16(tbase + cDA, tc::sdesc(sG + 8 * kCH + ks * 256, 128, kCH),
-                                 tc::sdesc(sF + ks * 256, 128, kCH), id80_mn, acc);
-                    tc::mma_bf16(tbase + cDB, tc::sdesc(sG + ks * 256, 128, kCH), tc::sdesc(sY + ks * 256, 128, kCH),
-                                 id16_mn, acc);
-                }
-                tc::commit(bar);
-            }
-            mma_wait();
         }
+#pragma unroll
+        for (int o = 0; o < 16; ++o) {
+            float d = 0.0f;
+            if (valid) {
+                const float e = v[o] - tv[o];
+                const float w = __ldg(out_w + o);
+                loss += w * e * e;
+                d = bf16_round(coef * w * e);
+            }
+            db3[o] += d;
+            v[o] = d;
+        }
+        store8(Yb, 0, tid, v);
+        store8(Yb, 1, tid, v + 8);
+        publish();
+        // dH2 = dY [128 x 16] x W3 (W3 read MN-major)
+        if (tid == 0) {
+            tc::mma_bf16(tbase + cAcc2, tc::sdesc(sY, kCH, 128), tc::sdesc(sW3, 128, 256), id64_bmn, 0);
+            tc::commit(bar);
+        }
+        mma_wait();
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            tc::tmem_ld16(tlane + cAcc2 + 16 * q, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (!((mask2 >> (16 * q + i)) & 1ull)) v[i] = 0.0f;
+            store8(G, 8 + 2 * q, tid, v);
+            store8(G, 9 + 2 * q, tid, v + 8);
+        }
+        publish();
+        // dH1 = dH2 [128 x 64] x W2 (W2 read MN-major)
+        if (tid == 0) {
+#pragma unroll
+            for (uint32_t ks = 0; ks < 4; ++ks)
+                tc::mma_bf16(tbase + cAcc1, tc::sdesc(sG + (8 + 2 * ks) * kCH, kCH, 128),
+                             tc::sdesc(sW2 + ks * 256, 128, 1024), id64_bmn, ks > 0);
+            tc::commit(bar);
+        }
+        mma_wait();
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            tc::tmem_ld16(tlane + cAcc1 + 16 * q, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (!((mask1 >> (16 * q + i)) & 1ull)) v[i] = 0.0f;
+            store8(G, 16 + 2 * q, tid, v);
+            store8(G, 17 + 2 * q, tid, v + 8);
+        }
+        publish();
+        // weight gradients, reduced over the tile's samples (K = samples):
+        //   [dH2; dH1]^T-stack x [H1; X]  -> dW2 | db2 and dW1
+        //   [H2; dH2] x dY               -> dW3^T
+        if (tid == 0) {
+#pragma unroll
+            for (uint32_t ks = 0; ks < 8; ++ks) {
+                const uint32_t acc = (it > 0 || ks > 0) ? 1u : 0u;
+                tc::mma_bf16(tbase + cDA, tc::sdesc(sG + 8 * kCH + ks * 256, 128, kCH),
+                             tc::sdesc(sF + ks * 256, 128, kCH), id80_mn, acc);
+                tc::mma_bf16(tbase + cDB, tc::sdesc(sG + ks * 256, 128, kCH), tc::sdesc(sY + ks * 256, 128, kCH),
+                             id16_mn, acc);
+            }
+            tc::commit(bar);
+        }
+        mma_wait();
     }
 
-    if constexpr (kTrain) {
-        float* part = partials + (size_t)blockIdx.x * kPartialStride;
-        float g[16];
-        if (warp < 2) {
-            const uint32_t i = 32 * warp + lane;   // hidden-2 unit (row of dW2, column of dW3)
+    // ---- the CTA's partial
+    float* part = partials + (size_t)blockIdx.x * kPartialStride;
+    float g[16];
+    if (warp < 2) {
+        const uint32_t i = 32 * warp + lane;   // hidden-2 unit (row of dW2, column of dW3)
 #pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                if (it > 0) tc::tmem_ld16(tlane + cDA + 16 * q, g);
+        for (uint32_t q = 0; q < 4; ++q) {
+            tc::tmem_ld16(tlane + cDA + 16 * q, g);
+            store16(part + kW2 + i * 64 + 16 * q, g);
+        }
+        tc::tmem_ld16(tlane + cDA + 64, g);
+        part[kB2 + i] = g[15];
+        tc::tmem_ld16(tlane + cDB, g);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) part[kW2 + i * 64 + 16 * q + j] = it > 0 ? g[j] : 0.0f;
+        for (int o = 0; o < 16; ++o) part[kW3 + o * 64 + i] = g[o];
+    } else {
+        const uint32_t i = 32 * (warp - 2) + lane;   // hidden-1 unit (row of dW1)
+        tc::tmem_ld16(tlane + cDA + 64, g);
+        store16(part + kW1 + i * 16, g);
+    }
+    // db3 and the loss: fixed-order warp trees, then the warps in order
+#pragma unroll
+    for (int o = 0; o < 17; ++o) {
+        float r = o < 16 ? db3[o] : loss;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
+        if (lane == 0) sred[warp * 17 + o] = r;
+    }
+    __syncthreads();
+    if (tid < 17) {
+        const float r = ((sred[tid] + sred[17 + tid]) + sred[34 + tid]) + sred[51 + tid];
+        part[tid < 16 ? kB3 + tid : kLossSlot] = tid < 16 ? r : r * coef * 0.5f;   // loss = sum / n
+    }
+}
+
+// Gradient, or a run of training steps: forward and backward over the CTA's tiles, one
+// partial per CTA, a grid barrier, the sum of the partials in CTA order with the Adam
+// update, and a barrier before the next step's weights.  As three launches a step (round
+// the weights, tiles, sum and update) a step of 8,192 samples took 23.4 us, of which the
+// sum's loads, four at a time, took 6.8; as steps of one cooperative launch it takes 12.1.
+// Takes steps [0, steps) of `plan`; with `grad` non-null a single step that leaves the
+// parameters alone.  The tiles' CTAs are the first `parts`; the others only sum.
+__global__ void __launch_bounds__(kThreads)
+k_mlp_train(float* params, const float* __restrict__ x, const float* __restrict__ t, const float* __restrict__ out_w,
+            const __grid_constant__ TrainPlan plan, float* partials, uint32_t parts, float* grad, float* losses,
+            float* m, float* v, uint32_t* barrier, uint32_t* __restrict__ error_flags) {
+    using L = TrainLayout;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::SLOT);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t n = plan.batch;
+    if (tid == 0) tc::mbar_init(reinterpret_cast<uint64_t*>(smem + L::BAR), 1);
+    if (warp == 0) tc::tmem_alloc(tslot, kTmemCols);
+    publish();
+    const uint32_t tbase = *tslot;
+    uint32_t phase = 0, offset = plan.offset;
+    for (uint32_t step = 0; step < plan.steps; ++step) {
+        if (offset + n > plan.samples) offset = 0;   // batches walk the (pre-shuffled) samples cyclically
+        if (blockIdx.x < parts)
+            train_tiles(smem, params, x + (size_t)offset * 16, t + (size_t)offset * 16, out_w, n, parts, tbase, phase,
+                        partials, error_flags);
+        offset += n;
+        if (step + 1 < plan.steps) {   // the next step's first tile, into L2 meanwhile
+            const uint32_t s = blockIdx.x * kTile + tid;
+            if (blockIdx.x < parts && s < n) {
+                const size_t at = ((size_t)(offset + n > plan.samples ? 0u : offset) + s) * 16;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(x + at));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(t + at));
             }
-            if (it > 0) tc::tmem_ld16(tlane + cDA + 64, g);
-            part[kB2 + i] = it > 0 ? g[15] : 0.0f;
-            if (it > 0) tc::tmem_ld16(tlane + cDB, g);
-#pragma unroll
-            for (int o = 0; o < 16; ++o) part[kW3 + o * 64 + i] = it > 0 ? g[o] : 0.0f;
-        } else {
-            const uint32_t i = 32 * (warp - 2) + lane;   // hidden-1 unit (row of dW1)
-            if (it > 0) tc::tmem_ld16(tlane + cDA + 64, g);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) part[kW1 + i * 16 + k] = it > 0 ? g[k] : 0.0f;
         }
-        // db3 and the loss: fixed-order warp trees, then the warps in order
-#pragma unroll
-        for (int o = 0; o < 17; ++o) {
-            float r = o < 16 ? db3[o] : loss;
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
-            if (lane == 0) sred[warp * 17 + o] = r;
+        grid_barrier(barrier, error_flags, gridDim.x);
+        // ---- sums in CTA order, and the Adam update
+        for (uint32_t i = blockIdx.x * kThreads + tid; i <= kLossSlot; i += gridDim.x * kThreads) {
+            float g = 0.0f;
+#pragma unroll 16
+            for (uint32_t c = 0; c < parts; ++c) g += __ldcg(partials + (size_t)c * kPartialStride + i);
+            if (grad) grad[i] = g;
+            if (i == kLossSlot) {
+                if (losses) losses[step] = g;
+            } else if (!grad) {
+                const float mi = plan.beta1 * m[i] + (1.0f - plan.beta1) * g;
+                const float vi = plan.beta2 * v[i] + (1.0f - plan.beta2) * g * g;
+                m[i] = mi;
+                v[i] = vi;
+                const float mh = mi / plan.bias[step].x, vh = vi / plan.bias[step].y;
+                params[i] = __ldcg(params + i) - plan.lr * mh / (sqrtf(vh) + plan.eps);
+            }
         }
-        __syncthreads();
-        if (tid < 17) {
-            const float r = ((sred[tid] + sred[17 + tid]) + sred[34 + tid]) + sred[51 + tid];
-            part[tid < 16 ? kB3 + tid : kLossSlot] = tid < 16 ? r : r * coef * 0.5f;   // loss = sum / n
-        }
+        if (step + 1 < plan.steps) grid_barrier(barrier, error_flags, gridDim.x);
     }
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_free(tbase, kTmemCols);
-}
-
-// f32 parameters -> bf16 weights (round to nearest even)
-__global__ void k_mlp_pack(const float* __restrict__ params, __nv_bfloat16* __restrict__ wts) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kWeights) wts[i] = __float2bfloat16_rn(params[i]);
-}
-
-// Sum of the per-CTA partials in CTA order; optionally one Adam step.
-__global__ void k_mlp_reduce_adam(const float* __restrict__ partials, uint32_t nparts, float* __restrict__ grad,
-                                  float* __restrict__ loss_out, float* __restrict__ params, float* __restrict__ m,
-                                  float* __restrict__ v, AdamStep a) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > kLossSlot) return;
-    float g = 0.0f;
-    for (uint32_t c = 0; c < nparts; ++c) g += partials[(size_t)c * kPartialStride + i];
-    if (grad) grad[i] = g;
-    if (i == kLossSlot) {
-        if (loss_out) *loss_out = g;
-        return;
-    }
-    if (!params) return;
-    const float mi = a.beta1 * m[i] + (1.0f - a.beta1) * g;
-    const float vi = a.beta2 * v[i] + (1.0f - a.beta2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    const float mh = mi / a.bias1, vh = vi / a.bias2;
-    params[i] -= a.lr * mh / (sqrtf(vh) + a.eps);
 }
 
 static int g_sm_count = 0;
@@ -379,9 +540,7 @@ static int g_sm_count = 0;
 static cudaError_t prepare_attributes() {
     static bool done = false;
     if (done) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(k_mlp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<true>::BYTES);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<false>::BYTES);
+    cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainLayout::BYTES);
     if (e == cudaSuccess) {
         int dev = 0;
         cudaGetDevice(&dev);
@@ -399,37 +558,37 @@ uint64_t scratch_bytes(uint32_t max_samples) {
 
 cudaError_t init(void) { return prepare_attributes(); }
 
-cudaError_t pack(const float* params, void* scratch, cudaStream_t s) {
-    k_mlp_pack<<<(kWeights + 255) / 256, 256, 0, s>>>(params, reinterpret_cast<__nv_bfloat16*>(scratch));
-    return cudaGetLastError();
-}
-
 cudaError_t forward(const float* params, const float* x, uint32_t n, const uint32_t* n_dev, uint32_t max_n, float* y,
-                    uint32_t y_cols, void* scratch, uint32_t* error_flags, cudaStream_t s) {
+                    uint32_t y_cols, uint32_t* error_flags, cudaStream_t s) {
     cudaError_t e = prepare_attributes();
     if (e != cudaSuccess) return e;
-    const uint32_t tiles = ((n_dev ? max_n : n) + kTile - 1) / kTile;
-    const uint32_t grid = std::max(1u, std::min<uint32_t>(tiles, 2u * (uint32_t)g_sm_count));
-    k_mlp<false><<<grid, kThreads, Layout<false>::BYTES, s>>>(reinterpret_cast<const __nv_bfloat16*>(scratch), params,
-                                                               x, n, n_dev, y, y_cols, nullptr, nullptr, nullptr,
-                                                               error_flags);
+    // as many tiles for every CTA, with all CTAs resident
+    const uint32_t tiles = std::max(1u, ((n_dev ? max_n : n) + kTile - 1) / kTile);
+    const uint32_t most = kForwardCtas * (uint32_t)g_sm_count;
+    const uint32_t each = (tiles + most - 1) / most;
+    k_mlp_forward<<<(tiles + each - 1) / each, kThreads, ForwardLayout::BYTES, s>>>(params, x, n, n_dev, y, y_cols,
+                                                                                    error_flags);
     return cudaGetLastError();
 }
 
-cudaError_t gradient(const float* params, const float* x, const float* t, const float* out_w, uint32_t n, void* scratch,
-                     float* grad, float* loss_out, float* m, float* v, float* update_params, const AdamStep& a,
-                     uint32_t* error_flags, cudaStream_t s) {
+cudaError_t train(float* params, const float* x, const float* t, const float* out_w, const TrainPlan& plan,
+                  void* scratch, float* grad, float* losses, float* m, float* v, uint32_t* error_flags, cudaStream_t s) {
     cudaError_t e = prepare_attributes();
     if (e != cudaSuccess) return e;
-    const uint32_t tiles = (n + kTile - 1) / kTile;
-    const uint32_t grid = std::max(1u, std::min<uint32_t>(tiles, (uint32_t)g_sm_count));
-    char* base = reinterpret_cast<char*>(scratch);
-    const __nv_bfloat16* wts = reinterpret_cast<const __nv_bfloat16*>(base);
-    float* partials = reinterpret_cast<float*>(base + align256((uint64_t)kWeights * 2));
-    k_mlp<true><<<grid, kThreads, Layout<true>::BYTES, s>>>(wts, params, x, n, nullptr, nullptr, 0, t, out_w, partials,
-                                                             error_flags);
-    k_mlp_reduce_adam<<<(kLossSlot + 256) / 256, 256, 0, s>>>(partials, grid, grad, loss_out, update_params, m, v, a);
-    return cudaGetLastError();
+    const uint32_t sms = (uint32_t)g_sm_count;
+    const uint32_t tiles = (plan.batch + kTile - 1) / kTile;
+    uint32_t parts = std::max(1u, std::min(tiles, sms));
+    // at least a thread per parameter for the sums
+    const uint32_t grid = std::max(parts, std::min(sms, (kLossSlot + kThreads) / kThreads));
+    uint32_t* barrier = reinterpret_cast<uint32_t*>(scratch);
+    float* partials = reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + 256);
+    e = cudaMemsetAsync(barrier, 0, sizeof(uint32_t), s);
+    if (e != cudaSuccess) return e;
+    TrainPlan by_value = plan;
+    void* args[] = {&params, &x,      &t, &out_w, &by_value, &partials,   &parts,
+                    &grad,   &losses, &m, &v,     &barrier,  &error_flags};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_mlp_train), dim3(grid), dim3(kThreads), args,
+                                       TrainLayout::BYTES, s);
 }
 
 }  // namespace mlp
@@ -467,8 +626,7 @@ MK_API int mk_op_mlp_forward(const float* params, const float* x, uint32_t n, fl
     if (mk::mlp::init() != cudaSuccess) return check_mlp(cudaGetLastError(), "mlp init");
     if (scratch_bytes < mk::mlp::scratch_bytes(n)) return bad_mlp("mlp forward: scratch too small");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    cudaError_t e = mk::mlp::pack(params, scratch, s);
-    if (e == cudaSuccess && n) e = mk::mlp::forward(params, x, n, nullptr, n, y, y_cols, scratch, error_flags, s);
+    const cudaError_t e = n ? mk::mlp::forward(params, x, n, nullptr, n, y, y_cols, error_flags, s) : cudaSuccess;
     return check_mlp(e, "mlp forward");
 }
 
@@ -482,11 +640,11 @@ MK_API int mk_op_mlp_gradient(const float* params, const float* x, const float* 
     if (mk::mlp::init() != cudaSuccess) return check_mlp(cudaGetLastError(), "mlp init");
     if (scratch_bytes < mk::mlp::scratch_bytes(n)) return bad_mlp("mlp gradient: scratch too small");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    mk::mlp::AdamStep a{0, 0, 0, 0, 1, 1};
-    cudaError_t e = mk::mlp::pack(params, scratch, s);
-    if (e == cudaSuccess)
-        e = mk::mlp::gradient(params, x, targets, out_weights, n, scratch, grad, nullptr, nullptr, nullptr, nullptr, a,
-                              error_flags, s);
+    mk::mlp::TrainPlan plan{};
+    plan.samples = plan.batch = n;
+    plan.steps = 1;
+    const cudaError_t e = mk::mlp::train(const_cast<float*>(params), x, targets, out_weights, plan, scratch, grad,
+                                         nullptr, nullptr, nullptr, error_flags, s);
     return check_mlp(e, "mlp gradient");
 }
 
@@ -504,17 +662,22 @@ MK_API int mk_op_mlp_train(float* params, float* adam_m, float* adam_v, const fl
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const float b1 = 0.9f, b2 = 0.999f;
     cudaError_t e = cudaSuccess;
-    uint32_t offset = 0;
-    for (uint32_t k = 0; k < steps && e == cudaSuccess; ++k) {
-        const float step = (float)(first_step + k + 1);
-        const mk::mlp::AdamStep a{lr, b1, b2, 1.0e-8f, 1.0f - std::pow(b1, step), 1.0f - std::pow(b2, step)};
-        if (offset + batch > n) offset = 0;   // batches walk the (pre-shuffled) samples cyclically
-        e = mk::mlp::pack(params, scratch, s);
-        if (e == cudaSuccess)
-            e = mk::mlp::gradient(params, x + (size_t)offset * 16, targets + (size_t)offset * 16, out_weights, batch,
-                                  scratch, nullptr, losses ? losses + k : nullptr, adam_m, adam_v, params, a,
-                                  error_flags, s);
-        offset += batch;
+    mk::mlp::TrainPlan plan{};
+    plan.samples = n;
+    plan.batch = batch;
+    plan.lr = lr;
+    plan.beta1 = b1;
+    plan.beta2 = b2;
+    plan.eps = 1.0e-8f;
+    for (uint32_t k = 0; k < steps && e == cudaSuccess; k += plan.steps) {
+        plan.steps = std::min(steps - k, mk::mlp::kPlanSteps);
+        for (uint32_t j = 0; j < plan.steps; ++j) {
+            const float step = (float)(first_step + k + j + 1);
+            plan.bias[j] = make_float2(1.0f - std::pow(b1, step), 1.0f - std::pow(b2, step));
+        }
+        e = mk::mlp::train(params, x, targets, out_weights, plan, scratch, nullptr, losses ? losses + k : nullptr,
+                           adam_m, adam_v, error_flags, s);
+        for (uint32_t j = 0; j < plan.steps; ++j) plan.offset = (plan.offset + batch > n ? 0u : plan.offset) + batch;
     }
     return check_mlp(e, "mlp train");
 }

@@ -16,23 +16,25 @@ constexpr uint32_t kB2 = 6144, kB3 = 6208, kParams = 6224;
 constexpr uint32_t kLossSlot = kParams;           // gradient arrays carry the loss after the parameters
 constexpr uint32_t kPartialStride = 6240;         // floats per CTA partial
 
-struct AdamStep {
+// Steps of one training launch: step k takes the `batch` samples from the running offset
+// (from 0 again where they would pass `samples`).
+constexpr uint32_t kPlanSteps = 256;
+struct TrainPlan {
+    uint32_t samples, batch, offset, steps;
     float lr, beta1, beta2, eps;
-    float bias1, bias2;   // 1 - beta^step
+    float2 bias[kPlanSteps];   // per step: 1 - beta1^step, 1 - beta2^step
 };
 
 cudaError_t init(void);   // function attributes; call once outside stream capture
 uint64_t scratch_bytes(uint32_t max_samples);
-// bf16 weights into scratch (first kWeights * 2 bytes); run after every parameter change.
-cudaError_t pack(const float* params, void* scratch, cudaStream_t s);
 // y[n][y_cols] = net(x[n][16]); n from n_dev when non-null (then max_n bounds the grid).
 cudaError_t forward(const float* params, const float* x, uint32_t n, const uint32_t* n_dev, uint32_t max_n, float* y,
-                    uint32_t y_cols, void* scratch, uint32_t* error_flags, cudaStream_t s);
-// Gradient of (1/n) sum_s sum_o out_w[o] (y_so - t_so)^2 into grad[kParams + 1] (loss last);
-// with update_params non-null, one Adam step on update_params (moments m, v).
-cudaError_t gradient(const float* params, const float* x, const float* t, const float* out_w, uint32_t n, void* scratch,
-                     float* grad, float* loss_out, float* m, float* v, float* update_params, const AdamStep& a,
-                     uint32_t* error_flags, cudaStream_t s);
+                    uint32_t y_cols, uint32_t* error_flags, cudaStream_t s);
+// Each step's gradient of (1/batch) sum_s sum_o out_w[o] (y_so - t_so)^2 and one Adam step on
+// the parameters (moments m, v), its loss into losses[step].  With `grad` non-null (one step):
+// the gradient into grad[kParams + 1] (loss last), and no update.
+cudaError_t train(float* params, const float* x, const float* t, const float* out_w, const TrainPlan& plan, void* scratch,
+                  float* grad, float* losses, float* m, float* v, uint32_t* error_flags, cudaStream_t s);
 
 }  // namespace mlp
 }  // namespace mk
