@@ -63,15 +63,24 @@ struct TrainLayout {
 };
 // Forward only: X, H1 and H2 take one another's place in one tile of 8 chunks (each is
 // dead once the MMAs of its layer are complete), and the three accumulators the same 64
-// TMEM columns, so that 7 CTAs fit on an SM.
-constexpr uint32_t kForwardTmem = 64, kForwardCtas = 7;
+// TMEM columns, so that 8 tiles are worked on beside one another on an SM.
+constexpr uint32_t kForwardTmem = 64, kForwardGroups = 8;   // columns of a tile, tiles of a CTA
 struct ForwardLayout {
-    static constexpr uint32_t H = 0;
-    using W = WeightLayout<8 * kCH>;
-    static constexpr uint32_t BAR = W::END;
-    static constexpr uint32_t SLOT = BAR + 8;
-    static constexpr uint32_t BYTES = SLOT + 8;
+    using W = WeightLayout<0>;
+    static constexpr uint32_t BAR = W::END;                // one mbarrier per tile
+    static constexpr uint32_t SLOT = BAR + 8 * kForwardGroups;
+    static constexpr uint32_t H = (SLOT + 8 + 1023) / 1024 * 1024;   // 8 chunks per tile
+    static constexpr uint32_t bytes(uint32_t groups) { return H + groups * 8 * kCH; }
 };
+// A training CTA waits for its peers, so no CTA on its SM may hold it up at the TMEM allocation
+// while that one waits for another training launch.  It asks for so much shared memory that
+// it never shares an SM with a forward CTA of 512 columns; beside what fits with it, the
+// columns are there or come free with a forward CTA that already has its own.
+constexpr uint32_t kSmShared = 233472, kCtaReserved = 1024;   // bytes of an SM, of each CTA beyond its own
+constexpr uint32_t kTrainBytes =
+    std::max(TrainLayout::BYTES, kSmShared - ForwardLayout::bytes(kForwardGroups) - 2 * kCtaReserved + 1024);
+static_assert(2 * (kTrainBytes + kCtaReserved) <= kSmShared && 3 * (kTrainBytes + kCtaReserved) > kSmShared,
+              "two training CTAs per SM, which have 512 columns between them");
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
@@ -91,40 +100,56 @@ __device__ __forceinline__ void publish() {
     __syncthreads();
     tc::fence_after_sync();
 }
+// The same among the 128 threads of one tile of the CTA.
+__device__ __forceinline__ void group_sync(uint32_t group) {
+    tc::fence_before_sync();
+    asm volatile("bar.sync %0, 128;" ::"r"(group + 1u) : "memory");
+    tc::fence_after_sync();
+}
+__device__ __forceinline__ void publish(uint32_t group) {
+    tc::fence_async_smem();
+    group_sync(group);
+}
 
 // Weights (rounded to bf16) into the core-matrix layout, W1 64 rows x 2 chunks, W2 64 x 8,
 // W3 16 x 8, and the biases.  Units of 8 consecutive parameters are one row of a chunk.
 // Read past L1: a training launch rewrites the parameters between its steps.
-template <class W>
-__device__ __forceinline__ void load_weights(unsigned char* smem, const float* params, uint32_t tid) {
-    constexpr uint32_t kUnits = kWeights / 8 / kThreads;
-    float w[kUnits][8];
-    if ((reinterpret_cast<uintptr_t>(params) & 15u) == 0) {
+template <class W, uint32_t kUnits, uint32_t kBlock>   // kBlock: threads of the CTA, 0 if known at the launch only
+__device__ __forceinline__ void load_weights(unsigned char* smem, const float* params) {
+    const bool rows16 = (reinterpret_cast<uintptr_t>(params) & 15u) == 0;
+    const uint32_t block = kBlock ? kBlock : blockDim.x;
+    constexpr bool kExact = kBlock != 0 && kWeights / 8 % (kUnits * kBlock + (kBlock == 0)) == 0;
+    for (uint32_t u0 = 0; u0 < kWeights / 8; u0 += kUnits * block) {
+        float w[kUnits][8];
 #pragma unroll
         for (uint32_t k = 0; k < kUnits; ++k) {
-            const float4* q = reinterpret_cast<const float4*>(params + 8 * (tid + k * kThreads));
-            const float4 lo = __ldcg(q), hi = __ldcg(q + 1);
-            w[k][0] = lo.x; w[k][1] = lo.y; w[k][2] = lo.z; w[k][3] = lo.w;
-            w[k][4] = hi.x; w[k][5] = hi.y; w[k][6] = hi.z; w[k][7] = hi.w;
+            const uint32_t u = u0 + k * block + threadIdx.x;
+            if (!kExact && u >= kWeights / 8) continue;
+            if (rows16) {
+                const float4* q = reinterpret_cast<const float4*>(params + 8 * u);
+                const float4 lo = __ldcg(q), hi = __ldcg(q + 1);
+                w[k][0] = lo.x; w[k][1] = lo.y; w[k][2] = lo.z; w[k][3] = lo.w;
+                w[k][4] = hi.x; w[k][5] = hi.y; w[k][6] = hi.z; w[k][7] = hi.w;
+            } else {
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) w[k][i] = __ldcg(params + 8 * u + i);
+            }
         }
-    } else {
 #pragma unroll
-        for (uint32_t k = 0; k < kUnits; ++k)
-#pragma unroll
-            for (uint32_t i = 0; i < 8; ++i) w[k][i] = __ldcg(params + 8 * (tid + k * kThreads) + i);
+        for (uint32_t k = 0; k < kUnits; ++k) {
+            const uint32_t u = u0 + k * block + threadIdx.x;
+            if (!kExact && u >= kWeights / 8) continue;
+            uint32_t at;
+            if (u < 128) at = W::W1 + (u & 1u) * 1024 + (u >> 4) * 128 + ((u >> 1) & 7u) * 16;
+            else if (u < 640) at = W::W2 + (u & 7u) * 1024 + ((u - 128) >> 6) * 128 + ((u >> 3) & 7u) * 16;
+            else at = W::W3 + (u & 7u) * 256 + ((u - 640) >> 6) * 128 + ((u >> 3) & 7u) * 16;
+            *reinterpret_cast<uint4*>(smem + at) =
+                make_uint4(pack_bf16(w[k][0], w[k][1]), pack_bf16(w[k][2], w[k][3]), pack_bf16(w[k][4], w[k][5]),
+                           pack_bf16(w[k][6], w[k][7]));
+        }
     }
-#pragma unroll
-    for (uint32_t k = 0; k < kUnits; ++k) {
-        const uint32_t u = tid + k * kThreads;
-        uint32_t at;
-        if (u < 128) at = W::W1 + (u & 1u) * 1024 + (u >> 4) * 128 + ((u >> 1) & 7u) * 16;
-        else if (u < 640) at = W::W2 + (u & 7u) * 1024 + ((u - 128) >> 6) * 128 + ((u >> 3) & 7u) * 16;
-        else at = W::W3 + (u & 7u) * 256 + ((u - 640) >> 6) * 128 + ((u >> 3) & 7u) * 16;
-        *reinterpret_cast<uint4*>(smem + at) = make_uint4(pack_bf16(w[k][0], w[k][1]), pack_bf16(w[k][2], w[k][3]),
-                                                          pack_bf16(w[k][4], w[k][5]), pack_bf16(w[k][6], w[k][7]));
-    }
-    if (tid < 64) reinterpret_cast<float*>(smem + W::B2)[tid] = __ldcg(params + kB2 + tid);
-    if (tid < 16) reinterpret_cast<float*>(smem + W::B3)[tid] = __ldcg(params + kB3 + tid);
+    if (threadIdx.x < 64) reinterpret_cast<float*>(smem + W::B2)[threadIdx.x] = __ldcg(params + kB2 + threadIdx.x);
+    if (threadIdx.x < 16) reinterpret_cast<float*>(smem + W::B3)[threadIdx.x] = __ldcg(params + kB3 + threadIdx.x);
 }
 
 // One sample's inputs (slot 15 is the constant 1); zeros past the end.
@@ -144,29 +169,35 @@ __device__ __forceinline__ void load_input(const float* __restrict__ x, uint32_t
 }
 
 // Forward pass.  A tile is a chain (inputs, three times MMA, read-back, ReLU and store)
-// that leaves the SM idle unless other tiles run beside it: with 2 CTAs per SM (256 TMEM
-// columns, 49 KB) 300,001 samples took 51 us, 6.4 us a tile; with 7, and the next tile's
-// inputs loaded during this one's first layer, 28 (24.6 in a run of calls, 48.1 before).
-__global__ void __launch_bounds__(kThreads, kForwardCtas)
+// that leaves the SM idle unless other tiles run beside it, so a CTA has up to 8 groups of
+// 128 threads with a tile each, which share the weights.  300,001 samples: 51 us with 2
+// CTAs of one tile per SM; 28 with 7, whose start is held up (until a CTA has given up its
+// right to allocate TMEM, its SM starts no other: 0.75 us between them, 2.5 with the weights
+// loaded first); one CTA of 8 tiles, with the next inputs loaded during layer 1, 18
+// (16.4 in a run of calls, where the first form took 48.1 and the second 24.6).
+__global__ void __launch_bounds__(kThreads * kForwardGroups)
 k_mlp_forward(const float* params, const float* __restrict__ x, uint32_t n_host, const uint32_t* n_dev,
               float* __restrict__ y, uint32_t y_cols, uint32_t* __restrict__ error_flags) {
     using L = ForwardLayout;
     extern __shared__ __align__(1024) unsigned char smem[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + L::SLOT);
     const float* sb2 = reinterpret_cast<const float*>(smem + L::W::B2);
     const float* sb3 = reinterpret_cast<const float*>(smem + L::W::B3);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t group = threadIdx.x / kThreads, groups = blockDim.x / kThreads;
+    const uint32_t tid = threadIdx.x % kThreads, warp = tid >> 5;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR) + group;
+    unsigned char* H = smem + L::H + group * 8 * kCH;
     const uint32_t n = n_dev ? *n_dev : n_host;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     if (blockIdx.x >= tiles) return;
+    if (threadIdx.x < 32) tc::tmem_alloc(tslot, kForwardTmem * groups);
+    const uint32_t first = blockIdx.x + group * gridDim.x, stride = groups * gridDim.x;
     float next[16];
-    load_input(x, blockIdx.x * kTile + tid, n, next);
-    load_weights<L::W>(smem, params, tid);
+    if (first < tiles) load_input(x, first * kTile + tid, n, next);
     if (tid == 0) tc::mbar_init(bar, 1);
-    if (warp == 0) tc::tmem_alloc(tslot, kForwardTmem);
+    load_weights<L::W, 1, 0>(smem, params);
     publish();
-    const uint32_t tbase = *tslot;
+    const uint32_t tbase = *tslot + kForwardTmem * group;
     const uint32_t tlane = tbase + ((32u * warp) << 16);
     uint32_t phase = 0;
     bool timed_out = false;
@@ -178,23 +209,23 @@ k_mlp_forward(const float* params, const float* __restrict__ x, uint32_t n_host,
         phase ^= 1u;
         tc::fence_after_sync();
     };
-    const uint32_t sH = tc::smem_u32(smem + L::H);
+    const uint32_t sH = tc::smem_u32(H);
     const uint32_t sW1 = tc::smem_u32(smem + L::W::W1), sW2 = tc::smem_u32(smem + L::W::W2);
     const uint32_t sW3 = tc::smem_u32(smem + L::W::W3);
     constexpr uint32_t id64 = tc::idesc_bf16(128, 64, false, false);
     constexpr uint32_t id16 = tc::idesc_bf16(128, 16, false, false);
     const bool rows4 = (y_cols & 3u) == 0u && (reinterpret_cast<uintptr_t>(y) & 15u) == 0;
-    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    for (uint32_t tile = first; tile < tiles; tile += stride) {
         const uint32_t s = tile * kTile + tid;
-        store8(smem + L::H, 0, tid, next);
-        store8(smem + L::H, 1, tid, next + 8);
-        publish();
+        store8(H, 0, tid, next);
+        store8(H, 1, tid, next + 8);
+        publish(group);
         // layer 1: [128 x 16] x W1^T
         if (tid == 0) {
             tc::mma_bf16(tbase, tc::sdesc(sH, kCH, 128), tc::sdesc(sW1, 1024, 128), id64, 0);
             tc::commit(bar);
         }
-        if (tile + gridDim.x < tiles) load_input(x, s + gridDim.x * kTile, n, next);
+        if (tile + stride < tiles) load_input(x, s + stride * kTile, n, next);
         mma_wait();
         float v[16];
 #pragma unroll
@@ -202,10 +233,10 @@ k_mlp_forward(const float* params, const float* __restrict__ x, uint32_t n_host,
             tc::tmem_ld16(tlane + 16 * q, v);
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = v[i] > 0.0f ? v[i] : 0.0f;
-            store8(smem + L::H, 2 * q, tid, v);
-            store8(smem + L::H, 2 * q + 1, tid, v + 8);
+            store8(H, 2 * q, tid, v);
+            store8(H, 2 * q + 1, tid, v + 8);
         }
-        publish();
+        publish(group);
         // layer 2: H1 [128 x 64] x W2^T
         if (tid == 0) {
 #pragma unroll
@@ -223,10 +254,10 @@ k_mlp_forward(const float* params, const float* __restrict__ x, uint32_t n_host,
                 v[i] += sb2[16 * q + i];
                 v[i] = v[i] > 0.0f ? v[i] : 0.0f;
             }
-            store8(smem + L::H, 2 * q, tid, v);
-            store8(smem + L::H, 2 * q + 1, tid, v + 8);
+            store8(H, 2 * q, tid, v);
+            store8(H, 2 * q + 1, tid, v + 8);
         }
-        publish();
+        publish(group);
         // layer 3: H2 [128 x 64] x W3^T
         if (tid == 0) {
 #pragma unroll
@@ -252,11 +283,11 @@ k_mlp_forward(const float* params, const float* __restrict__ x, uint32_t n_host,
                     if (o < y_cols) row[o] = v[o];
             }
         }
-        tc::fence_before_sync();
-        __syncthreads();   // the accumulator is read by all before the next tile's layer 1 overwrites it
-        tc::fence_after_sync();
+        group_sync(group);   // the accumulator is read by all before the next tile's layer 1 overwrites it
     }
-    if (warp == 0) tc::tmem_free(tbase, kForwardTmem);
+    tc::fence_before_sync();
+    __syncthreads();
+    if (threadIdx.x < 32) tc::tmem_free(*tslot, kForwardTmem * groups);
 }
 
 __device__ __forceinline__ void store16(float* at, const float* v) {
@@ -294,28 +325,38 @@ __device__ __forceinline__ void train_tiles(unsigned char* smem, const float* pa
     constexpr uint32_t id80_mn = tc::idesc_bf16(128, 80, true, true);
     constexpr uint32_t id16_mn = tc::idesc_bf16(128, 16, true, true);
 
-    load_weights<L::W>(smem, params, tid);
     const float coef = n > 0 ? 2.0f / (float)n : 0.0f;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     float loss = 0.0f;
     float db3[16];
 #pragma unroll
     for (int o = 0; o < 16; ++o) db3[o] = 0.0f;
+    float next[16];
+    load_input(x, blockIdx.x * kTile + tid, n, next);
+    load_weights<L::W, kWeights / 8 / kThreads, kThreads>(smem, params);
     uint32_t it = 0;
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += parts, ++it) {
         const uint32_t s = tile * kTile + tid;
         const bool valid = s < n;
-        float v[16];
-        load_input(x, s, n, v);
-        store8(F, 8, tid, v);
-        store8(F, 9, tid, v + 8);
+        store8(F, 8, tid, next);
+        store8(F, 9, tid, next + 8);
         publish();
         // layer 1: [128 x 16] x W1^T
         if (tid == 0) {
             tc::mma_bf16(tbase + cAcc1, tc::sdesc(sF + 8 * kCH, kCH, 128), tc::sdesc(sW1, 1024, 128), id64, 0);
             tc::commit(bar);
         }
+        float tv[16];
+        if (valid) {
+            const float4* tr = reinterpret_cast<const float4*>(t + (size_t)s * 16);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 f = __ldg(tr + q);
+                tv[4 * q] = f.x; tv[4 * q + 1] = f.y; tv[4 * q + 2] = f.z; tv[4 * q + 3] = f.w;
+            }
+        }
         mma_wait();
+        float v[16];
         uint64_t mask1 = 0, mask2 = 0;
 #pragma unroll
         for (uint32_t q = 0; q < 4; ++q) {
@@ -364,15 +405,6 @@ __device__ __forceinline__ void train_tiles(unsigned char* smem, const float* pa
 #pragma unroll
         for (int o = 0; o < 16; ++o) v[o] += sb3[o];
         // dL/dy of L = (1/n) sum w_o (y_o - t_o)^2
-        float tv[16];
-        if (valid) {
-            const float4* tr = reinterpret_cast<const float4*>(t + (size_t)s * 16);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float4 f = __ldg(tr + q);
-                tv[4 * q] = f.x; tv[4 * q + 1] = f.y; tv[4 * q + 2] = f.z; tv[4 * q + 3] = f.w;
-            }
-        }
 #pragma unroll
         for (int o = 0; o < 16; ++o) {
             float d = 0.0f;
@@ -437,6 +469,7 @@ __device__ __forceinline__ void train_tiles(unsigned char* smem, const float* pa
             }
             tc::commit(bar);
         }
+        if (tile + parts < tiles) load_input(x, s + parts * kTile, n, next);
         mma_wait();
     }
 
@@ -477,9 +510,11 @@ __device__ __forceinline__ void train_tiles(unsigned char* smem, const float* pa
 
 // Gradient, or a run of training steps: forward and backward over the CTA's tiles, one
 // partial per CTA, a grid barrier, the sum of the partials in CTA order with the Adam
-// update, and a barrier before the next step's weights.  As three launches a step (round
-// the weights, tiles, sum and update) a step of 8,192 samples took 23.4 us, of which the
-// sum's loads, four at a time, took 6.8; as steps of one cooperative launch it takes 12.1.
+// update, and a barrier before the next step's weights.  Bound by latency: six MMAs and
+// read-backs in a chain, the sums over up to 148 partials, two barriers.  As three launches a
+// step (round the weights, tiles, sum and update) a step of 8,192 samples took 23.4 us, of
+// which the sum's loads, four at a time, took 6.8; as steps of one cooperative launch, with
+// 32 loads at a time and the inputs loaded ahead, it takes 11.
 // Takes steps [0, steps) of `plan`; with `grad` non-null a single step that leaves the
 // parameters alone.  The tiles' CTAs are the first `parts`; the others only sum.
 __global__ void __launch_bounds__(kThreads)
@@ -513,19 +548,20 @@ k_mlp_train(float* params, const float* __restrict__ x, const float* __restrict_
         grid_barrier(barrier, error_flags, gridDim.x);
         // ---- sums in CTA order, and the Adam update
         for (uint32_t i = blockIdx.x * kThreads + tid; i <= kLossSlot; i += gridDim.x * kThreads) {
+            const bool update = !grad && i != kLossSlot;
+            const float m0 = update ? m[i] : 0.0f, v0 = update ? v[i] : 0.0f, p0 = update ? __ldcg(params + i) : 0.0f;
             float g = 0.0f;
-#pragma unroll 16
+#pragma unroll 32
             for (uint32_t c = 0; c < parts; ++c) g += __ldcg(partials + (size_t)c * kPartialStride + i);
             if (grad) grad[i] = g;
-            if (i == kLossSlot) {
-                if (losses) losses[step] = g;
-            } else if (!grad) {
-                const float mi = plan.beta1 * m[i] + (1.0f - plan.beta1) * g;
-                const float vi = plan.beta2 * v[i] + (1.0f - plan.beta2) * g * g;
+            if (i == kLossSlot && losses) losses[step] = g;
+            if (update) {
+                const float mi = plan.beta1 * m0 + (1.0f - plan.beta1) * g;
+                const float vi = plan.beta2 * v0 + (1.0f - plan.beta2) * g * g;
                 m[i] = mi;
                 v[i] = vi;
                 const float mh = mi / plan.bias[step].x, vh = vi / plan.bias[step].y;
-                params[i] = __ldcg(params + i) - plan.lr * mh / (sqrtf(vh) + plan.eps);
+                params[i] = p0 - plan.lr * mh / (sqrtf(vh) + plan.eps);
             }
         }
         if (step + 1 < plan.steps) grid_barrier(barrier, error_flags, gridDim.x);
@@ -540,7 +576,10 @@ static int g_sm_count = 0;
 static cudaError_t prepare_attributes() {
     static bool done = false;
     if (done) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainLayout::BYTES);
+    cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainBytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 ForwardLayout::bytes(kForwardGroups));
     if (e == cudaSuccess) {
         int dev = 0;
         cudaGetDevice(&dev);
@@ -562,12 +601,13 @@ cudaError_t forward(const float* params, const float* x, uint32_t n, const uint3
                     uint32_t y_cols, uint32_t* error_flags, cudaStream_t s) {
     cudaError_t e = prepare_attributes();
     if (e != cudaSuccess) return e;
-    // as many tiles for every CTA, with all CTAs resident
+    // one CTA per SM, with as many tiles beside one another (1, 2, 4 or 8) as there are for it
     const uint32_t tiles = std::max(1u, ((n_dev ? max_n : n) + kTile - 1) / kTile);
-    const uint32_t most = kForwardCtas * (uint32_t)g_sm_count;
-    const uint32_t each = (tiles + most - 1) / most;
-    k_mlp_forward<<<(tiles + each - 1) / each, kThreads, ForwardLayout::BYTES, s>>>(params, x, n, n_dev, y, y_cols,
-                                                                                    error_flags);
+    const uint32_t grid = std::min(tiles, (uint32_t)g_sm_count);
+    uint32_t groups = 1;
+    while (groups < kForwardGroups && groups * grid < tiles) groups *= 2;
+    k_mlp_forward<<<grid, kThreads * groups, ForwardLayout::bytes(groups), s>>>(params, x, n, n_dev, y, y_cols,
+                                                                                error_flags);
     return cudaGetLastError();
 }
 
@@ -588,7 +628,7 @@ cudaError_t train(float* params, const float* x, const float* t, const float* ou
     void* args[] = {&params, &x,      &t, &out_w, &by_value, &partials,   &parts,
                     &grad,   &losses, &m, &v,     &barrier,  &error_flags};
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_mlp_train), dim3(grid), dim3(kThreads), args,
-                                       TrainLayout::BYTES, s);
+                                       kTrainBytes, s);
 }
 
 }  // namespace mlp

@@ -1,5 +1,5 @@
-"""The network's launches at their edges: forward passes around one and two tiles per
-resident CTA and at every row width, parameters that are only 4-byte aligned, and training
+"""The network's launches at their edges: forward passes around 1, 2, 4 and 8 tiles beside one
+another per CTA and at several row widths, parameters that are only 4-byte aligned, and training
 runs of more steps than one launch takes."""
 import pytest
 import torch
@@ -10,11 +10,11 @@ from test_gpu_mlp import _data, _params
 
 pytestmark = pytest.mark.gpu
 
-RESIDENT = 7 * 148 * 128   # samples of one tile for every resident CTA
+WAVE = 148 * 128   # samples of one tile per SM
 
 
-@pytest.mark.parametrize("n,cols", [(RESIDENT, 1), (RESIDENT + 1, 3), (2 * RESIDENT + 129, 4), (1000, 8), (129, 15),
-                                    (257, 12)])
+@pytest.mark.parametrize("n,cols", [(WAVE, 1), (WAVE + 1, 3), (2 * WAVE + 1, 4), (4 * WAVE, 5), (4 * WAVE + 1, 2),
+                                    (8 * WAVE + 129, 4), (17 * WAVE + 5, 1), (1000, 8), (129, 15), (257, 12)])
 def test_forward_tiles_and_row_widths(cuda_lib, n, cols):
     """A sample's outputs depend neither on its tile's place nor on the row width: the same
     bits as in calls of 1,000 samples and 16 columns."""
