@@ -330,7 +330,8 @@ constexpr uint32_t kLeafCode = 0x80000000u;
 // come from prefix/suffix unions within 32-leaf chunks (warp scans), within
 // 1024-leaf super-chunks (over chunk totals) and a sparse table over the
 // super-chunk totals.
-constexpr uint32_t kRefitBlock = 1024;   // one super-chunk of 32 chunks per block
+constexpr uint32_t kRefitBlock = 1024;     // leaves per block: one super-chunk of 32 chunks
+constexpr uint32_t kRefitThreads = 512;    // each warp takes two chunks, two blocks share an SM
 
 struct Box2 {
     float4 mn, mx;
@@ -391,7 +392,7 @@ struct TravEntry {
     Box2 box;
     uint32_t code, last;
 };
-__device__ __forceinline__ void store_record(float4* rec, const TravEntry (&e)[4], uint32_t m) {
+__device__ __forceinline__ void fill_record(float4 (&rec)[8], const TravEntry (&e)[4], uint32_t m) {
 #pragma unroll
     for (uint32_t k = 0; k < 4; ++k) {
         if (k < m) {
@@ -403,6 +404,36 @@ __device__ __forceinline__ void store_record(float4* rec, const TravEntry (&e)[4
         }
     }
 }
+__device__ __forceinline__ void store_record(float4* dst, const TravEntry (&e)[4], uint32_t m) {
+    float4 rec[8];
+    fill_record(rec, e, m);
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) dst[k] = rec[k];
+}
+
+// A warp's rows of Q float4, lane l's to dst + Q l where `rows` has bit l, by way of
+// shared memory (128 float4 per warp): neighbouring lanes write neighbouring sectors, where
+// a row per lane takes a line of its own for each lane and leaves every sector half written.
+template <uint32_t Q>
+__device__ __forceinline__ void store_rows(float4* stage, const float4 (&v)[Q], float4* dst, uint32_t rows,
+                                           uint32_t lane) {
+    constexpr uint32_t kRows = Q == 8 ? 16 : 32;   // rows at a time
+    auto at = [](uint32_t row, uint32_t q) { return row * Q + (q ^ ((row / (8 / Q)) & (Q - 1))); };   // bank-free
+#pragma unroll
+    for (uint32_t r0 = 0; r0 < 32; r0 += kRows) {
+        __syncwarp();
+        if (lane - r0 < kRows) {
+#pragma unroll
+            for (uint32_t q = 0; q < Q; ++q) stage[at(lane - r0, q)] = v[q];
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t k = 0; k < kRows * Q / 32; ++k) {
+            const uint32_t i = k * 32 + lane, row = i / Q;
+            if ((rows >> (r0 + row)) & 1u) dst[r0 * Q + i] = stage[at(row, i % Q)];
+        }
+    }
+}
 
 // Traversal records of the in-chunk nodes, written by the warp that owns the
 // chunk: every descendant of a node whose leaf range lies in one 32-leaf
@@ -411,9 +442,10 @@ __device__ __forceinline__ void store_record(float4* rec, const TravEntry (&e)[4
 // the lane of the node or leaf -- no global reads besides the node's own
 // children.  `v`/`j` are this lane's leaf box and collider index, `r` its
 // node's box (valid where `inner`).  Every lane takes part in the shuffles.
-__device__ __forceinline__ void write_chunk_records(const StepBuffers& b, bool inner, uint2 rg, Box2 r, Box2 v,
-                                                    uint32_t j, uint32_t t, uint32_t leaf_base, uint32_t lane) {
-    const uint2 ch = inner ? b.children[t] : make_uint2(0u, 0u);
+__device__ __forceinline__ void write_chunk_records(const StepBuffers& b, bool inner, uint2 rg, uint2 ch, Box2 r, Box2 v,
+                                                    uint32_t j, uint32_t t, uint32_t leaf_base, uint32_t lane,
+                                                    float4* stage) {
+    if (!inner) ch = make_uint2(0u, 0u);
     const Box2 nb = inner ? r : box_empty();
     auto lane_of_node = [&](uint32_t c) { return inner && c < leaf_base ? (c & 31u) : lane; };
     const uint32_t lx = lane_of_node(ch.x), ly = lane_of_node(ch.y);
@@ -447,7 +479,9 @@ __device__ __forceinline__ void write_chunk_records(const StepBuffers& b, bool i
     // compact in leaf order: a leaf child leaves its second slot empty
     const bool li = use[1], ri = use[3];
     const TravEntry e[4] = {sl[0], li ? sl[1] : sl[2], li ? sl[2] : sl[3], sl[3]};
-    if (inner) store_record(b.node_records + 8ull * t, e, (li ? 2u : 1u) + (ri ? 2u : 1u));
+    float4 rec[8];
+    fill_record(rec, e, (li ? 2u : 1u) + (ri ? 2u : 1u));
+    store_rows<8>(stage, rec, b.node_records + 8ull * (t - lane), __ballot_sync(0xffffffffu, inner), lane);
 }
 
 // Leaf boxes in sorted order, their prefix/suffix unions within 32-leaf chunks,
@@ -456,60 +490,77 @@ __device__ __forceinline__ void write_chunk_records(const StepBuffers& b, bool i
 // leaf i owns node i), the chunks' prefix/suffix unions and sparse table within
 // the block's super-chunk, and the super-chunk's total (level 0 of the sparse
 // table over super-chunks).
-__global__ void __launch_bounds__(kRefitBlock) k_refit_leaves(StepBuffers b, StepParams p) {
+// Bound by the latency of each chunk's chain (collider index, its box, the scans, the
+// range unions) and by the load-store unit.  On 401,946 colliders it took 47 us with 1,024
+// threads per block (alone on their SM, idle while one warp does the block's last part), a
+// row stored per lane and the nodes listed by an atomic per warp; 40 with 512 threads, rows
+// through shared memory and an atomic per block.
+__global__ void __launch_bounds__(kRefitThreads, 2) k_refit_leaves(StepBuffers b, StepParams p) {
     __shared__ Box2 s_chunk[32];
+    __shared__ uint32_t s_cross[32];
+    __shared__ __align__(16) float4 s_stage[kRefitThreads / 32][128];
     const uint32_t n = p.collider_count;
-    const uint32_t t = blockIdx.x * kRefitBlock + threadIdx.x;
     const uint32_t lane = lane_id(), w = warp_id();
     const uint32_t leaf_base = n - 1;
-    Box2 v = box_empty();
-    const uint32_t j = t < n ? b.svals[t] : 0u;
-    if (t < n) {
-        float4 mn = b.aabbs[2ull * j], mx = b.aabbs[2ull * j + 1];
-        mn.w = __uint_as_float(t);
-        b.node_aabbs[2ull * (leaf_base + t)] = mn;
-        b.node_aabbs[2ull * (leaf_base + t) + 1] = mx;
-        v = {make_float4(mn.x, mn.y, mn.z, 0.0f), make_float4(mx.x, mx.y, mx.z, 0.0f)};
-    }
-    Box2 pre = v, suf = v;
+    float4* stage = s_stage[w];
+#pragma unroll 1
+    for (uint32_t at = threadIdx.x; at < kRefitBlock; at += kRefitThreads) {
+        const uint32_t t = blockIdx.x * kRefitBlock + at;
+        const uint32_t live = __ballot_sync(0xffffffffu, t < n);
+        // the node's range and children, on their way while the leaf's box is fetched
+        const bool node = n > 1 && t < n - 1;
+        const uint2 rg = node ? __ldg(b.node_ranges + t) : make_uint2(1u, 0u);
+        const uint2 ch = node ? __ldg(b.children + t) : make_uint2(0u, 0u);
+        Box2 v = box_empty();
+        float4 box[2];
+        const uint32_t j = t < n ? b.svals[t] : 0u;
+        if (t < n) {
+            float4 mn = b.aabbs[2ull * j], mx = b.aabbs[2ull * j + 1];
+            mn.w = __uint_as_float(t);
+            box[0] = mn;
+            box[1] = mx;
+            v = {make_float4(mn.x, mn.y, mn.z, 0.0f), make_float4(mx.x, mx.y, mx.z, 0.0f)};
+        }
+        store_rows<2>(stage, box, b.node_aabbs + 2ull * (leaf_base + (t - lane)), live, lane);
+        const bool inner = node && (rg.x >> 5) == (rg.y >> 5);
+        const uint32_t cross = __ballot_sync(0xffffffffu, node && !inner);
+        if (lane == 0) s_cross[at >> 5] = cross;
+        Box2 pre = v, suf = v;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const Box2 u = shfl_box(pre, o, true);
-        if ((int)lane >= o) pre = box_union(pre, u);
-        const Box2 d = shfl_box(suf, o, false);
-        if ((int)lane + o < 32) suf = box_union(suf, d);
-    }
-    if (t < n) {
-        float4* ls = b.leaf_scan + 4ull * t;
-        ls[0] = pre.mn; ls[1] = pre.mx; ls[2] = suf.mn; ls[3] = suf.mx;
-    }
-    {
-        Box2 T[5];
-        warp_sparse_table(T, v, lane);
-        uint2 rg = make_uint2(1u, 0u);
-        bool inner = false;
-        if (n > 1 && t < n - 1) {
-            rg = b.node_ranges[t];
-            inner = (rg.x >> 5) == (rg.y >> 5);
+        for (int o = 1; o < 32; o <<= 1) {
+            const Box2 u = shfl_box(pre, o, true);
+            if ((int)lane >= o) pre = box_union(pre, u);
+            const Box2 d = shfl_box(suf, o, false);
+            if ((int)lane + o < 32) suf = box_union(suf, d);
         }
-        const Box2 r = warp_range_union(T, inner, rg.x & 31u, rg.y & 31u, lane);
-        if (inner) {
-            b.node_aabbs[2ull * t] = make_float4(r.mn.x, r.mn.y, r.mn.z, __uint_as_float(rg.y));
-            b.node_aabbs[2ull * t + 1] = make_float4(r.mx.x, r.mx.y, r.mx.z, 0.0f);
+        const float4 ls[4] = {pre.mn, pre.mx, suf.mn, suf.mx};
+        store_rows<4>(stage, ls, b.leaf_scan + 4ull * (t - lane), live, lane);
+        {
+            Box2 T[5];
+            warp_sparse_table(T, v, lane);
+            const Box2 r = warp_range_union(T, inner, rg.x & 31u, rg.y & 31u, lane);
+            box[0] = make_float4(r.mn.x, r.mn.y, r.mn.z, __uint_as_float(rg.y));
+            box[1] = make_float4(r.mx.x, r.mx.y, r.mx.z, 0.0f);
+            store_rows<2>(stage, box, b.node_aabbs + 2ull * (t - lane), __ballot_sync(0xffffffffu, inner), lane);
+            write_chunk_records(b, inner, rg, ch, r, v, j, t, leaf_base, lane, stage);
         }
-        write_chunk_records(b, inner, rg, r, v, j, t, leaf_base, lane);
-        // the other internal nodes, listed for k_refit_nodes (one reservation per warp)
-        const bool cross = n > 1 && t < n - 1 && !inner;
-        const uint32_t cm = __ballot_sync(0xffffffffu, cross);
-        if (cm) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(&b.counts->cross_nodes, (uint32_t)__popc(cm));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (cross) b.cross_nodes[base + __popc(cm & ((1u << lane) - 1u))] = t;
-        }
+        if (lane == 31) s_chunk[at >> 5] = pre;
     }
-    if (lane == 31) s_chunk[w] = pre;
     __syncthreads();
+    if (w == 1) {   // the nodes across chunks, listed for k_refit_nodes (one reservation per block)
+        uint32_t m = s_cross[lane];
+        uint32_t at = __popc(m);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, at, o);
+            if ((int)lane >= o) at += u;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, at, 31);
+        uint32_t base = 0;
+        if (lane == 0 && total) base = atomicAdd(&b.counts->cross_nodes, total);
+        at += __shfl_sync(0xffffffffu, base, 0) - __popc(m);
+        for (; m; m &= m - 1u) b.cross_nodes[at++] = blockIdx.x * kRefitBlock + lane * 32u + (uint32_t)__ffs(m) - 1u;
+    }
     if (w == 0) {
         const Box2 c = s_chunk[lane];
         Box2 cp = c, cs = c;
@@ -2982,7 +3033,7 @@ cudaError_t launch_broadphase(const StepBuffers& b, const StepParams& p, const S
                                 true);   // bins and tickets cleared by the tick's reset
     if (e != cudaSuccess) return e;
     k_karras<<<blocks_for(C, kBlock), kBlock, 0, s>>>(b, p);
-    k_refit_leaves<<<blocks_for(C, kRefitBlock), kRefitBlock, 0, s>>>(b, p);
+    k_refit_leaves<<<blocks_for(C, kRefitBlock), kRefitThreads, 0, s>>>(b, p);
     k_refit_super<<<1, 1024, 0, s>>>(b, p);
     // persistent over the listed nodes (their count is known on the device only)
     k_refit_nodes<<<std::min<uint32_t>(blocks_for(C, kBlock), (uint32_t)l.sm_count * 2u), kBlock, 0, s>>>(b, p);
