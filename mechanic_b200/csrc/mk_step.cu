@@ -331,7 +331,10 @@ constexpr uint32_t kLeafCode = 0x80000000u;
 // 1024-leaf super-chunks (over chunk totals) and a sparse table over the
 // super-chunk totals.
 constexpr uint32_t kRefitBlock = 1024;     // leaves per block: one super-chunk of 32 chunks
-constexpr uint32_t kRefitThreads = 512;    // each warp takes two chunks, two blocks share an SM
+// Threads of a block: 1,024 where every block has an SM to itself (a warp per chunk), else 512, two
+// chunks per warp and two blocks per SM.
+static inline uint32_t refit_threads(uint32_t blocks, int sm_count) { return blocks <= (uint32_t)sm_count ? 1024u : 512u; }
+constexpr uint32_t kRefitStage = 128;      // float4 of shared memory per warp
 
 struct Box2 {
     float4 mn, mx;
@@ -491,20 +494,21 @@ __device__ __forceinline__ void write_chunk_records(const StepBuffers& b, bool i
 // the block's super-chunk, and the super-chunk's total (level 0 of the sparse
 // table over super-chunks).
 // Bound by the latency of each chunk's chain (collider index, its box, the scans, the
-// range unions) and by the load-store unit.  On 401,946 colliders it took 47 us with 1,024
+// range unions) and by the load-store unit.  On 400k colliders it took 47 us with 1,024
 // threads per block (alone on their SM, idle while one warp does the block's last part), a
-// row stored per lane and the nodes listed by an atomic per warp; 40 with 512 threads, rows
-// through shared memory and an atomic per block.
-__global__ void __launch_bounds__(kRefitThreads, 2) k_refit_leaves(StepBuffers b, StepParams p) {
+// row stored per lane and the nodes listed by an atomic per warp; 38.5 with 512 threads, rows
+// through shared memory and an atomic per block.  On 100,000 colliders, where every block has
+// an SM to itself either way, 14.7 with 1,024 threads and 16.4 with 512.
+__global__ void __launch_bounds__(1024, 1) k_refit_leaves(StepBuffers b, StepParams p) {
     __shared__ Box2 s_chunk[32];
     __shared__ uint32_t s_cross[32];
-    __shared__ __align__(16) float4 s_stage[kRefitThreads / 32][128];
+    extern __shared__ __align__(16) float4 s_stage[];
     const uint32_t n = p.collider_count;
     const uint32_t lane = lane_id(), w = warp_id();
     const uint32_t leaf_base = n - 1;
-    float4* stage = s_stage[w];
+    float4* stage = s_stage + w * kRefitStage;
 #pragma unroll 1
-    for (uint32_t at = threadIdx.x; at < kRefitBlock; at += kRefitThreads) {
+    for (uint32_t at = threadIdx.x; at < kRefitBlock; at += blockDim.x) {
         const uint32_t t = blockIdx.x * kRefitBlock + at;
         const uint32_t live = __ballot_sync(0xffffffffu, t < n);
         // the node's range and children, on their way while the leaf's box is fetched
@@ -3033,8 +3037,9 @@ cudaError_t launch_broadphase(const StepBuffers& b, const StepParams& p, const S
                                 true);   // bins and tickets cleared by the tick's reset
     if (e != cudaSuccess) return e;
     k_karras<<<blocks_for(C, kBlock), kBlock, 0, s>>>(b, p);
-    k_refit_leaves<<<blocks_for(C, kRefitBlock), kRefitThreads, 0, s>>>(b, p);
-    k_refit_super<<<1, 1024, 0, s>>>(b, p);
+    const uint32_t refit_blocks = blocks_for(C, kRefitBlock), refit_block = refit_threads(refit_blocks, l.sm_count);
+    k_refit_leaves<<<refit_blocks, refit_block, refit_block / 32 * kRefitStage * sizeof(float4), s>>>(b, p);
+    if (refit_blocks > 1) k_refit_super<<<1, 1024, 0, s>>>(b, p);   // (one super-chunk: no level above it)
     // persistent over the listed nodes (their count is known on the device only)
     k_refit_nodes<<<std::min<uint32_t>(blocks_for(C, kBlock), (uint32_t)l.sm_count * 2u), kBlock, 0, s>>>(b, p);
     if (b.collider_scene) k_traverse<true><<<blocks_for(C, kTravThreads), kTravThreads, 0, s>>>(b, p);
@@ -3087,6 +3092,9 @@ cudaError_t step_prepare() {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_solve_block<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)BlockSolve<false>::kBytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_refit_leaves, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 32 * kRefitStage * (int)sizeof(float4));
     if (e == cudaSuccess) done.fetch_or(bit);
     return e;
 }
