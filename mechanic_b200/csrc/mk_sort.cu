@@ -488,7 +488,10 @@ cudaError_t launch_sort(const uint64_t* keys_in, const uint32_t* vals_in, uint64
         cudaError_t e = cudaMemsetAsync(c.hist, 0, (uint64_t)((char*)c.tickets - (char*)c.hist) + passes * 4, stream);
         if (e != cudaSuccess) return e;
     }
-    uint32_t hist_blocks = (uint32_t)std::min<uint64_t>((n + 4095) / 4096, (uint64_t)sm_count * 4);
+    // 1,024 keys per block while that fills the SMs no more than four deep: the histogram is a
+    // short chain of loads and shared atomics, and its bins' global sums cost less than idle SMs
+    // (402k keys 13.2 us with 4,096 keys per block, 9.1 with 2,048, 8.8 with 1,024)
+    uint32_t hist_blocks = (uint32_t)std::min<uint64_t>((n + 1023) / 1024, (uint64_t)sm_count * 4);
     k_radix_histogram<<<hist_blocks, kSortThreads, 0, stream>>>(keys_in, n, passes, c.hist, c.lookback,
                                                                 c.lookback_words, tile_keys);
     const uint32_t per_sm = ctas_per_sm ? ctas_per_sm : default_sort_ctas(items);
