@@ -697,6 +697,13 @@ typedef struct MkWaitProbe {
 } MkWaitProbe;
 MK_API int mk_selftest_bounded_wait(uint32_t which, uint32_t spin_limit, MkWaitProbe* out, MkError* err);
 
+/* What a wait that gave up may leave behind in the pair-key sort: a pass over
+ * keys that are not the ones its digit counts were taken from.  Runs one pass
+ * over n (1..2^20) such keys, whose places all lie past the end of the result,
+ * and counts the words stored there (0: a pass stores inside its n words
+ * whatever its counts say). */
+MK_API int mk_selftest_sort_bounds(uint32_t n, uint32_t* stored_outside, MkError* err);
+
 #ifdef __cplusplus
 }
 #endif

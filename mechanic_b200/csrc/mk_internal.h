@@ -123,6 +123,8 @@ cudaError_t launch_sort(const uint64_t* keys_in, const uint32_t* vals_in, uint64
 cudaError_t launch_sort_counted(const uint64_t* keys_in, uint64_t* keys_out, uint32_t capacity, const uint32_t* n_dev,
                                 uint32_t key_bits, void* scratch, uint64_t scratch_bytes, uint32_t* error_flags,
                                 cudaStream_t stream, int sm_count, uint32_t items);
+cudaError_t launch_stale_sort_pass(const uint64_t* keys, uint64_t* out, uint32_t n, uint32_t* scratch,
+                                   uint32_t* error_flags, cudaStream_t stream);
 void sort_clear_region(void* scratch, uint32_t n, uint32_t key_bits, bool values, void** ptr, uint64_t* bytes);
 
 // Device buffers of one handle's step (all device pointers).

@@ -296,8 +296,10 @@ __device__ __forceinline__ void onesweep_pass(const uint64_t* __restrict__ keys_
             if (j < total) {
                 const uint64_t kk = s_keys[j];
                 const uint32_t dst = s_global_base[(uint32_t)((kk >> shift) & 0xffu)] + j;
-                keys_out[dst] = kk;
-                if (vals_out) vals_out[dst] = s_vals[j];
+                if (dst < n) {   // always, unless a wait before this pass gave up and its bins are of other keys
+                    keys_out[dst] = kk;
+                    if (vals_out) vals_out[dst] = s_vals[j];
+                }
             }
         }
         __syncthreads();
@@ -459,6 +461,19 @@ static SortScratch sort_scratch(void* scratch, uint32_t n, uint32_t passes, bool
     c.lookback = (uint32_t*)p;
     c.lookback_words = (uint64_t)((n + 511) / 512) * kRadixBins;   // smallest tile: 512 keys
     return c;
+}
+
+// One pass over `n` keys whose bins are of other keys: every key has digit 200, the bins say digit 100, so the pass
+// places all of them past the n words of `out`.  `scratch` holds the bins, a ticket and the look-back words.
+cudaError_t launch_stale_sort_pass(const uint64_t* keys, uint64_t* out, uint32_t n, uint32_t* scratch,
+                                   uint32_t* error_flags, cudaStream_t stream) {
+    cudaError_t e = sort_prepare();
+    if (e != cudaSuccess) return e;
+    constexpr uint32_t kItems = 8, kTile = kSortThreads * kItems;
+    k_radix_onesweep<kSortThreads, kItems><<<(n + kTile - 1) / kTile, kSortThreads,
+                                             SortTile<kSortThreads, kItems>::kBytes, stream>>>(
+        keys, nullptr, out, nullptr, n, 0u, scratch, scratch + 512, scratch + 256, error_flags);
+    return cudaGetLastError();
 }
 
 // Stream-ordered sort of n keys with values.

@@ -15,6 +15,7 @@
 // thread arrives on.  Each probe is a few small blocks that all end by
 // themselves once the limit is reached.
 #include <cstdio>
+#include <vector>
 
 #include "mk_device.cuh"
 #include "mk_internal.h"
@@ -119,5 +120,45 @@ extern "C" int mk_selftest_bounded_wait(uint32_t which, uint32_t spin_limit, MkW
     out->blocks_launched = blocks;
     out->lookback_prefix = h.prefix;
     out->elapsed_ms = (double)ms;
+    return MK_OK;
+}
+
+extern "C" int mk_selftest_sort_bounds(uint32_t n, uint32_t* stored_outside, MkError* err) {
+    char msg[200];
+    auto fail = [&](int code, const char* what) {
+        if (err) {
+            err->code = code;
+            std::snprintf(err->message, sizeof(err->message), "%s", what);
+        }
+        mk::set_last_error(what);
+        return code;
+    };
+    if (!stored_outside || n == 0 || n > (1u << 20))
+        return fail(MK_ERR_INVALID_ARGUMENT, "selftest_sort_bounds: null result or n outside 1..2^20");
+    // keys | n result words and n more that no store may reach | bins, ticket, look-back words of 2,048-key tiles
+    const uint64_t tiles = (n + 2047ull) / 2048ull, words = 512ull + 256ull * tiles;
+    std::vector<uint64_t> keys(n, 200ull), out(2ull * n, ~0ull);
+    std::vector<uint32_t> scratch(words, 0u);
+    scratch[100] = n;
+    uint64_t* d = nullptr;
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaMalloc(&d, 24ull * n + 4ull * words + 16);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    uint32_t* ds = d ? reinterpret_cast<uint32_t*>(d + 3ull * n) : nullptr;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d, keys.data(), 8ull * n, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d + n, out.data(), 16ull * n, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ds, scratch.data(), 4ull * words, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = mk::launch_stale_sort_pass(d, d + n, n, ds, nullptr, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(out.data(), d + n, 16ull * n, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (s) cudaStreamDestroy(s);
+    if (d) cudaFree(d);
+    if (e != cudaSuccess) {
+        std::snprintf(msg, sizeof(msg), "selftest_sort_bounds: %s", cudaGetErrorString(e));
+        return fail(MK_ERR_DEVICE_FAILURE, msg);
+    }
+    uint32_t outside = 0;
+    for (uint64_t i = n; i < 2ull * n; ++i) outside += out[i] != ~0ull;
+    *stored_outside = outside;
     return MK_OK;
 }

@@ -29,6 +29,7 @@ EXPORTS = [
     "mk_op_mlp_train", "mk_set_warm_start_network", "mk_read_warm_start_samples",
     "mk_set_preconditioner_network", "mk_create_batch", "mk_scene_offsets", "mk_get_handle_tuning",
     "mk_set_handle_tuning", "mk_autotune", "mk_selftest_bounded_wait", "mk_published_state",
+    "mk_selftest_sort_bounds",
     "mk_interpolate_snapshot",
 ]
 
@@ -85,6 +86,7 @@ def library(path: str | None = None):
         "mk_set_handle_tuning": (i32, [vp, vp, vp]),
         "mk_autotune": (i32, [vp, u32, vp, vp, vp]),
         "mk_selftest_bounded_wait": (i32, [u32, u32, vp, vp]),
+        "mk_selftest_sort_bounds": (i32, [u32, vp, vp]),
         "mk_published_state": (i32, [vp, vp]),
         "mk_interpolate_snapshot": (i32, [vp, C.c_float, vp, vp, vp, vp]),
     }
@@ -544,6 +546,13 @@ def selftest_bounded_wait(which: int, spin_limit: int = 1000) -> abi.MkWaitProbe
     err = abi.MkError()
     _raise(library().mk_selftest_bounded_wait(int(which), int(spin_limit), C.byref(out), C.byref(err)), err)
     return out
+
+
+def selftest_sort_bounds(n: int) -> int:
+    """Words that a sort pass over n keys with the digit counts of other keys stores past its result."""
+    err, outside = abi.MkError(), C.c_uint32()
+    _raise(library().mk_selftest_sort_bounds(n, C.byref(outside), C.byref(err)), err)
+    return outside.value
 
 
 def version() -> str:
