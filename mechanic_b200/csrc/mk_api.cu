@@ -203,9 +203,10 @@ uint64_t carve(MkHandle* h, char* base) {
     }
     b.active = c.take<uint32_t>(P);
     b.contact_deltas = c.take<int32_t>(12 * P);
-    b.inc_count = c.take<uint32_t>(B);
+    b.inc_count = c.take<uint32_t>(B + 1ull);
     b.inc_off = c.take<uint32_t>(B + 1ull);
     b.inc_list = c.take<uint32_t>(2 * P);
+    b.long_chunks = c.take<uint2>(mk::long_chunk_capacity((uint32_t)P));
     b.inc_blocks = c.take<uint32_t>(1024);
     b.lam_heavy = c.take<float>(P);
     b.lookback_words = std::max<uint64_t>(P / 256 + 2, C / 256 + 2);
@@ -303,7 +304,7 @@ cudaError_t enqueue_tick(MkHandle* h, int parity, bool capturing) {
         if (h->collisions) {
             z.add(b.deltas, sizeof(int32_t) * 6ull * std::max(h->B, 1u));
             z.add(b.scene_bounds, 8 * sizeof(uint32_t));
-            z.add(b.inc_count, sizeof(uint32_t) * std::max(h->B, 1u));
+            z.add(b.inc_count, sizeof(uint32_t) * (std::max(h->B, 1u) + 1ull));
             z.add(b.grid_barrier, 64 * sizeof(uint32_t));
             z.add(b.ground_tile_count, sizeof(uint32_t) * ((h->C + 1023) / 1024));
             z.add(b.lookback, sizeof(uint64_t) * 4 * b.lookback_words);

@@ -175,10 +175,12 @@ struct StepBuffers {
     int32_t* contact_deltas;     // gather form: 12 per active contact, fixed-point deltas of body a, then of body b;
                                  // split form: 6 per active contact, body b's
     uint32_t* inc_count;         // per body: entries of its list, then a countdown while they are listed
-                                 // (cleared per tick; the split form's are counted by k_prepare)
+                                 // (cleared per tick; the split form's are counted by k_prepare);
+                                 // after the bodies, the number of long_chunks
     uint32_t* inc_off;           // body_count + 1: each body's first entry in inc_list
     uint32_t* inc_list;          // grouped by body.  Gather form, 2 x pair_capacity: 2 t + side of every active
                                  // contact t; split form: t of the active contacts where it is body b
+    uint2* long_chunks;          // split form, long_chunk_capacity: body and first entry of each chunk of a long list
     uint32_t* inc_blocks;        // per block of the cooperative solve: its bodies' entry total
     float* lam_heavy;            // split form: running normal impulse per active contact
     uint32_t heavy_form;         // heavy ticks: MK_HEAVY_SCATTER, MK_HEAVY_GATHER or MK_HEAVY_SPLIT
@@ -221,6 +223,9 @@ struct StepLaunch {
     uint32_t append_ctas;     // CTAs per SM of the ordered-append kernels (narrowphase, ground, prepare)
     uint32_t solve_items;     // 0: every block joins the cooperative solve; n: blocks for n contacts per thread
 };
+
+// Chunks that the long lists (more than 64 entries) of `pairs` entries can have.
+__host__ __device__ constexpr uint32_t long_chunk_capacity(uint32_t pairs) { return pairs / 64u + 1u; }
 
 // Device regions to clear at the start of a tick (16-byte aligned, sizes in 16-byte units).
 struct ZeroList {

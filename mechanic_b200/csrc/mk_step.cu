@@ -1849,9 +1849,12 @@ __device__ __forceinline__ void solve_fused_resident(const StepBuffers& b, const
 
 // Exclusive scan of inc_count[0, B) into inc_off over the grid: each
 // participating block scans a contiguous segment after adding up the totals
-// of the segments before it (published in inc_blocks).
+// of the segments before it (published in inc_blocks).  Lists of more than
+// `longest` entries are listed in chunks of kListChunk (at most `most_chunks`).
+constexpr uint32_t kListChunk = 512;
 __device__ __forceinline__ void gather_scan(const StepBuffers& b, uint32_t B, uint32_t parts, uint32_t* barrier,
-                                            uint32_t* flags, uint32_t* s_scan) {
+                                            uint32_t* flags, uint32_t* s_scan, uint32_t longest = 0xffffffffu,
+                                            uint32_t most_chunks = 0u) {
     const uint32_t seg = (B + parts - 1) / parts;
     const uint32_t lo = min(B, blockIdx.x * seg), hi = min(B, lo + seg);
     uint32_t sum = 0;
@@ -1869,6 +1872,11 @@ __device__ __forceinline__ void gather_scan(const StepBuffers& b, uint32_t B, ui
         uint32_t chunk;
         const uint32_t ex = block_exclusive_scan(v, s_scan, &chunk);
         if (i < hi) b.inc_off[i] = base + ex;
+        if (v > longest) {
+            const uint32_t n = (v + kListChunk - 1u) / kListChunk, at = atomicAdd(b.inc_count + B, n);
+            for (uint32_t k = 0; k < n && (uint64_t)at + k < most_chunks; ++k)
+                b.long_chunks[at + k] = make_uint2(i, base + ex + k * kListChunk);
+        }
         base += chunk;
     }
     if (blockIdx.x == parts - 1 && threadIdx.x == 0) b.inc_off[B] = base;
@@ -2001,41 +2009,106 @@ __device__ void solve_gather(const StepBuffers& b, const StepParams& p, GpuConta
 // whole warp per body on the 9.5M contacts (now 3.2).  The denominators kept per
 // contact instead of recomputed were slower there (3.81 ms: the passes are bound
 // by memory).
+//
+// A list of more than 16 rounds of that width (a floor or a container under
+// thousands of bodies; 32 rounds where the width is a warp), and of twice a
+// group's share of all entries, is cut into chunks of kListChunk entries, which
+// all warps take before the other bodies; the chunks' sums meet in the body's
+// delta row and the last one applies it.  The contact stage with a platform
+// under 20,000 boxes of four contacts takes 420 us, under 100,000 980 us; with
+// the platform's list left to its few lanes the former took 14,000 us with half
+// of the contacts, with one warp per body 3,640 and 18,300 us.  (Without the
+// share in the rule the 9.5M contacts' lists, 95 on average and up to 1,430,
+// were cut too, which cost their solve 80 us.)
+__device__ __forceinline__ void add_slot(const int2* slots, uint32_t t, uint32_t* sum) {
+    const int2* q = slots + 3ull * t;
+    const int2 v0 = __ldcg(q), v1 = __ldcg(q + 1), v2 = __ldcg(q + 2);
+    sum[0] += (uint32_t)v0.x; sum[1] += (uint32_t)v0.y;
+    sum[2] += (uint32_t)v1.x; sum[3] += (uint32_t)v1.y;
+    sum[4] += (uint32_t)v2.x; sum[5] += (uint32_t)v2.y;
+}
+// A body's new velocities from its slots' sums and body a's atomic sums, which it clears.
+__device__ __forceinline__ void apply_split(int32_t* deltas, uint32_t x, const uint32_t* sum, const float4* vl,
+                                            const float4* va, float4* dl, float4* da_out) {
+    const float s = (float)kFixedScale;
+    int2* d2 = reinterpret_cast<int2*>(deltas + 6ull * x);   // 24-byte rows are 8-byte aligned
+    const int2 v0 = __ldcg(d2), v1 = __ldcg(d2 + 1), v2 = __ldcg(d2 + 2);
+    if ((v0.x | v0.y | v1.x | v1.y | v2.x | v2.y) != 0) {
+        d2[0] = make_int2(0, 0);
+        d2[1] = make_int2(0, 0);
+        d2[2] = make_int2(0, 0);
+    }
+    const f3 ld = mkf3((float)(int32_t)(sum[0] + (uint32_t)v0.x), (float)(int32_t)(sum[1] + (uint32_t)v0.y),
+                       (float)(int32_t)(sum[2] + (uint32_t)v1.x)) / s;
+    const f3 ad = mkf3((float)(int32_t)(sum[3] + (uint32_t)v1.y), (float)(int32_t)(sum[4] + (uint32_t)v2.x),
+                       (float)(int32_t)(sum[5] + (uint32_t)v2.y)) / s;
+    dl[x] = f4(xyz(__ldg(vl + x)) + ld, 0.0f);
+    da_out[x] = f4(xyz(__ldg(va + x)) + ad, 0.0f);
+}
+// The chunks of the long lists, a warp each.  Not inlined: ticks without long lists keep
+// the registers of the solve's other loops.
+__device__ __noinline__ void split_long_lists(const uint2* table, uint32_t chunks, const uint32_t* off,
+                                              const uint32_t* list, uint32_t* count, const int2* slots,
+                                              int32_t* deltas, const float4* vl, const float4* va, float4* dl,
+                                              float4* da_out, uint32_t gwarp, uint32_t nwarps) {
+    const uint32_t lane = lane_id();
+    for (uint32_t c = gwarp; c < chunks; c += nwarps) {
+        const uint2 ch = __ldcg(table + c);
+        const uint32_t x = ch.x, e0 = __ldcg(off + x), e1 = __ldcg(off + x + 1);
+        const uint32_t end = min(e1, ch.y + kListChunk), rounds = end > ch.y ? (end - ch.y + 31u) >> 5 : 0u;
+        uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+#pragma unroll 4
+        for (uint32_t i = 0; i < rounds; ++i) {
+            const uint32_t e = ch.y + 32u * i + lane;
+            if (e < end) add_slot(slots, __ldcg(list + e), sum);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) sum[k] = __reduce_add_sync(0xffffffffu, sum[k]);
+        if (lane != 0) continue;
+        const uint32_t of = (e1 - e0 + kListChunk - 1u) / kListChunk;
+        if (of > 1u) {   // arrivals are counted in the list's countdown, zero once the first pass has filled it
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                if (sum[k]) atomicAdd(deltas + 6ull * x + k, (int32_t)sum[k]);
+                sum[k] = 0u;
+            }
+            __threadfence();
+            if (atomicAdd(count + x, 1u) != of - 1u) continue;
+            __threadfence();
+            count[x] = 0u;
+        }
+        apply_split(deltas, x, sum, vl, va, dl, da_out);
+    }
+}
 __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContact* cur, uint32_t A,
                             uint32_t iterations, uint32_t* barrier, uint32_t parts) {
     __shared__ uint32_t s_scan[33];
     uint32_t* flags = &b.diag->error_flags;
     const uint32_t B = p.body_count;
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, stride = parts * blockDim.x;
-    // ---- incidence lists of body b: offsets (the first pass fills in active positions t)
-    gather_scan(b, B, parts, barrier, flags, s_scan);
+    const uint32_t gwarp = gtid >> 5, nwarps = stride >> 5;
+    // ---- incidence lists of body b: offsets, and the chunks of those of more than `longest` entries (the
+    // first pass fills in active positions t)
+    uint32_t longest;
+    {
+        const uint32_t most = (A + B - 1u) / B;   // the average list is at most this
+        const uint32_t bits = most <= 8u ? 2u : most <= 24u ? 3u : most <= 64u ? 4u : 5u;
+        longest = max(bits == 5u ? 1024u : 16u << bits, 2u * (A / (nwarps << (5u - bits))));
+    }
+    gather_scan(b, B, parts, barrier, flags, s_scan, longest, long_chunk_capacity(p.pair_capacity));
     grid_barrier(barrier, flags, parts);
     const size_t Bs = B;
-    const float s = (float)kFixedScale;
     const uint32_t lane = lane_id();
     const uint32_t entries = __ldcg(b.inc_off + B);
+    const uint32_t chunks = min(__ldcg(b.inc_count + B), long_chunk_capacity(p.pair_capacity));
     const uint32_t average = (entries + B - 1u) / B;
     const uint32_t group_bits = average <= 8u ? 2u : average <= 24u ? 3u : 4u;
     const uint32_t group = 1u << group_bits;
     const uint32_t in_group = lane & (group - 1u), per_warp = 32u >> group_bits;
-    const uint32_t gwarp = gtid >> 5, nwarps = stride >> 5;
     const uint2 sl = contact_slice(A, parts);
     int2* slots = reinterpret_cast<int2*>(b.contact_deltas);   // 3 x int2 per active contact
-    // a body's new velocities from its slots' sums and body a's atomic sums, which it clears
     auto apply = [&](uint32_t x, const uint32_t* sum, const float4* vl, const float4* va, float4* dl, float4* da_out) {
-        int2* d2 = reinterpret_cast<int2*>(b.deltas + 6ull * x);   // 24-byte rows are 8-byte aligned
-        const int2 v0 = __ldcg(d2), v1 = __ldcg(d2 + 1), v2 = __ldcg(d2 + 2);
-        if ((v0.x | v0.y | v1.x | v1.y | v2.x | v2.y) != 0) {
-            d2[0] = make_int2(0, 0);
-            d2[1] = make_int2(0, 0);
-            d2[2] = make_int2(0, 0);
-        }
-        const f3 ld = mkf3((float)(int32_t)(sum[0] + (uint32_t)v0.x), (float)(int32_t)(sum[1] + (uint32_t)v0.y),
-                           (float)(int32_t)(sum[2] + (uint32_t)v1.x)) / s;
-        const f3 ad = mkf3((float)(int32_t)(sum[3] + (uint32_t)v1.y), (float)(int32_t)(sum[4] + (uint32_t)v2.x),
-                           (float)(int32_t)(sum[5] + (uint32_t)v2.y)) / s;
-        dl[x] = f4(xyz(__ldg(vl + x)) + ld, 0.0f);
-        da_out[x] = f4(xyz(__ldg(va + x)) + ad, 0.0f);
+        apply_split(b.deltas, x, sum, vl, va, dl, da_out);
     };
     for (uint32_t it = 0; it < iterations; ++it) {
         const float4* vl = it == 0 ? b.lin : b.vel_iter + (2 * (it - 1)) * Bs;
@@ -2090,17 +2163,15 @@ __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContac
         }
         grid_barrier(barrier, flags, parts);
         // ---- apply: body a's atomic sums plus the slots of the contacts where it is b
+        if (chunks)
+            split_long_lists(b.long_chunks, chunks, b.inc_off, b.inc_list, b.inc_count, slots, b.deltas, vl, va, dl, da_out,
+                             gwarp, nwarps);
         if (average > 64u) {
             for (uint32_t x = gwarp; x < B; x += nwarps) {   // a warp per body
                 const uint32_t e0 = __ldcg(b.inc_off + x), e1 = __ldcg(b.inc_off + x + 1);
+                if (e1 > e0 + longest) continue;
                 uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
-                for (uint32_t e = e0 + lane; e < e1; e += 32) {
-                    const int2* q = slots + 3ull * __ldcg(b.inc_list + e);
-                    const int2 v0 = __ldcg(q), v1 = __ldcg(q + 1), v2 = __ldcg(q + 2);
-                    sum[0] += (uint32_t)v0.x; sum[1] += (uint32_t)v0.y;
-                    sum[2] += (uint32_t)v1.x; sum[3] += (uint32_t)v1.y;
-                    sum[4] += (uint32_t)v2.x; sum[5] += (uint32_t)v2.y;
-                }
+                for (uint32_t e = e0 + lane; e < e1; e += 32) add_slot(slots, __ldcg(b.inc_list + e), sum);
 #pragma unroll
                 for (int c = 0; c < 6; ++c) sum[c] = __reduce_add_sync(0xffffffffu, sum[c]);
                 if (lane == 0) apply(x, sum, vl, va, dl, da_out);
@@ -2109,22 +2180,19 @@ __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContac
             for (uint32_t x0 = gwarp * per_warp; x0 < B; x0 += nwarps * per_warp) {   // a group of lanes per body
                 const uint32_t x = x0 + (lane >> group_bits);
                 uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
-                if (x < B) {
-                    const uint32_t e0 = __ldcg(b.inc_off + x) + in_group, e1 = __ldcg(b.inc_off + x + 1);
-                    const uint32_t rounds = e1 > e0 ? (e1 - e0 + group - 1u) >> group_bits : 0u;
+                bool whole = x < B;   // its list is not cut
+                if (whole) {
+                    const uint32_t begin = __ldcg(b.inc_off + x), e0 = begin + in_group, e1 = __ldcg(b.inc_off + x + 1);
+                    whole = e1 <= begin + longest;
+                    const uint32_t rounds = whole && e1 > e0 ? (e1 - e0 + group - 1u) >> group_bits : 0u;
 #pragma unroll 4
-                    for (uint32_t i = 0; i < rounds; ++i) {   // (a counted loop: its loads are issued together)
-                        const int2* q = slots + 3ull * __ldcg(b.inc_list + e0 + (i << group_bits));
-                        const int2 v0 = __ldcg(q), v1 = __ldcg(q + 1), v2 = __ldcg(q + 2);
-                        sum[0] += (uint32_t)v0.x; sum[1] += (uint32_t)v0.y;
-                        sum[2] += (uint32_t)v1.x; sum[3] += (uint32_t)v1.y;
-                        sum[4] += (uint32_t)v2.x; sum[5] += (uint32_t)v2.y;
-                    }
+                    for (uint32_t i = 0; i < rounds; ++i)   // (a counted loop: its loads are issued together)
+                        add_slot(slots, __ldcg(b.inc_list + e0 + (i << group_bits)), sum);
                 }
                 for (uint32_t o = group >> 1; o > 0; o >>= 1)
 #pragma unroll
                     for (int c = 0; c < 6; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
-                if (x < B && in_group == 0u) apply(x, sum, vl, va, dl, da_out);
+                if (whole && in_group == 0u) apply(x, sum, vl, va, dl, da_out);
             }
         }
         grid_barrier(barrier, flags, parts);
