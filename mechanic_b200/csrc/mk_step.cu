@@ -2200,7 +2200,7 @@ __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContac
 }
 
 // Whether this tick's contacts go to the one-block solve (k_solve_block).
-__device__ __forceinline__ bool block_solve_takes(const DevCounts* c);
+__device__ __forceinline__ bool block_solve_takes(const DevCounts* c, bool residual);
 
 // All solver iterations in one cooperative launch: warm start, then
 // (iterations - 1) projections, each followed by the velocity apply
@@ -2222,7 +2222,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_all(StepBuffers b, Step
                                                       uint32_t iterations, uint32_t* barrier, uint32_t items) {
     const uint32_t A = b.counts->active;
     if (A == 0u) return;   // collision.wgsl:744-747: no solve and no apply dispatch
-    if (block_solve_takes(b.counts)) return;   // solved by k_solve_block
+    if (block_solve_takes(b.counts, false)) return;   // solved by k_solve_block
     const uint32_t parts = solve_participants(A, p.body_count, items);
     if (blockIdx.x >= parts) return;
     const uint32_t first = blockIdx.x * blockDim.x;
@@ -2521,7 +2521,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_residual(StepBuffers b,
         if (blockIdx.x == 0 && threadIdx.x == 0) *b.solve_stats = SolveStats{0u, 0u, 1u, 0u, 0.0, 0.0};
         return;
     }
-    if (!learned && block_solve_takes(b.counts)) return;   // solved by k_solve_block
+    if (!learned && block_solve_takes(b.counts, true)) return;   // solved by k_solve_block
     const size_t B = p.body_count;
     const double tol2 = (double)p.contact_tol * (double)p.contact_tol;
     // candidate c ping-pongs between velocity pairs 2c and 2c + 1
@@ -2598,16 +2598,20 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_residual(StepBuffers b,
 // velocities are those of the cooperative forms bit for bit; bodies without an
 // active contact get the reference's apply of zero deltas from the other
 // blocks of the launch.  Bound: the dependent chain of one contact's projection
-// and the barriers.  Measured on one B200, 1,000 falling cubes, 170-250 active
-// contacts: a pass to a residual 12.3 us on the grid, 2.1 us here; eight fixed
-// passes 48 us on the grid, 35 us here with the set-up.  The line lies at one
-// contact per thread: beyond it a pass would take the one SM twice the issue
-// slots, while the grid's time hardly grows.
-constexpr uint32_t kBlockContacts = 1024;
+// and the barriers, then the one SM's issue slots.  Where the lines lie: to a
+// residual, a pass costs the block 2.1 us with 170-250 contacts and 7.1 with
+// 1,000, the grid 11.5 to 13.3, so every contact that has a thread is taken.
+// Fixed passes have a cheaper grid form (one barrier a pass), and the block pays
+// for its set-up: contact stage on one B200, block / grid, with as many bodies a
+// as contacts and a body b each: 256 contacts 37 / 49 us, 384 45 / 49, 512
+// 51 / 49, 1,000 80 / 51; contacts with the ground alone: 512 37 / 43, 768
+// 45 / 43, 1,000 53 / 45.
+constexpr uint32_t kBlockContacts = 1024;   // one per thread
+constexpr uint32_t kBlockPasses = 448;      // with a fixed number of passes
 constexpr uint32_t kBlockBodies = 2 * kBlockContacts;
 
-__device__ __forceinline__ bool block_solve_takes(const DevCounts* c) {
-    return c->active != 0u && c->active <= kBlockContacts && c->contacts <= kStampContacts;
+__device__ __forceinline__ bool block_solve_takes(const DevCounts* c, bool residual) {
+    return c->active != 0u && c->active <= (residual ? kBlockContacts : kBlockPasses) && c->contacts <= kStampContacts;
 }
 
 template <bool kResidual>
@@ -2691,7 +2695,7 @@ __global__ void __launch_bounds__(kBlockContacts) k_solve_block(StepBuffers b, S
                                                                 uint32_t iterations) {
     using L = BlockSolve<kResidual>;
     using Fixed = typename L::Fixed;
-    if (!block_solve_takes(b.counts)) return;
+    if (!block_solve_takes(b.counts, kResidual)) return;
     const uint32_t gen = b.tick->generation;
     if (blockIdx.x != 0) {   // bodies without an active contact: the apply of zero deltas
         for (uint32_t i = (blockIdx.x - 1) * blockDim.x + threadIdx.x; i < p.body_count;
