@@ -181,12 +181,15 @@ MechTopology derive_topology(const MkCreation* cr, MechParams& p) {
         }
         pad_to((t.side_body.size() + kPassBlock - 1) / kPassBlock * kPassBlock);
         p.padded_sides = (uint32_t)t.side_body.size();
-        t.hub_off.push_back(0u);
-        for (uint32_t body : t.hub_bodies) {
+        for (uint32_t h = 0; h < (uint32_t)t.hub_bodies.size(); ++h) {
+            const uint32_t body = t.hub_bodies[h], n = off[body + 1] - off[body];
+            for (uint32_t k = 0; k < n; k += kPassBlock)
+                t.hub_chunks.push_back(make_uint4(body, (uint32_t)t.side_entries.size() + k,
+                                                  std::min(n - k, kPassBlock) | h << 8, (n + kPassBlock - 1) / kPassBlock));
             for (uint32_t q = off[body]; q < off[body + 1]; ++q) put_side(entries[q]);
-            t.hub_off.push_back((uint32_t)t.side_entries.size() - p.padded_sides);
         }
         p.hub_bodies = (uint32_t)t.hub_bodies.size();
+        p.hub_chunks = (uint32_t)t.hub_chunks.size();
         p.all_sides = (uint32_t)t.side_entries.size();
     }
     // depth levels 1..max_depth (roots are skipped by the reconstruction)
@@ -333,8 +336,8 @@ void carve_mechanism(MechBuffers& m, const MechParams& p, uint32_t B, uint32_t J
     m.side_entries = reinterpret_cast<uint2*>(take(8ull * std::max(1u, p.all_sides)));
     m.side_place = reinterpret_cast<uint2*>(take(8ull * J));
     m.side_cache = reinterpret_cast<float4*>(take(16ull * kSideRows * std::max(1u, p.all_sides)));
-    m.hub_bodies = u32(p.hub_bodies);
-    m.hub_off = u32(p.hub_bodies + 1ull);
+    m.hub_chunks = reinterpret_cast<uint4*>(take(16ull * p.hub_chunks));
+    m.hub_sums = u32(8ull * p.hub_bodies);
     m.level_bodies = u32(B);
     if (p.walk_levels) {
         m.level_begin = u32(p.walk_levels + 1ull);
@@ -425,8 +428,7 @@ bool upload_mechanism(MechBuffers& m, const MechParams& p, const MechTopology& t
     if (e == cudaSuccess) e = put(m.side_body, t.side_body, s);
     if (e == cudaSuccess) e = put(m.side_entries, t.side_entries, s);
     if (e == cudaSuccess) e = put(m.side_place, t.side_place, s);
-    if (e == cudaSuccess) e = put(m.hub_bodies, t.hub_bodies, s);
-    if (e == cudaSuccess) e = put(m.hub_off, t.hub_off, s);
+    if (e == cudaSuccess) e = put(m.hub_chunks, t.hub_chunks, s);
     if (e == cudaSuccess) e = put(m.level_bodies, t.level_bodies, s);
     if (e == cudaSuccess && p.walk_levels) e = put(m.level_begin, t.level_offsets, s);
     if (e == cudaSuccess && p.walk_levels) e = put(m.level_parent, t.level_parent, s);
@@ -569,8 +571,11 @@ __device__ __forceinline__ void apply_fixed(const int32_t* v, float4& lin, float
     ang = f4(xyz(ang) + mkf3((float)v[3], (float)v[4], (float)v[5]) / s, 0.0f);
 }
 // Blocks [0, side_blocks): padded bearing sides.  [side_blocks, side_blocks +
-// hub_blocks): bodies of more than 32 bearings, a warp each.  Then the rest.
-template <bool kContacts>
+// hub_blocks): chunks of kPassBlock sides of bodies with more than 32 bearings; a body's
+// last chunk finishes it (a warp per body walked 5,000 sides in 190 us a pass, this takes 6).
+// Then the rest.  kHubs: there are such bodies (a kernel of its own: their part in the
+// common one cost the lattice's pass 0.5 us of 24).
+template <bool kContacts, bool kHubs>
 __global__ void __launch_bounds__(kPassBlock) k_bearing_pass(StepBuffers b, MechBuffers m, MechParams p, VelocityPass f,
                                                             uint32_t side_blocks, uint32_t hub_blocks) {
     const bool contacts = kContacts && b.counts->active != 0u;   // collision.wgsl:744: no apply without active contacts
@@ -605,6 +610,13 @@ __global__ void __launch_bounds__(kPassBlock) k_bearing_pass(StepBuffers b, Mech
         const uint64_t n = p.all_sides;
         const float4 ca = __ldg(cache), cb = __ldg(cache + n), t3 = __ldg(cache + 2 * n), t4 = __ldg(cache + 3 * n);
         const float4 in3 = __ldg(cache + 4 * n), in4 = __ldg(cache + 5 * n);
+        // the body's rotation and inertia rows before the branches that use them (the lattice's ticks 1% shorter)
+        const float4 rot = __ldg(b.rot + body), *rows = b.mass + 4ull * body;
+        const float4 i1 = __ldg(rows + 1), i2 = __ldg(rows + 2), i3 = __ldg(rows + 3);
+        auto inertia_of = [&](f3 v) {   // wii
+            const f3 l = quat_rotate(conjq(rot), v);
+            return quat_rotate(rot, xyz(i1) * l.x + xyz(i2) * l.y + xyz(i3) * l.z);
+        };
         float4 ol, oa;
         velocity(ent.y, ol, oa);
         auto add = [&](f3 l, f3 a) {
@@ -626,8 +638,8 @@ __global__ void __launch_bounds__(kPassBlock) k_bearing_pass(StepBuffers b, Mech
             const float den = row == 0 ? cb.w : row == 1 ? in3.w : in4.w;
             if (den <= 1.0e-12f) continue;
             const f3 imp = d * (0.5f * dot(rel, d) / den);
-            if (side_b) add(-imp * ca.w, wii(b, body, cross(arm_b, -imp)));
-            else add(imp * ca.w, wii(b, body, cross(arm_a, imp)));
+            if (side_b) add(-imp * ca.w, inertia_of(cross(arm_b, -imp)));
+            else add(imp * ca.w, inertia_of(cross(arm_a, imp)));
         }
         const f3 rang = side_b ? xyz(ang) - xyz(oa) : xyz(oa) - xyz(ang);
 #pragma unroll
@@ -663,20 +675,41 @@ __global__ void __launch_bounds__(kPassBlock) k_bearing_pass(StepBuffers b, Mech
         if (body != kInvalid && (lane == 31u || after != body)) finish(body, sum, lin, ang);
         return;
     }
-    if (blockIdx.x < side_blocks + hub_blocks) {
-        const uint32_t h = ((blockIdx.x - side_blocks) * blockDim.x + threadIdx.x) >> 5;
-        if (h >= p.hub_bodies) return;
-        const uint32_t body = m.hub_bodies[h];
+    if (kHubs && blockIdx.x < side_blocks + hub_blocks) {
+        __shared__ uint32_t s_sum[kPassBlock / 32][6];
+        const uint4 ch = __ldg(m.hub_chunks + (blockIdx.x - side_blocks));   // body, first side, sides | hub << 8, chunks
+        const uint32_t body = ch.x;
         uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
         float4 lin, ang;
         velocity(body, lin, ang);
-        for (uint32_t e = m.hub_off[h] + lane; e < m.hub_off[h + 1]; e += 32u)
-            add_side(body, p.padded_sides + e, lin, ang, sum);
+        if (threadIdx.x < (ch.z & 0xffu)) add_side(body, ch.y + threadIdx.x, lin, ang, sum);
 #pragma unroll
-        for (uint32_t o = 16; o > 0; o >>= 1)
+        for (int c = 0; c < 6; ++c) {
+            sum[c] = __reduce_add_sync(0xffffffffu, sum[c]);
+            if (lane == 0) s_sum[threadIdx.x >> 5][c] = sum[c];
+        }
+        __syncthreads();
+        if (threadIdx.x != 0) return;
 #pragma unroll
-            for (int c = 0; c < 6; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
-        if (lane == 0) finish(body, sum, lin, ang);
+        for (int c = 0; c < 6; ++c)
+#pragma unroll
+            for (uint32_t w = 1; w < kPassBlock / 32; ++w) sum[c] += s_sum[w][c];
+        if (ch.w > 1u) {
+            uint32_t* all = m.hub_sums + 8ull * (ch.z >> 8);   // six sums and the arrivals, zero between passes
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+                if (sum[c]) atomicAdd(all + c, sum[c]);
+            __threadfence();
+            if (atomicAdd(all + 6, 1u) != ch.w - 1u) return;
+            __threadfence();
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                sum[c] = __ldcg(all + c);
+                all[c] = 0u;
+            }
+            all[6] = 0u;
+        }
+        finish(body, sum, lin, ang);
         return;
     }
     // bodies without bearings: the apply of zero deltas
@@ -2729,7 +2762,6 @@ static void velocity_buffers(const StepBuffers& b, const MechParams& p, float4* 
     ang[1] = b.vel_iter + p.body_count;
 }
 static uint32_t side_blocks(const MechParams& p) { return p.padded_sides / kPassBlock; }
-static uint32_t hub_blocks(const MechParams& p) { return (p.hub_bodies * 32u + kPassBlock - 1) / kPassBlock; }
 static uint32_t rest_blocks(const MechParams& p) {
     return (p.body_count - p.bearing_bodies + kPassBlock - 1) / kPassBlock;
 }
@@ -2739,13 +2771,14 @@ static uint32_t rest_blocks(const MechParams& p) {
 static cudaError_t bearing_projections(MechBuffers& m, const StepBuffers& b, const MechParams& p, cudaStream_t s) {
     float4 *lin[2], *ang[2];
     velocity_buffers(b, p, lin, ang);
-    const uint32_t sides = side_blocks(p), hubs = hub_blocks(p), passes = std::max(1u, p.iterations);
+    const uint32_t sides = side_blocks(p), hubs = p.hub_chunks, passes = std::max(1u, p.iterations);
     for (uint32_t it = 0; it < passes; ++it) {
         const uint32_t from = it & 1u, to = from ^ 1u;
         const uint32_t rest = it == 0 ? rest_blocks(p) : 0u;
         if (sides + hubs + rest == 0) continue;
         const VelocityPass f{lin[from], ang[from], lin[to], ang[to], lin[from], ang[from], nullptr, nullptr};
-        k_bearing_pass<false><<<sides + hubs + rest, kPassBlock, 0, s>>>(b, m, p, f, sides, hubs);
+        auto* kernel = hubs ? k_bearing_pass<false, true> : k_bearing_pass<false, false>;
+        kernel<<<sides + hubs + rest, kPassBlock, 0, s>>>(b, m, p, f, sides, hubs);
     }
     if ((passes & 1u) && p.bearing_bodies)
         k_pass_back<<<nblocks(p.bearing_bodies), kMBlock, 0, s>>>(m, p.bearing_bodies,
@@ -2952,10 +2985,11 @@ cudaError_t enqueue_contact_solver_with_bearings(MechBuffers& m, const StepBuffe
         }, s);
     float4 *lin[2], *ang[2];
     velocity_buffers(b, p, lin, ang);
-    const uint32_t sides = side_blocks(p), hubs = hub_blocks(p), iterations = std::max(1u, l.iterations);
+    const uint32_t sides = side_blocks(p), hubs = p.hub_chunks, iterations = std::max(1u, l.iterations);
     cudaError_t e = launch_contact_solver_passes(b, sp, l, parity, lin, ang, [&](uint32_t it, int32_t* deltas, int32_t* clear) {
         const uint32_t from = it & 1u, to = from ^ 1u;
-        k_bearing_pass<true><<<sides + hubs + rest_blocks(p), kPassBlock, 0, s>>>(
+        auto* kernel = hubs ? k_bearing_pass<true, true> : k_bearing_pass<true, false>;
+        kernel<<<sides + hubs + rest_blocks(p), kPassBlock, 0, s>>>(
             b, m, p, VelocityPass{lin[from], ang[from], lin[to], ang[to], lin[to], ang[to], deltas, clear}, sides, hubs);
         return cudaGetLastError();
     }, s);

@@ -22,6 +22,7 @@ struct MechParams {
     uint32_t padded_sides = 0;       // bearing sides with their padding, whole blocks
     uint32_t most_sides = 1;         // most sides of a body in that list (at most 32)
     uint32_t hub_bodies = 0;         // bodies of more than 32 bearings
+    uint32_t hub_chunks = 0;         // blocks that their sides take
     uint32_t all_sides = 0;          // padded_sides and the hub bodies' sides
     uint32_t serial_contacts = 0;    // dynamic root and <= 64 bearings (device.rs:1370-1373)
     float dt = 1.0f / 60.0f, ang_damp = 0.98f;
@@ -71,8 +72,10 @@ struct MechBuffers {
     uint2* side_entries = nullptr;              // all_sides: {side, the other body}; those of hub bodies at the end
     uint2* side_place = nullptr;                // J: places of a bearing's two sides in that list
     float4* side_cache = nullptr;               // rows x all_sides: pose-only parts of each side's projection rows
-    uint32_t* hub_bodies = nullptr;             // bodies of more than 32 bearings
-    uint32_t* hub_off = nullptr;
+    uint4* hub_chunks = nullptr;                // of bodies with more than 32 bearings: {body, first side,
+                                                // sides | hub << 8, chunks of the body}
+    uint32_t* hub_sums = nullptr;               // 8 per hub body: sums of its chunks, and how many have arrived
+                                                // (zero between passes; the arena starts zeroed)
     // reconstruct_body_velocities by depth level (level l: bodies [off[l], off[l+1]))
     uint32_t* level_bodies = nullptr;
     const uint32_t* level_offsets = nullptr;    // host memory owned by the handle, level_count + 1 entries
@@ -134,7 +137,8 @@ MechParams make_mech_params(const MkCreation* cr, const StepParams& p, uint32_t 
                             float closure_tol, uint32_t closure_max_it, uint32_t precond);
 // Host-side closure topology and depth levels; fills the counts in `p`.
 struct MechTopology {
-    std::vector<uint32_t> pass_bodies, side_body, hub_bodies, hub_off;
+    std::vector<uint32_t> pass_bodies, side_body, hub_bodies;
+    std::vector<uint4> hub_chunks;
     std::vector<uint2> side_entries, side_place;
     std::vector<uint32_t> level_bodies, level_offsets, level_parent;
     std::vector<uint32_t> cl_bearings, cl_slot_off, cl_split, slot_body, cq_coords, cq_off, cq_slots, cb_bodies;
