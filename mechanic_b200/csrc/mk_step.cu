@@ -1388,7 +1388,8 @@ constexpr uint32_t kPrepareWarps = kBlock / 32;
 constexpr uint32_t kStampContacts = 4096;
 __global__ void __launch_bounds__(kBlock) k_prepare(StepBuffers b, StepParams p, AppendSite site, GpuContact* cur,
                                                     uint64_t* cur_keys, uint32_t* cur_feat, const GpuContact* prev,
-                                                    const uint64_t* prev_keys, const uint32_t* prev_feat) {
+                                                    const uint64_t* prev_keys, const uint32_t* prev_feat,
+                                                    uint32_t count_above) {
     __shared__ uint32_t s_rows[kPrepareItems * kPrepareWarps];   // active count of each (row, warp), then its offset
     __shared__ uint32_t s_total;
     __shared__ uint32_t s_tile;
@@ -1476,7 +1477,7 @@ __global__ void __launch_bounds__(kBlock) k_prepare(StepBuffers b, StepParams p,
                         row[2] = f4(arm_a, cached);
                         cur_feat[k] |= 1u << 24;
                         act = np.w > 1.0e-5f || vn < -1.0e-5f || cached > 1.0e-6f;
-                        if (act && bb != kInvalid && n > 2u * p.body_count)   // for the split solve's lists
+                        if (act && bb != kInvalid && n > count_above)   // for the split solve's lists
                             atomicAdd(b.inc_count + bb, 1u);
                         if (act && n <= kStampContacts) {   // for the one-block solve
                             b.body_stamp[a] = b.tick->generation;
@@ -2016,8 +2017,8 @@ __device__ void solve_gather(const StepBuffers& b, const StepParams& p, GpuConta
 // all warps take before the other bodies; the chunks' sums meet in the body's
 // delta row and the last one applies it.  The contact stage with a platform
 // under 20,000 boxes of four contacts takes 420 us, under 100,000 980 us; with
-// the platform's list left to its few lanes the former took 14,000 us with half
-// of the contacts, with one warp per body 3,640 and 18,300 us.  (Without the
+// the platform's list left to four lanes the former took 57,000 us, with one
+// warp per body they took 3,640 and 18,300 us.  (Without the
 // share in the rule the 9.5M contacts' lists, 95 on average and up to 1,430,
 // were cut too, which cost their solve 80 us.)
 __device__ __forceinline__ void add_slot(const int2* slots, uint32_t t, uint32_t* sum) {
@@ -3187,12 +3188,15 @@ void set_heavy_solve_form(uint32_t form) { g_heavy_solve_form = form <= MK_HEAVY
 uint32_t heavy_solve_form() { return g_heavy_solve_form; }
 constexpr uint32_t kDefaultHeavyForm = MK_HEAVY_SPLIT;   // measured fastest: tick 1 of the 100,000-body config 4.44 ms (scatter 5.12, gather 6.02)
 
-static void launch_prepare(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity, cudaStream_t s) {
+// split: a heavy tick will take the split solve, whose lists are counted here.
+static void launch_prepare(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity, bool split,
+                           cudaStream_t s) {
     const uint32_t grid = (uint32_t)l.sm_count * (l.append_ctas ? l.append_ctas : 8u);
     AppendSite prep{b.lookback + 3 * b.lookback_words, b.tickets + 3};
     const int prev = parity ^ 1;
     k_prepare<<<grid, kBlock, 0, s>>>(b, p, prep, b.contacts[parity], b.contact_keys[parity], b.features[parity],
-                                       b.contacts[prev], b.contact_keys[prev], b.features[prev]);
+                                       b.contacts[prev], b.contact_keys[prev], b.features[prev],
+                                       split ? 2u * p.body_count : 0xffffffffu);
 }
 
 // Dynamic shared memory of the one-block solves, set once per device (outside
@@ -3218,7 +3222,9 @@ cudaError_t step_prepare() {
 
 cudaError_t launch_contact_solver(const StepBuffers& b, const StepParams& p, const StepLaunch& l, int parity,
                                   cudaStream_t s, const std::function<cudaError_t()>& before_solve) {
-    launch_prepare(b, p, l, parity, s);
+    const bool residual = p.contact_tol > 0.0f;
+    const uint32_t heavy_form = g_heavy_solve_form ? g_heavy_solve_form : kDefaultHeavyForm;
+    launch_prepare(b, p, l, parity, !residual && heavy_form == MK_HEAVY_SPLIT, s);
     if (before_solve) {
         cudaError_t eb = before_solve();
         if (eb != cudaSuccess) return eb;
@@ -3233,10 +3239,9 @@ cudaError_t launch_contact_solver(const StepBuffers& b, const StepParams& p, con
     GpuContact* cur = b.contacts[parity];
     uint32_t* barrier = b.grid_barrier;
     StepBuffers bb = b;
-    bb.heavy_form = g_heavy_solve_form ? g_heavy_solve_form : kDefaultHeavyForm;
+    bb.heavy_form = heavy_form;
     StepParams pp = p;
     uint32_t learned = l.learned_warm ? 1u : 0u;
-    const bool residual = p.contact_tol > 0.0f;
     if (residual) {
         if (!b.deltas64 || !b.vel_res) return cudaErrorInvalidValue;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve_residual, kSolveThreads, 0);
@@ -3274,7 +3279,7 @@ cudaError_t launch_contact_solver_passes(const StepBuffers& b, const StepParams&
                                          cudaStream_t s) {
     const uint32_t grid = (uint32_t)l.sm_count * (l.append_ctas ? l.append_ctas : 8u);
     GpuContact* cur = b.contacts[parity];
-    launch_prepare(b, p, l, parity, s);
+    launch_prepare(b, p, l, parity, false, s);
     int32_t* deltas[2] = {b.deltas, b.deltas_extra};   // a pass clears the next iteration's
     for (uint32_t it = 0; it < std::max<uint32_t>(1u, l.iterations); ++it) {
         StepBuffers bb = b;
@@ -3291,7 +3296,7 @@ cudaError_t launch_contact_solver_serial(const StepBuffers& b, const StepParams&
                                          const std::function<cudaError_t()>& after_apply, cudaStream_t s) {
     const uint32_t grid = (uint32_t)l.sm_count * (l.append_ctas ? l.append_ctas : 8u);
     GpuContact* cur = b.contacts[parity];
-    launch_prepare(b, p, l, parity, s);
+    launch_prepare(b, p, l, parity, false, s);
     const uint32_t body_blocks = std::max<uint32_t>(1u, std::min<uint32_t>(blocks_for(p.body_count, kBlock), grid));
     k_solve_iter<true><<<grid, kBlock, 0, s>>>(b, p, cur, b.lin, b.ang);
     k_apply_iter<<<body_blocks, kBlock, 0, s>>>(b, p);
