@@ -7,7 +7,7 @@ from mechanic_b200.physics import InvalidArgument, selftest_sort_bounds
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 2048, 5000, 100_001])
+@pytest.mark.parametrize("n", [1, 2048, 5000, 65_537, 100_001])
 def test_pass_with_other_counts_stays_inside(cuda_lib, n):
     assert selftest_sort_bounds(n) == 0
 
