@@ -512,9 +512,11 @@ MK_API uint32_t mk_tick_kernel_count(const MkHandle* handle);
  * radix-sort tile: 2, 4, 6, 8, 11 or 16, or 32 for the 8,192-key tile of 512
  * threads x 16 keys; 0 = size-based default);
  * MK_TUNE_CLOSURE_GRID (the closure solves, the reference's loop and the PCG
- * to a residual: 0 = by size, one block below 512 closures and the whole grid
- * from there, 1 = always one block, 2 = always the grid; both give the same
- * results).  Returns the
+ * to a residual: 0 = by size, 1 = always one block, 2 = always the grid; all
+ * give the same results.  By size: a system whose data fit one block's shared
+ * memory is solved there (its evaluation spread over a cluster of eight blocks
+ * above 512 joints or bodies); the others by one block below 512 closures and by
+ * the whole grid from there, the two forms that 1 and 2 force).  Returns the
  * previous value, or -1 for an unknown key. */
 #define MK_TUNE_SORT_ITEMS 1u
 #define MK_TUNE_CLOSURE_GRID 2u

@@ -6,7 +6,8 @@
 //   and apply_velocity_deltas :318-337                     -> k_bearing_pass
 //   articulated.wgsl advance_coordinates :366-415          -> k_advance_coordinates
 //   mechanism.wgsl prepare_links / jump_* :72-149          -> k_prepare_links / k_jump (list-restricted)
-//   closure.wgsl evaluate / finalize / solve_closure_pcg   -> k_closure_loop (one block, all 12 Newton steps)
+//   closure.wgsl evaluate / finalize / solve_closure_pcg   -> k_closure_block (systems that fit its shared memory, all
+//                                                             12 Newton steps), else k_closure_loop (one block or grid)
 //   mechanism.wgsl publish_* :151-185                      -> k_publish
 //   articulated.wgsl reconstruct_body_velocities :431-456  -> k_reconstruct_level (one launch per depth)
 //   articulated.wgsl capture_coordinates :417-429          -> k_capture_coordinates
@@ -2812,12 +2813,16 @@ static cudaError_t reconstruct(MechBuffers& m, const StepBuffers& b, const MechP
     return cudaGetLastError();
 }
 
-// Closure solves (the reference's loop and the PCG to a residual): one block
-// below kGridClosures closures, the whole grid from there (both compute the
-// same values); a tuning override.  Measured on five-body chains: one block is
-// faster at 254 closures, even at 410, and the grid from about 1,000 (grid
-// barriers cost more than a block's syncs until one closure per thread no
-// longer fits).
+// Closure solves (the reference's loop and the PCG to a residual), all with the
+// same values: a system that fits takes k_closure_block (closure_block_shape);
+// of the others, those below kGridClosures closures take one block of the
+// kernels that keep their vectors in global memory, the rest the whole grid.
+// The tuning forces one block (1) or the grid (2) of the latter.  Mechanism
+// stage on one B200, reference loop and PCG, k_closure_block / one block / grid:
+// 300 loops of five bodies 540 / 1,155 / 1,756 and 332 / 818 / 1,019 us; loops
+// of three bodies, 512 476 / 754 / 1,532 and 307 / 555 / 844, 700 559 / 1,102 /
+// 1,463 and 354 / 723 / 852, 1,000 629 / 1,262 / 1,622 (PCG does not fit); one
+// loop of 200 bodies 983 / 3,040 / 6,952.
 constexpr uint32_t kGridClosures = 512;
 static uint32_t g_closure_grid = 0;
 void set_closure_grid(uint32_t mode) { g_closure_grid = mode <= 2u ? mode : 0u; }
@@ -2940,7 +2945,7 @@ cudaError_t enqueue_mechanism(MechBuffers& m, const StepBuffers& b, const MechPa
     const uint32_t mode = g_closure_grid;
     const bool grid = p.closures > 0 && (mode == 2u || (mode == 0u && p.closures >= kGridClosures));
     ClosureShape shape;
-    if (mode != 2u && closure_block_shape(p, shape)) {
+    if (mode == 0u && closure_block_shape(p, shape)) {
         if ((e = launch_closure_block(m, b, p, shape, s)) != cudaSuccess) return e;
     } else if (pcg_residual_mode(p)) {
         for (uint32_t step = 0; step < kClosureSteps; ++step) {

@@ -148,7 +148,7 @@ struct MechTopology {
 };
 MechTopology derive_topology(const MkCreation* cr, MechParams& p);
 cudaError_t mechanism_prepare();   // per-device kernel attributes; call outside stream capture
-// Reference-mode closure loop: 0 = by size, 1 = one block, 2 = the whole grid.
+// Closure solves: 0 = by size (in shared memory where the system fits), 1 = one block, 2 = the whole grid.
 void set_closure_grid(uint32_t mode);
 uint32_t closure_grid_mode();
 // Regions of the mechanism buffers to clear at the start of every tick.
