@@ -389,7 +389,7 @@ uint32_t sort_items_for(uint32_t n, int sm_count) {
     (void)sm_count;
     // above 2M keys the 8,192-key tile (standalone sort with values, one B200: 3.6M keys
     // 245 against 271 us at 16 keys per thread, 14M keys 817 against 868 us)
-    return n <= (1u << 16) ? 8u : n <= (1u << 21) ? 11u : 32u;
+    return n <= (1u << 21) ? 11u : 32u;
 }
 
 // The histogram bins and tile tickets of a sort's scratch: the region that must
