@@ -655,7 +655,8 @@ MK_API int mk_set_preconditioner_network(MkHandle* handle, const float* params, 
  * bf16 weights and activations on the tcgen05 tensor cores, f32 accumulation.
  * All pointers are device pointers; x and targets rows are 16 floats,
  * 16-byte aligned.  Waits inside the kernels are bounded: a timeout sets
- * MK_DEVICE_WAIT_TIMEOUT_FLAG in *error_flags (device memory). */
+ * MK_DEVICE_WAIT_TIMEOUT_FLAG in *error_flags (device memory).  `scratch` holds
+ * mk_op_mlp_scratch_bytes(n) bytes; the forward pass checks it but writes nothing there. */
 MK_API uint32_t mk_mlp_param_count(void);
 MK_API uint64_t mk_op_mlp_scratch_bytes(uint32_t max_samples);
 /* y[n][y_cols] = net(x[n][16]), 1 <= y_cols <= 16. */

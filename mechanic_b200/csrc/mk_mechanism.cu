@@ -9,7 +9,8 @@
 //   closure.wgsl evaluate / finalize / solve_closure_pcg   -> k_closure_block (systems that fit its shared memory, all
 //                                                             12 Newton steps), else k_closure_loop (one block or grid)
 //   mechanism.wgsl publish_* :151-185                      -> k_publish
-//   articulated.wgsl reconstruct_body_velocities :431-456  -> k_reconstruct_level (one launch per depth)
+//   articulated.wgsl reconstruct_body_velocities :431-456  -> k_reconstruct_level (one launch per depth), or
+//                                                             k_reconstruct_rows / _walk / _store (deep, narrow trees)
 //   articulated.wgsl capture_coordinates :417-429          -> k_capture_coordinates
 //   articulated.wgsl validate_articulated_state :458-484   -> k_validate_state
 //   bearings.wgsl validate_* :68-102                       -> k_validate_bearings

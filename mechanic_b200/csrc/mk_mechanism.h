@@ -169,6 +169,5 @@ void enqueue_validate_bearings(MechBuffers& m, const StepBuffers& b, const MechP
                                cudaStream_t s);
 void read_mechanism_readback(const MechBuffers& m, const MechParams& p, const GpuDiagnostics& d,
                              const ClosureState* cs, MkTickReadback* out);
-// bytes of network scratch the learned preconditioner needs (0 without it)
 
 }  // namespace mk

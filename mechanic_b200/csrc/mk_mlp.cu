@@ -9,7 +9,8 @@
 // W3 16x64 | b2 64 | b3 16; every CTA rounds the weights to bf16 as it brings
 // them into shared memory.
 //
-// A CTA of 128 threads takes 128-sample tiles.  Thread t owns sample t of
+// 128 threads take a tile of 128 samples: a training CTA one at a time, a forward CTA
+// up to 8 beside one another (1,024 threads).  Thread t of the 128 owns sample t of
 // the tile, which is TMEM lane t of every accumulator, so the epilogues are
 // one tcgen05.ld per 16 columns and no shuffles.  The backward pass reuses
 // the activations where they lie: the same shared-memory tiles are read
@@ -589,6 +590,8 @@ static cudaError_t prepare_attributes() {
     return e;
 }
 
+// The barrier word and the partials, in the size that callers have been asked for since the
+// weights were kept there too (12 KB, unused now): sizes refused before stay refused.
 uint64_t scratch_bytes(uint32_t max_samples) {
     (void)max_samples;
     int sms = g_sm_count > 0 ? g_sm_count : 148;
