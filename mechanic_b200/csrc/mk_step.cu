@@ -2046,12 +2046,11 @@ __device__ __forceinline__ void apply_split(int32_t* deltas, uint32_t x, const u
     dl[x] = f4(xyz(__ldg(vl + x)) + ld, 0.0f);
     da_out[x] = f4(xyz(__ldg(va + x)) + ad, 0.0f);
 }
-// The chunks of the long lists, a warp each.  Not inlined: ticks without long lists keep
-// the registers of the solve's other loops.
-__device__ __noinline__ void split_long_lists(const uint2* table, uint32_t chunks, const uint32_t* off,
-                                              const uint32_t* list, uint32_t* count, const int2* slots,
-                                              int32_t* deltas, const float4* vl, const float4* va, float4* dl,
-                                              float4* da_out, uint32_t gwarp, uint32_t nwarps) {
+// The chunks of the long lists, a warp each.
+__device__ __forceinline__ void split_long_lists(const uint2* table, uint32_t chunks, const uint32_t* off,
+                                                 const uint32_t* list, uint32_t* count, const int2* slots,
+                                                 int32_t* deltas, const float4* vl, const float4* va, float4* dl,
+                                                 float4* da_out, uint32_t gwarp, uint32_t nwarps) {
     const uint32_t lane = lane_id();
     for (uint32_t c = gwarp; c < chunks; c += nwarps) {
         const uint2 ch = __ldcg(table + c);
@@ -2111,93 +2110,100 @@ __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContac
     auto apply = [&](uint32_t x, const uint32_t* sum, const float4* vl, const float4* va, float4* dl, float4* da_out) {
         apply_split(b.deltas, x, sum, vl, va, dl, da_out);
     };
-    for (uint32_t it = 0; it < iterations; ++it) {
-        const float4* vl = it == 0 ? b.lin : b.vel_iter + (2 * (it - 1)) * Bs;
-        const float4* va = it == 0 ? b.ang : b.vel_iter + (2 * (it - 1) + 1) * Bs;
-        float4* dl = it + 1 == iterations ? b.lin : b.vel_iter + (2 * it) * Bs;
-        float4* da_out = it + 1 == iterations ? b.ang : b.vel_iter + (2 * it + 1) * Bs;
-        // ---- projections: body a by run sums and atomics, body b into the slot
-        for (uint32_t base = sl.x; base < sl.y; base += blockDim.x) {
-            const uint32_t t = base + threadIdx.x;
-            bool live = false;
-            uint32_t a = kInvalid;
-            int32_t da[6] = {0, 0, 0, 0, 0, 0}, db[6] = {0, 0, 0, 0, 0, 0};
-            // the row this thread reads next, fetched into L2 while this one is projected
-            const uint32_t kn = t + blockDim.x < sl.y ? __ldcg(b.active + t + blockDim.x) : kInvalid;
-            if (t < sl.y) {
-                const uint32_t k = __ldcg(b.active + t);
-                const float4* row = reinterpret_cast<const float4*>(cur + k);
-                const float4 r0 = __ldg(row), np = __ldg(row + 1), aa = __ldg(row + 2), ab = __ldg(row + 3);
-                a = __float_as_uint(r0.x);
-                const uint32_t bb = __float_as_uint(r0.y);
-                const f3 arm_a = xyz(aa), arm_b = xyz(ab);
-                const float4* wa = b.world_mass + 3ull * a;
-                const float4* wb = bb != kInvalid ? b.world_mass + 3ull * bb : nullptr;
-                const f3 vb = bb != kInvalid ? contact_velocity_it(vl, va, bb, arm_b) : mkf3(0, 0, 0);
-                const f3 nrm = xyz(np);
-                const float den = impulse_denominator(wa, wb, arm_a, arm_b, nrm);
-                float acc = it == 0 ? aa.w : __ldcg(b.lam_heavy + t);
-                if (!(den <= 0.0f)) {
-                    const f3 rel = vb - contact_velocity_it(vl, va, a, arm_a);
-                    live = it == 0
-                        ? contact_project<true>(p, wa, wb, arm_a, arm_b, nrm, np.w, ab.w < 0.0f, den, rel, acc, da, db)
-                        : contact_project<false>(p, wa, wb, arm_a, arm_b, nrm, np.w, ab.w < 0.0f, den, rel, acc, da, db);
-                    if (!live) {
+    // compiled for both: the long lists' part in the common loop cost the 9.5M contacts' solve 9 us and a
+    // lattice at rest 1.5 us a tick
+    auto passes = [&](auto any_long) {
+        constexpr bool kLong = decltype(any_long)::value;
+        for (uint32_t it = 0; it < iterations; ++it) {
+            const float4* vl = it == 0 ? b.lin : b.vel_iter + (2 * (it - 1)) * Bs;
+            const float4* va = it == 0 ? b.ang : b.vel_iter + (2 * (it - 1) + 1) * Bs;
+            float4* dl = it + 1 == iterations ? b.lin : b.vel_iter + (2 * it) * Bs;
+            float4* da_out = it + 1 == iterations ? b.ang : b.vel_iter + (2 * it + 1) * Bs;
+            // ---- projections: body a by run sums and atomics, body b into the slot
+            for (uint32_t base = sl.x; base < sl.y; base += blockDim.x) {
+                const uint32_t t = base + threadIdx.x;
+                bool live = false;
+                uint32_t a = kInvalid;
+                int32_t da[6] = {0, 0, 0, 0, 0, 0}, db[6] = {0, 0, 0, 0, 0, 0};
+                // the row this thread reads next, fetched into L2 while this one is projected
+                const uint32_t kn = t + blockDim.x < sl.y ? __ldcg(b.active + t + blockDim.x) : kInvalid;
+                if (t < sl.y) {
+                    const uint32_t k = __ldcg(b.active + t);
+                    const float4* row = reinterpret_cast<const float4*>(cur + k);
+                    const float4 r0 = __ldg(row), np = __ldg(row + 1), aa = __ldg(row + 2), ab = __ldg(row + 3);
+                    a = __float_as_uint(r0.x);
+                    const uint32_t bb = __float_as_uint(r0.y);
+                    const f3 arm_a = xyz(aa), arm_b = xyz(ab);
+                    const float4* wa = b.world_mass + 3ull * a;
+                    const float4* wb = bb != kInvalid ? b.world_mass + 3ull * bb : nullptr;
+                    const f3 vb = bb != kInvalid ? contact_velocity_it(vl, va, bb, arm_b) : mkf3(0, 0, 0);
+                    const f3 nrm = xyz(np);
+                    const float den = impulse_denominator(wa, wb, arm_a, arm_b, nrm);
+                    float acc = it == 0 ? aa.w : __ldcg(b.lam_heavy + t);
+                    if (!(den <= 0.0f)) {
+                        const f3 rel = vb - contact_velocity_it(vl, va, a, arm_a);
+                        live = it == 0
+                            ? contact_project<true>(p, wa, wb, arm_a, arm_b, nrm, np.w, ab.w < 0.0f, den, rel, acc, da, db)
+                            : contact_project<false>(p, wa, wb, arm_a, arm_b, nrm, np.w, ab.w < 0.0f, den, rel, acc, da, db);
+                        if (!live) {
 #pragma unroll
-                        for (int c = 0; c < 6; ++c) da[c] = db[c] = 0;
+                            for (int c = 0; c < 6; ++c) da[c] = db[c] = 0;
+                        }
                     }
+                    b.lam_heavy[t] = acc;
+                    if (it == 0 && bb != kInvalid)
+                        b.inc_list[__ldcg(b.inc_off + bb) + atomicSub(b.inc_count + bb, 1u) - 1u] = t;
+                    if (bb != kInvalid) {
+                        int2* q = slots + 3ull * t;
+                        q[0] = make_int2(db[0], db[1]);
+                        q[1] = make_int2(db[2], db[3]);
+                        q[2] = make_int2(db[4], db[5]);
+                    }
+                    if (it + 1 == iterations && !(den <= 0.0f))
+                        reinterpret_cast<float*>(cur + k)[11] = acc;   // the row's impulse (arm_a_impulse.w)
                 }
-                b.lam_heavy[t] = acc;
-                if (it == 0 && bb != kInvalid)
-                    b.inc_list[__ldcg(b.inc_off + bb) + atomicSub(b.inc_count + bb, 1u) - 1u] = t;
-                if (bb != kInvalid) {
-                    int2* q = slots + 3ull * t;
-                    q[0] = make_int2(db[0], db[1]);
-                    q[1] = make_int2(db[2], db[3]);
-                    q[2] = make_int2(db[4], db[5]);
-                }
-                if (it + 1 == iterations && !(den <= 0.0f))
-                    reinterpret_cast<float*>(cur + k)[11] = acc;   // the row's impulse (arm_a_impulse.w)
+                if (kn != kInvalid) asm volatile("prefetch.global.L2 [%0];" ::"l"(cur + kn));
+                add_contact_deltas(b.deltas, live, a, kInvalid, da, db);
             }
-            if (kn != kInvalid) asm volatile("prefetch.global.L2 [%0];" ::"l"(cur + kn));
-            add_contact_deltas(b.deltas, live, a, kInvalid, da, db);
-        }
-        grid_barrier(barrier, flags, parts);
-        // ---- apply: body a's atomic sums plus the slots of the contacts where it is b
-        if (chunks)
-            split_long_lists(b.long_chunks, chunks, b.inc_off, b.inc_list, b.inc_count, slots, b.deltas, vl, va, dl, da_out,
-                             gwarp, nwarps);
-        if (average > 64u) {
-            for (uint32_t x = gwarp; x < B; x += nwarps) {   // a warp per body
-                const uint32_t e0 = __ldcg(b.inc_off + x), e1 = __ldcg(b.inc_off + x + 1);
-                if (e1 > e0 + longest) continue;
-                uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
-                for (uint32_t e = e0 + lane; e < e1; e += 32) add_slot(slots, __ldcg(b.inc_list + e), sum);
+            grid_barrier(barrier, flags, parts);
+            // ---- apply: body a's atomic sums plus the slots of the contacts where it is b
+            if constexpr (kLong)
+                split_long_lists(b.long_chunks, chunks, b.inc_off, b.inc_list, b.inc_count, slots, b.deltas, vl, va, dl,
+                                 da_out, gwarp, nwarps);
+            if (average > 64u) {
+                for (uint32_t x = gwarp; x < B; x += nwarps) {   // a warp per body
+                    const uint32_t e0 = __ldcg(b.inc_off + x), e1 = __ldcg(b.inc_off + x + 1);
+                    if (kLong && e1 > e0 + longest) continue;
+                    uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+                    for (uint32_t e = e0 + lane; e < e1; e += 32) add_slot(slots, __ldcg(b.inc_list + e), sum);
 #pragma unroll
-                for (int c = 0; c < 6; ++c) sum[c] = __reduce_add_sync(0xffffffffu, sum[c]);
-                if (lane == 0) apply(x, sum, vl, va, dl, da_out);
-            }
-        } else {
-            for (uint32_t x0 = gwarp * per_warp; x0 < B; x0 += nwarps * per_warp) {   // a group of lanes per body
-                const uint32_t x = x0 + (lane >> group_bits);
-                uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
-                bool whole = x < B;   // its list is not cut
-                if (whole) {
-                    const uint32_t begin = __ldcg(b.inc_off + x), e0 = begin + in_group, e1 = __ldcg(b.inc_off + x + 1);
-                    whole = e1 <= begin + longest;
-                    const uint32_t rounds = whole && e1 > e0 ? (e1 - e0 + group - 1u) >> group_bits : 0u;
+                    for (int c = 0; c < 6; ++c) sum[c] = __reduce_add_sync(0xffffffffu, sum[c]);
+                    if (lane == 0) apply(x, sum, vl, va, dl, da_out);
+                }
+            } else {
+                for (uint32_t x0 = gwarp * per_warp; x0 < B; x0 += nwarps * per_warp) {   // a group of lanes per body
+                    const uint32_t x = x0 + (lane >> group_bits);
+                    uint32_t sum[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+                    bool whole = x < B;   // its list is not cut
+                    if (whole) {
+                        const uint32_t begin = __ldcg(b.inc_off + x), e0 = begin + in_group, e1 = __ldcg(b.inc_off + x + 1);
+                        whole = !kLong || e1 <= begin + longest;
+                        const uint32_t rounds = whole && e1 > e0 ? (e1 - e0 + group - 1u) >> group_bits : 0u;
 #pragma unroll 4
-                    for (uint32_t i = 0; i < rounds; ++i)   // (a counted loop: its loads are issued together)
-                        add_slot(slots, __ldcg(b.inc_list + e0 + (i << group_bits)), sum);
-                }
-                for (uint32_t o = group >> 1; o > 0; o >>= 1)
+                        for (uint32_t i = 0; i < rounds; ++i)   // (a counted loop: its loads are issued together)
+                            add_slot(slots, __ldcg(b.inc_list + e0 + (i << group_bits)), sum);
+                    }
+                    for (uint32_t o = group >> 1; o > 0; o >>= 1)
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
-                if (whole && in_group == 0u) apply(x, sum, vl, va, dl, da_out);
+                        for (int c = 0; c < 6; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+                    if (whole && in_group == 0u) apply(x, sum, vl, va, dl, da_out);
+                }
             }
+            grid_barrier(barrier, flags, parts);
         }
-        grid_barrier(barrier, flags, parts);
-    }
+    };
+    if (chunks) passes(std::true_type{});
+    else passes(std::false_type{});
 }
 
 // Whether this tick's contacts go to the one-block solve (k_solve_block).
