@@ -937,7 +937,7 @@ __device__ __forceinline__ f3 sat_axis(const Box& a, const Box& b, f3 delta, uin
 }
 
 // collision.wgsl:422-486: axes A0 B0 A1 B1 A2 B2 then Ai x Bj, first negative
-// penetration returns immediately.  Bound by instruction issue (0.91 of the
+// penetration returns immediately.  Bound by instruction issue (0.89 of the
 // slots), so only penetrations and the best one's number are kept, and the axis
 // is formed once at the end: 1,000,003 box pairs 49.2 us (53.3 with the axis carried along).
 // Packed pairs of axes (f32x2) were slower, 73 us for a fifth fewer instructions: a packed
@@ -1996,7 +1996,7 @@ __device__ void solve_gather(const StepBuffers& b, const StepParams& p, GpuConta
 // sums its slots through an incidence list in the apply.  k_prepare counts the
 // lists, a scan here places them and the first pass fills them (with passes of
 // their own over the contacts the set-up took 410 us of 3,686 on a tick of 9.5M
-// contacts; k_prepare is 23 us longer).  The running normal impulses live in a
+// contacts; k_prepare is 26 us longer).  The running normal impulses live in a
 // dense array during the solve (the rows are read-only until the last pass
 // writes them back).  Same integer sums, same bits.
 //
