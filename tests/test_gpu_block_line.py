@@ -35,15 +35,21 @@ def test_both_sides_of_the_line_bitexact(cuda_lib, n):
     gpu.close()
 
 
-def test_a_thousand_contacts_are_not_left_to_one_block(cuda_lib):
-    """Eight fixed passes over 1,000 contacts: the contact stage within 1.25 times the 51 us that
-    the grid takes; the block took 80."""
-    gpu = GpuPhysics(_pairs(1000), GpuPhysicsConfig(), capacities={"pair_capacity": 1 << 16})
+def stage_us(scene, cfg, ticks=10):
+    """The shortest contact stage of the ticks after the second, and that tick's passes."""
+    gpu = GpuPhysics(scene, cfg, capacities={"pair_capacity": 1 << 18})
     stage = []
-    for tick in range(1, 11):
+    for tick in range(1, ticks + 1):
         gpu.dispatch_tick(tick)
         rb = gpu.read_last_tick()
-        assert 980 <= rb.active_contact_count <= 1000
-        stage.append(rb.kernel_timings.contact_solver_ms * 1e3)
+        assert rb.error_flags == 0
+        stage.append((rb.kernel_timings.contact_solver_ms * 1e3, rb.contact_iterations))
     gpu.close()
-    assert min(stage[2:]) < 64.0
+    return min(stage[2:])
+
+
+def test_a_thousand_contacts_are_not_left_to_one_block(cuda_lib):
+    """Eight fixed passes over 1,000 contacts on the grid against 448 in the block (47 and 49 us); left to
+    the block, 1,000 took 80."""
+    many, few = (stage_us(_pairs(n), GpuPhysicsConfig())[0] for n in (1000, 448))
+    assert many < 1.35 * few

@@ -23,7 +23,7 @@ def _us(keys, values, bits):
 
 @pytest.mark.parametrize("n", [30_000, 65_000])
 def test_default_tile_is_near_the_best(cuda_lib, n):
-    """Within a tenth of the best tile of 256 threads; 8 keys per thread took 91 and 111 us at these
+    """Within 15% of the best tile of 256 threads; 8 keys per thread took 91 and 111 us at these
     sizes, 11 take 73 and 89."""
     g = torch.Generator(device="cuda").manual_seed(n)
     keys = torch.randint(0, (1 << 63) - 1, (n,), dtype=torch.int64, device="cuda", generator=g)
@@ -35,7 +35,7 @@ def test_default_tile_is_near_the_best(cuda_lib, n):
             tiles.append(_us(keys, values, 63))
         finally:
             physics.set_tuning(physics.TUNE_SORT_ITEMS, max(prev, 0))
-    assert default < 1.1 * min(tiles)
+    assert default < 1.15 * min(tiles)
 
 
 @pytest.mark.parametrize("n", [4097, 2816, 2816 * 2 + 1, 2816 * 16, 65_535, 65_537])
