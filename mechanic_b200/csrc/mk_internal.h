@@ -224,7 +224,7 @@ struct StepLaunch {
     uint32_t solve_items;     // 0: every block joins the cooperative solve; n: blocks for n contacts per thread
 };
 
-// Chunks that the long lists (more than 64 entries) of `pairs` entries can have.
+// Chunks that the long lists (more than 128 entries) of `pairs` entries can have.
 __host__ __device__ constexpr uint32_t long_chunk_capacity(uint32_t pairs) { return pairs / 64u + 1u; }
 
 // Device regions to clear at the start of a tick (16-byte aligned, sizes in 16-byte units).

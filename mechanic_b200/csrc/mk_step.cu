@@ -2011,16 +2011,16 @@ __device__ void solve_gather(const StepBuffers& b, const StepParams& p, GpuConta
 // contact instead of recomputed were slower there (3.81 ms: the passes are bound
 // by memory).
 //
-// A list of more than 16 rounds of that width (a floor or a container under
-// thousands of bodies; 32 rounds where the width is a warp), and of twice a
+// A list of more than 32 rounds of that width (a floor or a container under
+// thousands of bodies; 64 rounds where the width is a warp), and of twice a
 // group's share of all entries, is cut into chunks of kListChunk entries, which
 // all warps take before the other bodies; the chunks' sums meet in the body's
-// delta row and the last one applies it.  The contact stage with a platform
-// under 20,000 boxes of four contacts takes 420 us, under 100,000 980 us; with
-// the platform's list left to four lanes the former took 57,000 us, with one
-// warp per body they took 3,640 and 18,300 us.  (Without the
-// share in the rule the 9.5M contacts' lists, 95 on average and up to 1,430,
-// were cut too, which cost their solve 80 us.)
+// delta row and the last one applies it, about 7 us a pass.  The contact stage
+// with a platform under 20,000 boxes of four contacts takes 420 us, under 100,000
+// 980 us; with the platform's list left to four lanes the former took 57,000 us,
+// with one warp per body they took 3,640 and 18,300 us.  (With lists over 1,024
+// cut, the overlapping start of 4,557 bodies, lists of up to 1,430, took 278 us
+// instead of 243; without the share in the rule 9.5M contacts took 80 us more.)
 __device__ __forceinline__ void add_slot(const int2* slots, uint32_t t, uint32_t* sum) {
     const int2* q = slots + 3ull * t;
     const int2 v0 = __ldcg(q), v1 = __ldcg(q + 1), v2 = __ldcg(q + 2);
@@ -2093,7 +2093,7 @@ __device__ void solve_split(const StepBuffers& b, const StepParams& p, GpuContac
     {
         const uint32_t most = (A + B - 1u) / B;   // the average list is at most this
         const uint32_t bits = most <= 8u ? 2u : most <= 24u ? 3u : most <= 64u ? 4u : 5u;
-        longest = max(bits == 5u ? 1024u : 16u << bits, 2u * (A / (nwarps << (5u - bits))));
+        longest = max(bits == 5u ? 2048u : 32u << bits, 2u * (A / (nwarps << (5u - bits))));
     }
     gather_scan(b, B, parts, barrier, flags, s_scan, longest, long_chunk_capacity(p.pair_capacity));
     grid_barrier(barrier, flags, parts);

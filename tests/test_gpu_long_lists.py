@@ -45,10 +45,10 @@ def _platforms(counts, sink=0.005, beside=()):
 
 
 @pytest.mark.parametrize("counts,box,cubes", [
-    ((16, 17, 128, 129, 256), 0.0, 0),      # 64, 68, 512, 516 and 1,024 entries beside short lists (4 lanes)
+    ((32, 33, 128, 129, 256), 0.0, 0),      # 128, 132, 512, 516 and 1,024 entries; cut above 128 (4 lanes)
     ((257, 600), 0.0, 0),                   # 1,028 and 2,400 entries
-    ((20, 300), 0.8, 500),                  # 16 lanes: a list is cut above 256 entries
-    ((200, 300), 0.1, 500),                 # a warp per body: above 1,024
+    ((20, 128, 129, 300), 0.8, 500),        # 16 lanes: cut above 512 entries
+    ((512, 513, 700), 0.1, 500),            # a warp per body: above 2,048
 ])
 def test_heavy_solve_with_long_lists_bitexact(cuda_lib, counts, box, cubes):
     beside = [scenes.falling_cubes(cubes, seed=5, box=box)] if cubes else []
