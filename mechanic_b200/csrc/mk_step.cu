@@ -2609,19 +2609,20 @@ __global__ void __launch_bounds__(kSolveThreads) k_solve_residual(StepBuffers b,
 // residual, a pass costs the block 2.1 us with 170-250 contacts and 7.1 with
 // 1,000, the grid 11.5 to 13.3, so every contact that has a thread is taken.
 // Fixed passes have a cheaper grid form (one barrier a pass), and the block pays
-// for its set-up: contact stage on one B200, block / grid, with as many bodies a
-// as contacts and a body b each: 256 contacts 37 / 49 us, 384 45 / 49, 512
-// 51 / 49, 1,000 80 / 51; contacts with the ground alone: 512 37 / 43, 768
-// 45 / 43, 1,000 53 / 45.  A list of more than kBlockList entries (a floor under
+// for its set-up and for each side of a contact: contact stage on one B200, block /
+// grid, with as many bodies a as contacts and a body b each: 256 contacts 37 / 49
+// us, 384 45 / 49, 512 51 / 49, 1,000 80 / 51; contacts with the ground alone: 512
+// 37 / 43, 768 45 / 43, 1,000 53 / 45.  A list of more than kBlockList entries (a floor under
 // the others) is summed by warps, not by a thread per component: a plate under
 // 1,000 cubes, to a residual, 24.2 -> 6.8 us a pass (the grid 13.3).
 constexpr uint32_t kBlockContacts = 1024;   // one per thread
-constexpr uint32_t kBlockPasses = 448;      // with a fixed number of passes
+constexpr uint32_t kBlockSides = 768;       // with a fixed number of passes: contacts, and those with a body b (at most)
 constexpr uint32_t kBlockBodies = 2 * kBlockContacts;
 constexpr uint32_t kBlockList = 32;   // entries of a list that one thread per component sums
 
 __device__ __forceinline__ bool block_solve_takes(const DevCounts* c, bool residual) {
-    return c->active != 0u && c->active <= (residual ? kBlockContacts : kBlockPasses) && c->contacts <= kStampContacts;
+    if (c->active == 0u || c->active > kBlockContacts || c->contacts > kStampContacts) return false;
+    return residual || c->active + min(c->active, c->narrow) <= kBlockSides;
 }
 
 template <bool kResidual>
