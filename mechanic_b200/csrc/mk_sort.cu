@@ -362,10 +362,14 @@ static uint64_t sort_mask(uint32_t passes) { return passes >= 8 ? ~0ull : (1ull 
 // its critical path is one tile's ranking (issue bound, so two tiles on one SM
 // take twice as long) plus the look-back chain (one L2 round trip per
 // kLookbackWindow tiles), so fewer, larger tiles win over spreading a sort
-// across every SM.  Measured per pass on B200: 100k keys 10.8 us at 8 keys per
-// thread (15.5 at 4); 400k 12.9 us at 11 or 16 (17.1 at 8); 1.6M 29.5 us at
-// 11; 6.4M 82 us at 16.  set_sort_items overrides the default (a tuning
-// parameter).
+// across every SM.  Measured per pass on B200: 400k keys 12.9 us at 11 or 16 keys
+// per thread (17.1 at 8); 1.6M 29.5 us at 11; 6.4M 82 us at 16.  Whole sorts of
+// 63-bit keys with values at 4 / 6 / 8 / 11 / 16 keys per thread: 6,000 keys 73 / 72
+// / 72 / 72 / 89 us; 20,000 101 / 84 / 77 / 72 / 89; 30,000 99 / 88 / 91 / 73 / 89;
+// 65,000 121 / 91 / 111 / 89 / 91 (and alike for fewer bits).  Up to 16,384 keys,
+// eight tiles of 8, a tick's broadphase is 1-2 us shorter with 8 than with 11 (10,000
+// colliders 97 and 99 us), from there on longer (20,000 109 and 105, 65,000 144 and
+// 125).  set_sort_items overrides the default (a tuning parameter).
 // 32 names the 8,192-key tile of 512 threads x 16 keys (the same keys per 256
 // threads as 32 keys each): half the tiles of the 4,096-key shape, so the
 // look-back frontier, which advances a window of tiles per L2 round trip,
@@ -389,7 +393,7 @@ uint32_t sort_items_for(uint32_t n, int sm_count) {
     (void)sm_count;
     // above 2M keys the 8,192-key tile (standalone sort with values, one B200: 3.6M keys
     // 245 against 271 us at 16 keys per thread, 14M keys 817 against 868 us)
-    return n <= (1u << 21) ? 11u : 32u;
+    return n <= (1u << 14) ? 8u : n <= (1u << 21) ? 11u : 32u;
 }
 
 // The histogram bins and tile tickets of a sort's scratch: the region that must
