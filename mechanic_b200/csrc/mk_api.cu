@@ -206,7 +206,6 @@ uint64_t carve(MkHandle* h, char* base) {
     b.inc_count = c.take<uint32_t>(B + 1ull);
     b.inc_off = c.take<uint32_t>(B + 1ull);
     b.inc_list = c.take<uint32_t>(2 * P);
-    b.long_chunks = c.take<uint2>(mk::long_chunk_capacity((uint32_t)P));
     b.inc_blocks = c.take<uint32_t>(1024);
     b.lam_heavy = c.take<float>(P);
     b.lookback_words = std::max<uint64_t>(P / 256 + 2, C / 256 + 2);
@@ -243,6 +242,7 @@ uint64_t carve(MkHandle* h, char* base) {
                             [&](uint64_t bytes) { return c.take<char>(bytes); });
     }
     if (h->config.mechanism_self_collisions == 0) b.components = c.take<uint32_t>(B);
+    b.long_chunks = c.take<uint2>(mk::long_chunk_capacity((uint32_t)P));
     return c.off;
 }
 
